@@ -42,8 +42,7 @@ struct vah_event {
     void *ep[2][2];    // [buffer][0 = e, 1 = p]
     int cur;           // current (e, p) buffer
     void *u[4], *up[4], *uS[4];
-    void *H[3][16];    // face fluxes as the left cell evaluates them (scratch of a stage)
-    void *HR[3][16];   // ... and as the right cell does (reference face semantics)
+    void *D[3][16];    // flux differences per axis (scratch of a stage)
     double *d_tab;
     uint32_t *d_exc;
     int nexc;
@@ -130,8 +129,7 @@ void free_all(vah_event *ev) {
     }
     for (int d = 0; d < 3; ++d)
         for (int n = 0; n < 16; ++n) {
-            cudaFree(ev->H[d][n]);
-            cudaFree(ev->HR[d][n]);
+            cudaFree(ev->D[d][n]);
         }
     cudaFree(ev->d_tab);
     cudaFree(ev->d_exc);
@@ -181,14 +179,7 @@ void fill_common(const vah_event *ev, StageArgs<S> &a) {
     a.zghosts = zghosts_eager(ev);
     a.counters = ev->d_counters;
     for (int d = 0; d < 3; ++d)
-        for (int n = 0; n < 16; ++n) {
-            a.H[d][n] = (S *)ev->H[d][n];
-            a.HR[d][n] = (S *)ev->HR[d][n];
-        }
-    // FP64 face/cell split: the x face launch writes each cell's x flux
-    // difference into the x face scratch, and the cell launch reads that
-    if (sizeof(S) == sizeof(double) && ev->opt.flux != VAH_FLUX_PER_CELL_FUSED)
-        for (int n = 0; n < 16; ++n) a.Dx[n] = (S *)ev->H[0][n];
+        for (int n = 0; n < 16; ++n) a.D[d][n] = (S *)ev->D[d][n];
     if (ev->validity)
         for (int m = 0; m < 11; ++m) a.regmap[m] = ev->vd[VAH_V_REGULATIONS + m];
 }
@@ -215,12 +206,11 @@ int timed(vah_event *ev, F launch) {
     return VAH_OK;
 }
 
-template <typename S>
-int timed_launch(vah_event *ev, const StageArgs<S> &a) {
+int timed_launch(vah_event *ev, const StageArgs<double> &a) {
     return timed(ev, [&]() {
-        if (ev->opt.flux == VAH_FLUX_PER_CELL_FUSED) return vah::launch_stage<S>(a, ev->opt.physics, ev->stream);
-        return vah::launch_stage_split<S>(a, ev->opt.physics, ev->opt.flux == VAH_FLUX_PER_CELL, ev->split,
-                                          ev->stream);
+        if (ev->opt.flux == VAH_FLUX_PER_CELL_FUSED) return vah::launch_stage<double>(a, ev->opt.physics, ev->stream);
+        return vah::launch_stage_split<double>(a, ev->opt.physics, ev->opt.flux == VAH_FLUX_PER_CELL, ev->split,
+                                               ev->stream);
     });
 }
 
@@ -519,10 +509,7 @@ extern "C" int vah_event_create(const vah_lattice *lat, const vah_hydro *hydro, 
     }
     if (opt->flux != VAH_FLUX_PER_CELL_FUSED && !ev->tile)
         for (int d = 0; d < (lat->nz > 1 ? 3 : 2); ++d)
-            for (int n = 0; n < ev->nq; ++n) {
-                alloc(&ev->H[d][n]);
-                if (opt->flux == VAH_FLUX_PER_CELL) alloc(&ev->HR[d][n]);
-            }
+            for (int n = 0; n < ev->nq; ++n) alloc(&ev->D[d][n]);
     if (rc == VAH_OK && cudaMalloc((void **)&ev->d_counters, 4 * sizeof(unsigned long long)) != cudaSuccess)
         rc = VAH_ERR_NOMEM;
     if (rc == VAH_OK) cudaMemset(ev->d_counters, 0, 4 * sizeof(unsigned long long));
@@ -858,7 +845,7 @@ int rk2_step_t(vah_event *ev, double t, double dt) {
         rc = tile_stage(ev, 1, t, dt);
         if (rc == VAH_OK) rc = tile_stage(ev, 2, t, dt);
     } else {
-        StageArgs<S> a;
+        StageArgs<double> a;
         stage1_args(ev, t, dt, a);
         rc = timed_launch(ev, a);
         if (rc != VAH_OK) return rc;
@@ -918,9 +905,8 @@ namespace {
 // event's current state, in stage-1 buffer roles (their outputs -- the face
 // buffers, qS, uS and the other (e, p) pair -- are scratch that the next step
 // rewrites), and keep the fastest. The device counters are restored after.
-template <typename S>
-int autotune_t(vah_event *ev, int reps, vah_tune_report *out) {
-    StageArgs<S> a;
+int autotune_split(vah_event *ev, int reps, vah_tune_report *out) {
+    StageArgs<double> a;
     stage1_args(ev, ev->last_t, ev->last_dt, a);
     const bool exact = ev->opt.flux == VAH_FLUX_PER_CELL;
     unsigned long long saved[4];
@@ -931,7 +917,7 @@ int autotune_t(vah_event *ev, int reps, vah_tune_report *out) {
     VAH_TRY(cudaEventCreate(&e1));
     int rc = VAH_OK;
     auto launch = [&](int kind, const vah::KindConfig &c) {
-        return vah::launch_split_kind<S>(a, ev->opt.physics, exact, kind, c, ev->stream);
+        return vah::launch_split_kind<double>(a, ev->opt.physics, exact, kind, c, ev->stream);
     };
     auto time_one = [&](int kind, const vah::KindConfig &c, double *ms) -> int {
         if (launch(kind, c) != cudaSuccess) return VAH_ERR_CUDA;  // warm-up
@@ -981,7 +967,7 @@ extern "C" int vah_event_autotune(vah_event *ev, int reps, vah_tune_report *out)
     memset(out, 0, sizeof(*out));
     if (ev->opt.flux == VAH_FLUX_PER_CELL_FUSED || ev->tile) return VAH_OK;  // one launch shape: nothing to tune
     VAH_TRY(cudaSetDevice(ev->opt.device));
-    return ev->elem == sizeof(float) ? autotune_t<float>(ev, reps, out) : autotune_t<double>(ev, reps, out);
+    return autotune_split(ev, reps, out);
 }
 
 extern "C" int vah_event_set_validity(vah_event *ev, int on) {

@@ -25,6 +25,7 @@
 #include "vah.h"
 #include "vah_ic_device.cuh"
 #include "vah_kernels.cuh"
+#include "vah_march.cuh"
 #include "vah_powf_exc.h"
 #include "vah_tile.cuh"
 
@@ -40,7 +41,7 @@ struct SlotDesc {
     long long plane;
     double dx, dy, dz, dt, etabar;
     S *q[16], *qS[16], *ep[2][2], *uA[4], *uB[4], *uS[4];
-    S *H[3][16], *HR[3][16];
+    S *D[3][16];  // flux differences per axis (FP64 form)
     unsigned char *fallback;  // per ghosted cell: 1 where the latest cell inversion fell back
     unsigned char *hot;       // per ghosted cell: 1 while e > e_freeze (freeze-out crossings)
     double e_freeze;
@@ -59,8 +60,11 @@ static_assert(sizeof(SlotClock) == sizeof(TileClock) && offsetof(SlotClock, pari
                   offsetof(SlotClock, t) == offsetof(TileClock, t),
               "SlotClock and TileClock share a layout");
 
+// One block's piece of work: a 32x4 tile of cells (cell kinds: its origin i0
+// and row r0), four strips of flux_x (from strip i0) or four strips of
+// flux_march (from strip i0) over the cells [r0, r1) along its axis.
 struct WorkItem {
-    int slot, i0, r0, pad;
+    int slot, i0, r0, r1;
 };
 
 enum { K_FX = 0, K_FY = 1, K_FZ = 2, K_C2 = 3, K_C3 = 4, K_NUM = 5 };
@@ -110,64 +114,70 @@ __device__ void make_args(StageArgs<S> &a, const SlotDesc<S> &d, const SlotClock
     a.eout = d.ep[stage == 1 ? 1 : 0][0];
     a.pout = d.ep[stage == 1 ? 1 : 0][1];
     for (int k = 0; k < 3; ++k)
-        for (int n = 0; n < 16; ++n) {
-            a.H[k][n] = d.H[k][n];
-            a.HR[k][n] = d.HR[k][n];
-        }
-    for (int n = 0; n < 16; ++n) a.Dx[n] = nullptr;  // the batch's cell launch differences H / HR itself
+        for (int n = 0; n < 16; ++n) a.D[k][n] = d.D[k][n];
     finish_args(a);
 }
 
-// Tiles are taken from the work-list in chunks of kChunk through an atomic
-// counter (reset before each launch): blocks that finish early take more,
-// so uneven events do not leave a tail; the list runs largest event first.
-constexpr int kChunk = 4;
+// Items are taken from the work-list in chunks through an atomic counter
+// (reset before each launch): blocks that finish early take more, so uneven
+// events do not leave a tail; the list runs largest event first. A march item
+// is a whole segment of four strips, so those go one by one.
+template <int KIND>
+constexpr int kChunk = KIND == K_FY || KIND == K_FZ ? 1 : 4;
 
-template <typename S, int PHYS, int KIND, bool EXACT, int MINB>
-__global__ void __launch_bounds__(kTX *kTY, MINB) batch_kernel(const SlotDesc<S> *__restrict__ descs,
-                                                         const SlotClock *__restrict__ clk,
-                                                         const WorkItem *__restrict__ work, int nwork, int stage,
-                                                         const Eos eos, unsigned *next) {
-    __shared__ StageArgs<S> sa;
+// The register caps of the event launches (vah_kernels.cuh).
+template <int KIND>
+constexpr int kKindMinb = KIND == K_FX ? kFluxXMinb : (KIND <= K_FZ ? kMarchMinb : kCellMinb);
+
+template <int PHYS, int KIND, bool EXACT>
+__global__ void __launch_bounds__(kTX *kTY, kKindMinb<KIND>) batch_kernel(const SlotDesc<double> *__restrict__ descs,
+                                                               const SlotClock *__restrict__ clk,
+                                                               const WorkItem *__restrict__ work, int nwork, int stage,
+                                                               const Eos eos, unsigned *next) {
+    extern __shared__ double march_sm[];  // march kinds: each warp's columns
+    __shared__ StageArgs<double> sa;
+    __shared__ HalfPointers hp;
     __shared__ int sa_slot, s_w0;
     const bool lead = threadIdx.x == 0 && threadIdx.y == 0;
+    const int warp = threadIdx.y;  // blockDim.x == 32
     if (lead) sa_slot = -1;
     for (;;) {
-    __syncthreads();  // s_w0 of the previous chunk has been read
-    if (lead) s_w0 = (int)atomicAdd(next, (unsigned)kChunk);
-    __syncthreads();
-    const int w0 = s_w0, w1 = min(nwork, w0 + kChunk);
-    if (w0 >= nwork) break;
-    // the per-event arguments in shared memory change only at event boundaries
-    for (int w = w0; w < w1; ++w) {
-        const WorkItem it = work[w];
+        __syncthreads();  // s_w0 of the previous chunk has been read
+        if (lead) s_w0 = (int)atomicAdd(next, (unsigned)kChunk<KIND>);
         __syncthreads();
-        if (lead && it.slot != sa_slot) {
-            make_args(sa, descs[it.slot], clk[it.slot], stage, eos);
-            sa_slot = it.slot;
-        }
-        __syncthreads();
-        const int i = it.i0 + threadIdx.x, r = it.r0 + threadIdx.y;
-        if (KIND <= K_FZ) {
-            const int ext0 = KIND == K_FX ? sa.nx + 1 : sa.nx;
-            const int ext1 = KIND == K_FY ? sa.ny + 1 : sa.ny;
-            const int ext2 = KIND == K_FZ ? sa.nz + 1 : sa.nz;
-            if (i < ext0 && r < ext1 * ext2) {
-                const int j = r % ext1, k = r / ext1;
-                const int gi = i + (KIND == K_FX ? 1 : 2), gj = j + (KIND == K_FY ? 1 : 2), gk = k + (KIND == K_FZ ? 1 : 2);
-                const long long st = KIND == K_FX ? 1 : (KIND == K_FY ? (long long)sa.ncx : sa.plane);
-                const long long s = gi + (long long)sa.ncx * gj + sa.plane * gk;
-                const int gl = KIND == K_FX ? gi : (KIND == K_FY ? gj : gk);
-                const int n = KIND == K_FX ? sa.nx : (KIND == K_FY ? sa.ny : sa.nz);
-                const unsigned fails = face_compute<S, PHYS, EXACT>(sa, s, KIND, st, gl >= 2, gl <= n);
-                if (fails & 255u) count_add(sa.counters + 0, fails & 255u);
-                if (fails >> 8) count_add(sa.counters + 2, 1ull);
+        const int w0 = s_w0, w1 = min(nwork, w0 + kChunk<KIND>);
+        if (w0 >= nwork) break;
+        // the per-event arguments in shared memory change only at event boundaries
+        for (int w = w0; w < w1; ++w) {
+            const WorkItem it = work[w];
+            __syncthreads();
+            const bool changed = it.slot != sa_slot;
+            __syncthreads();
+            if (changed) {
+                if (lead) {
+                    make_args(sa, descs[it.slot], clk[it.slot], stage, eos);
+                    sa_slot = it.slot;
+                }
+                __syncthreads();
+                if (KIND <= K_FZ) {
+                    set_half_pointers<PHYS>(hp, sa, threadIdx.y * kTX + threadIdx.x);
+                    __syncthreads();
+                }
             }
-        } else if (i < sa.nx && r < sa.ny * sa.nz) {
-            const int j = r % sa.ny, k = r / sa.ny;
-            cell_compute<S, PHYS, KIND == K_C3, EXACT>(sa, i + 2, j + 2, k + 2);
+            if (KIND == K_FX) {
+                if (it.i0 + warp < flux_x_strips(sa.nx, sa.ny, sa.nz)) flux_x<PHYS, EXACT>(sa, hp, it.i0 + warp);
+            } else if (KIND <= K_FZ) {
+                if (it.i0 + warp < march_strips(sa.nx * (KIND == K_FY ? sa.nz : sa.ny)))
+                    flux_march<PHYS, KIND == K_FY ? 1 : 2, EXACT>(sa, hp, it.i0 + warp, it.r0, it.r1,
+                                                                  march_sm + warp * kMarchDoubles<PHYS>);
+            } else {
+                const int i = it.i0 + threadIdx.x, r = it.r0 + threadIdx.y;
+                if (i < sa.nx && r < sa.ny * sa.nz) {
+                    const int j = r % sa.ny, k = r / sa.ny;
+                    cell_compute<double, PHYS, KIND == K_C3, true>(sa, i + 2, j + 2, k + 2);
+                }
+            }
         }
-    }
     }
 }
 
@@ -248,11 +258,7 @@ __global__ void observables_kernel(const SlotDesc<S> *__restrict__ descs, const 
             S *const *u = c.parity ? d.uB : d.uA;
             const double e = (double)d.ep[0][0][s], p = (double)d.ep[0][1][s], pl = (double)d.q[kSlotPL][s];
             const double ut = (double)u[0][s], ux = (double)u[1][s], uy = (double)u[2][s];
-            double ap[9];
-            ap[0] = 1.0;
-            ap[1] = pl / e;
-            for (int m = 2; m < 9; ++m) ap[m] = ap[m - 1] * ap[1];
-            double pt = 0.5 * (e - pl - poly::Rbar0(ap) * (e - 3 * p));
+            double pt = 0.5 * (e - pl - poly::Rbar0(pl / e) * (e - 3 * p));
             double pixx = 0, piyy = 0;
             if (Phys<PHYS>::PIMUNU) {
                 pixx = (double)d.q[9][s];
@@ -281,13 +287,16 @@ __global__ void observables_kernel(const SlotDesc<S> *__restrict__ descs, const 
     }
 }
 
-template <typename S, int PHYS, int KIND, bool EXACT, int MINB>
+template <int PHYS, int KIND>
+constexpr size_t kBatchSmem = KIND == K_FY || KIND == K_FZ ? kTY * kMarchDoubles<PHYS> * sizeof(double) : 0;
+
+template <int PHYS, int KIND, bool EXACT>
 int blocks_per_sm() {
     static int cached = 0;
     if (!cached) {
         int n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_kernel<S, PHYS, KIND, EXACT, MINB>, kTX * kTY,
-                                                          0) != cudaSuccess ||
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_kernel<PHYS, KIND, EXACT>, kTX * kTY,
+                                                          kBatchSmem<PHYS, KIND>) != cudaSuccess ||
             n < 1)
             n = 1;
         cached = n;
@@ -296,35 +305,21 @@ int blocks_per_sm() {
 }
 
 // A persistent grid of (SMs x resident blocks) walks the work-list.
-template <typename S, int PHYS, int KIND, bool EXACT, int MINB>
-cudaError_t launch_minb(const SlotDesc<S> *descs, const SlotClock *clk, const WorkItem *work, int nwork, int stage,
+template <int PHYS, int KIND, bool EXACT>
+cudaError_t launch_kind(const SlotDesc<double> *descs, const SlotClock *clk, const WorkItem *work, int nwork, int stage,
                         const Eos &eos, int sms, unsigned *next, cudaStream_t stream) {
-    const int grid = std::min((nwork + kChunk - 1) / kChunk, sms * blocks_per_sm<S, PHYS, KIND, EXACT, MINB>());
-    cudaError_t e = cudaMemsetAsync(next, 0, sizeof(unsigned), stream);
-    if (e != cudaSuccess) return e;
-    batch_kernel<S, PHYS, KIND, EXACT, MINB><<<grid, dim3(kTX, kTY), 0, stream>>>(descs, clk, work, nwork, stage, eos,
-                                                                                 next);
-    return cudaGetLastError();
-}
-
-// minb: the register-cap variant (face kinds 3, 4, 5; cell kinds 2, 3, 4).
-template <typename S, int PHYS, int KIND, bool EXACT>
-cudaError_t launch_kind(const SlotDesc<S> *descs, const SlotClock *clk, const WorkItem *work, int nwork, int stage,
-                        const Eos &eos, int sms, int minb, unsigned *next, cudaStream_t stream) {
     if (nwork <= 0) return cudaSuccess;
-    constexpr bool FACE = KIND <= K_FZ;
-    switch (minb) {
-    case 2:
-        if (FACE) break;
-        return launch_minb<S, PHYS, KIND, EXACT, 2>(descs, clk, work, nwork, stage, eos, sms, next, stream);
-    case 3: return launch_minb<S, PHYS, KIND, EXACT, 3>(descs, clk, work, nwork, stage, eos, sms, next, stream);
-    case 4: return launch_minb<S, PHYS, KIND, EXACT, 4>(descs, clk, work, nwork, stage, eos, sms, next, stream);
-    case 5:
-        if (!FACE) break;
-        return launch_minb<S, PHYS, KIND, EXACT, 5>(descs, clk, work, nwork, stage, eos, sms, next, stream);
-    default: break;
-    }
-    return cudaErrorInvalidValue;
+    constexpr size_t smem = kBatchSmem<PHYS, KIND>;
+    cudaError_t e = cudaSuccess;
+    if (smem)
+        e = cudaFuncSetAttribute(batch_kernel<PHYS, KIND, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)smem);
+    if (e != cudaSuccess) return e;
+    const int grid = std::min((nwork + kChunk<KIND> - 1) / kChunk<KIND>, sms * blocks_per_sm<PHYS, KIND, EXACT>());
+    if ((e = cudaMemsetAsync(next, 0, sizeof(unsigned), stream)) != cudaSuccess) return e;
+    batch_kernel<PHYS, KIND, EXACT><<<grid, dim3(kTX, kTY), smem, stream>>>(descs, clk, work, nwork, stage, eos,
+                                                                                  next);
+    return cudaGetLastError();
 }
 
 }  // namespace
@@ -367,7 +362,6 @@ struct vah_batch {
     std::vector<Slot> slots;
     std::vector<unsigned char> desc_host;  // host mirror of the descriptor array
     WorkItem *d_work[vah::K_NUM];
-    int minb[vah::K_NUM];  // register-cap variant per launch kind (autotuned)
     // FP32 form: tile descriptors per slot, tile work-lists (2+1D, 3+1D), launch counter and error flags
     bool tile;
     vah::TileSlot *d_tdesc;  // [kMaxSlots]
@@ -405,13 +399,11 @@ int cuda_status(cudaError_t e) {
 int nq_of(int physics) { return physics == VAH_IDEAL ? 5 : (physics == VAH_PIMUNU ? 15 : 16); }
 
 // Arrays of one event in its allocation: 16 q, 16 qS, 4 e/p, 4 uA, 4 uB,
-// 4 uS, and the face buffers (H, plus HR for reference faces) per axis; then
-// one byte per cell of fallback flags and one of freeze-out state.
+// 4 uS, and the flux differences per axis; then one byte per cell of fallback flags and one of freeze-out state.
 int arrays_per_event(const vah_batch *b, const vah_lattice *lat) {
     if (b->tile) return 48;  // the tile kernel keeps its face fluxes on chip
     const int ndir = lat->nz > 1 ? 3 : 2;
-    const int per_face = b->opt.flux == VAH_FLUX_PER_CELL ? 2 : 1;
-    return 48 + ndir * b->nq * per_face;
+    return 48 + ndir * b->nq;
 }
 
 // Row pitch of a slot's arrays: nx + 4, padded to 4 floats for the tile form.
@@ -493,10 +485,7 @@ int fill_slot(vah_batch *b, int slot) {
     const int ndir = sl.lat.nz > 1 ? 3 : 2;
     if (!b->tile)
         for (int k = 0; k < ndir; ++k)
-            for (int n = 0; n < b->nq; ++n) {
-                d.H[k][n] = next();
-                if (b->opt.flux == VAH_FLUX_PER_CELL) d.HR[k][n] = next();
-            }
+            for (int n = 0; n < b->nq; ++n) d.D[k][n] = next();
     d.fallback = (unsigned char *)(base + off);
     d.hot = (unsigned char *)(base + off + (ncell + 255) / 256 * 256);
     d.e_freeze = energy_at_temperature(b, sl.hydro.freezeout_T_GeV / 0.197326938);
@@ -593,19 +582,38 @@ int rebuild_work(vah_batch *b) {
         return (long long)l.nx * l.ny * l.nz;
     };
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cells(x) > cells(y); });
+    int seg[vah::K_NUM] = {};  // march segments, from the whole batch's warps
+    for (int kind : {vah::K_FY, vah::K_FZ}) {
+        int longest = 1;
+        for (int s : order) longest = std::max(longest, kind == vah::K_FY ? b->slots[s].lat.ny : b->slots[s].lat.nz);
+        seg[kind] = vah::march_segment(longest, [&](int len) {
+            long long w = 0;
+            for (int s : order) {
+                const vah_lattice &l = b->slots[s].lat;
+                if (kind == vah::K_FZ && l.nz == 1) continue;
+                const long long strips = vah::march_strips(kind == vah::K_FY ? l.nx * l.nz : l.nx * l.ny);
+                const int n = kind == vah::K_FY ? l.ny : l.nz;
+                w += (strips + 3) / 4 * 4 * ((n + len - 1) / len);
+            }
+            return w;
+        });
+    }
     for (int s : order) {
         const vah_batch::Slot &sl = b->slots[s];
         const int nx = sl.lat.nx, ny = sl.lat.ny, nz = sl.lat.nz;
-        auto add = [&](int kind, int ext0, int rows) {
-            for (int r0 = 0; r0 < rows; r0 += vah::kTY)
-                for (int i0 = 0; i0 < ext0; i0 += vah::kTX) lists[kind].push_back({s, i0, r0, 0});
+        auto march = [&](int kind, int strips, int n) {
+            for (int r0 = 0; r0 < n; r0 += seg[kind])
+                for (int i0 = 0; i0 < strips; i0 += vah::kTY)
+                    lists[kind].push_back({s, i0, r0, std::min(r0 + seg[kind], n)});
         };
         if (!b->tile) {
-            add(vah::K_FX, nx + 1, ny * nz);
-            add(vah::K_FY, nx, (ny + 1) * nz);
-            if (nz > 1) add(vah::K_FZ, nx, ny * (nz + 1));
+            const int xs = vah::flux_x_strips(nx, ny, nz);
+            for (int i0 = 0; i0 < xs; i0 += vah::kTY) lists[vah::K_FX].push_back({s, i0, 0, 0});
+            march(vah::K_FY, vah::march_strips(nx * nz), ny);
+            if (nz > 1) march(vah::K_FZ, vah::march_strips(nx * ny), nz);
         }
-        add(nz > 1 ? vah::K_C3 : vah::K_C2, nx, ny * nz);
+        for (int r0 = 0; r0 < ny * nz; r0 += vah::kTY)
+            for (int i0 = 0; i0 < nx; i0 += vah::kTX) lists[nz > 1 ? vah::K_C3 : vah::K_C2].push_back({s, i0, r0, 0});
     }
     for (int k = 0; k < vah::K_NUM; ++k) {
         const int n = (int)lists[k].size();
@@ -631,43 +639,42 @@ int rebuild_work(vah_batch *b) {
     return VAH_OK;
 }
 
-// One launch of a kind known at run time, with the batch's register-cap choice.
-template <typename S, int PHYS, bool EXACT>
-cudaError_t launch_kind_rt(vah_batch *b, const SlotDesc<S> *descs, int kind, int stage, const vah::Eos &eos) {
+// One launch of a kind known at run time.
+template <int PHYS, bool EXACT>
+cudaError_t launch_kind_rt(vah_batch *b, int kind, int stage, const vah::Eos &eos) {
     using namespace vah;
+    const SlotDesc<double> *descs = (const SlotDesc<double> *)b->d_desc;
     const WorkItem *w = b->d_work[kind];
-    const int n = b->nwork[kind], m = b->minb[kind];
+    const int n = b->nwork[kind];
     switch (kind) {
-    case K_FX: return launch_kind<S, PHYS, K_FX, EXACT>(descs, b->d_clk, w, n, stage, eos, b->sms, m, b->d_wcount + kind, b->stream);
-    case K_FY: return launch_kind<S, PHYS, K_FY, EXACT>(descs, b->d_clk, w, n, stage, eos, b->sms, m, b->d_wcount + kind, b->stream);
-    case K_FZ: return launch_kind<S, PHYS, K_FZ, EXACT>(descs, b->d_clk, w, n, stage, eos, b->sms, m, b->d_wcount + kind, b->stream);
-    case K_C2: return launch_kind<S, PHYS, K_C2, EXACT>(descs, b->d_clk, w, n, stage, eos, b->sms, m, b->d_wcount + kind, b->stream);
-    case K_C3: return launch_kind<S, PHYS, K_C3, EXACT>(descs, b->d_clk, w, n, stage, eos, b->sms, m, b->d_wcount + kind, b->stream);
+    case K_FX: return launch_kind<PHYS, K_FX, EXACT>(descs, b->d_clk, w, n, stage, eos, b->sms, b->d_wcount + kind, b->stream);
+    case K_FY: return launch_kind<PHYS, K_FY, EXACT>(descs, b->d_clk, w, n, stage, eos, b->sms, b->d_wcount + kind, b->stream);
+    case K_FZ: return launch_kind<PHYS, K_FZ, EXACT>(descs, b->d_clk, w, n, stage, eos, b->sms, b->d_wcount + kind, b->stream);
+    // the cell kinds read the differences whichever way the faces were evaluated
+    case K_C2: return launch_kind<PHYS, K_C2, true>(descs, b->d_clk, w, n, stage, eos, b->sms, b->d_wcount + kind, b->stream);
+    case K_C3: return launch_kind<PHYS, K_C3, true>(descs, b->d_clk, w, n, stage, eos, b->sms, b->d_wcount + kind, b->stream);
     default: return cudaErrorInvalidValue;
     }
 }
 
-template <typename S, int PHYS, bool EXACT>
+cudaError_t launch_kind_any(vah_batch *b, int kind, int stage, const vah::Eos &eos) {
+    const bool exact = b->opt.flux == VAH_FLUX_PER_CELL;
+    switch (b->opt.physics) {
+    case VAH_IDEAL: return exact ? launch_kind_rt<0, true>(b, kind, stage, eos) : launch_kind_rt<0, false>(b, kind, stage, eos);
+    case VAH_PIMUNU: return exact ? launch_kind_rt<1, true>(b, kind, stage, eos) : launch_kind_rt<1, false>(b, kind, stage, eos);
+    default: return exact ? launch_kind_rt<2, true>(b, kind, stage, eos) : launch_kind_rt<2, false>(b, kind, stage, eos);
+    }
+}
+
 int enqueue_step(vah_batch *b) {
     using namespace vah;
-    const SlotDesc<S> *descs = (const SlotDesc<S> *)b->d_desc;
     const Eos eos = batch_eos(b);
     for (int stage = 1; stage <= 2; ++stage)
-        for (int kind = 0; kind < K_NUM; ++kind) VAH_TRY((launch_kind_rt<S, PHYS, EXACT>(b, descs, kind, stage, eos)));
+        for (int kind = 0; kind < K_NUM; ++kind) VAH_TRY(launch_kind_any(b, kind, stage, eos));
     advance_kernel<<<(kMaxSlots + 255) / 256, 256, 0, b->stream>>>(b->d_clk, b->d_dt, kMaxSlots, b->d_cross, b->d_vol,
                                                                  b->d_dv);
     VAH_TRY(cudaGetLastError());
     return VAH_OK;
-}
-
-template <typename S>
-int enqueue_step_s(vah_batch *b) {
-    const bool exact = b->opt.flux == VAH_FLUX_PER_CELL;
-    switch (b->opt.physics) {
-    case VAH_IDEAL: return exact ? enqueue_step<S, 0, true>(b) : enqueue_step<S, 0, false>(b);
-    case VAH_PIMUNU: return exact ? enqueue_step<S, 1, true>(b) : enqueue_step<S, 1, false>(b);
-    default: return exact ? enqueue_step<S, 2, true>(b) : enqueue_step<S, 2, false>(b);
-    }
 }
 
 // FP32 form: per stage one persistent tile launch per tile shape, then the clocks advance.
@@ -686,8 +693,7 @@ int enqueue_tiles(vah_batch *b) {
 }
 
 int enqueue(vah_batch *b) {
-    if (b->tile) return enqueue_tiles(b);
-    return b->elem == sizeof(float) ? enqueue_step_s<float>(b) : enqueue_step_s<double>(b);
+    return b->tile ? enqueue_tiles(b) : enqueue_step(b);
 }
 
 int capture_graph(vah_batch *b) {
@@ -832,7 +838,6 @@ extern "C" int vah_batch_create(const vah_options *opt, const double *eos_table,
     b->own_stream = opt->stream == nullptr;
     b->capacity = capacity_bytes;
     b->used = 0;
-    for (int k = 0; k < vah::K_NUM; ++k) b->minb[k] = k <= vah::K_FZ ? 4 : 3;  // untuned default
     cudaDeviceGetAttribute(&b->sms, cudaDevAttrMultiProcessorCount, opt->device);
     int rc = VAH_OK;
     auto chk = [&](cudaError_t e) {
@@ -1226,14 +1231,12 @@ extern "C" int vah_batch_kernel_time(vah_batch *b, double *ms, long long *steps)
 
 namespace {
 
-// The batch form of vah_event_autotune: every register-cap variant of each
-// launch kind runs over the whole work-list in stage-1 buffer roles (outputs
-// are stage scratch), the fastest is kept, the per-slot counters are restored
-// and the step graph is re-captured at the next step.
-template <typename S, int PHYS, bool EXACT>
-int batch_autotune_t(vah_batch *b, int reps, vah_tune_report *out) {
+// The batch form of vah_event_autotune: each launch kind has one register cap
+// and a tile fixed by the work-list, so this times it: `reps` launches over the
+// whole work-list in stage-1 buffer roles (outputs are stage scratch); the
+// per-slot counters are restored.
+int batch_autotune(vah_batch *b, int reps, vah_tune_report *out) {
     using namespace vah;
-    const SlotDesc<S> *descs = (const SlotDesc<S> *)b->d_desc;
     const Eos eos = batch_eos(b);
     std::vector<unsigned long long> saved((size_t)kMaxSlots * 4);
     VAH_TRY(cudaStreamSynchronize(b->stream));
@@ -1245,37 +1248,17 @@ int batch_autotune_t(vah_batch *b, int reps, vah_tune_report *out) {
     int rc = VAH_OK;
     out->nkinds = K_NUM;
     for (int kind = 0; kind < K_NUM && rc == VAH_OK; ++kind) {
-        vah_launch_choice &r = out->kind[kind];
-        const int def = b->minb[kind];
-        r = {kTX, kTY, def, 0.0, 0.0};
+        const int minb = kind == K_FX ? kFluxXMinb : (kind <= K_FZ ? kMarchMinb : kCellMinb);
+        out->kind[kind] = {kTX, kTY, minb, 0.0, 0.0};
         if (b->nwork[kind] == 0) continue;
-        const int *cand = kind <= K_FZ ? kFaceMinb : kCellMinb;
-        double best = 1e300;
-        int pick = def;
-        for (int c = 0; c < kNumMinb && rc == VAH_OK; ++c) {
-            b->minb[kind] = cand[c];
-            auto launch = [&]() { return launch_kind_rt<S, PHYS, EXACT>(b, descs, kind, 1, eos); };
-            if (launch() != cudaSuccess || cudaEventRecord(e0, b->stream) != cudaSuccess) {
-                rc = VAH_ERR_CUDA;
-                break;
-            }
-            for (int k = 0; k < reps && rc == VAH_OK; ++k)
-                if (launch() != cudaSuccess) rc = VAH_ERR_CUDA;
-            float f = 0;
-            if (rc != VAH_OK || cudaEventRecord(e1, b->stream) != cudaSuccess ||
-                cudaEventSynchronize(e1) != cudaSuccess || cudaEventElapsedTime(&f, e0, e1) != cudaSuccess) {
-                rc = VAH_ERR_CUDA;
-                break;
-            }
-            const double ms = f / reps;
-            if (cand[c] == def) r.ms_default = ms;
-            if (ms < best) {
-                best = ms;
-                pick = cand[c];
-            }
-        }
-        b->minb[kind] = pick;
-        r = {kTX, kTY, pick, r.ms_default, best};
+        rc = VAH_ERR_CUDA;
+        bool ok = launch_kind_any(b, kind, 1, eos) == cudaSuccess && cudaEventRecord(e0, b->stream) == cudaSuccess;
+        for (int k = 0; k < reps && ok; ++k) ok = launch_kind_any(b, kind, 1, eos) == cudaSuccess;
+        float f = 0;
+        if (ok && cudaEventRecord(e1, b->stream) == cudaSuccess && cudaEventSynchronize(e1) == cudaSuccess &&
+            cudaEventElapsedTime(&f, e0, e1) == cudaSuccess)
+            rc = VAH_OK;
+        out->kind[kind] = {kTX, kTY, minb, f / reps, f / reps};
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -1283,18 +1266,7 @@ int batch_autotune_t(vah_batch *b, int reps, vah_tune_report *out) {
                    cudaMemcpyHostToDevice) != cudaSuccess &&
         rc == VAH_OK)
         rc = VAH_ERR_CUDA;
-    b->dirty = true;  // the step graph holds the old choice
     return rc;
-}
-
-template <typename S>
-int batch_autotune_s(vah_batch *b, int reps, vah_tune_report *out) {
-    const bool exact = b->opt.flux == VAH_FLUX_PER_CELL;
-    switch (b->opt.physics) {
-    case VAH_IDEAL: return exact ? batch_autotune_t<S, 0, true>(b, reps, out) : batch_autotune_t<S, 0, false>(b, reps, out);
-    case VAH_PIMUNU: return exact ? batch_autotune_t<S, 1, true>(b, reps, out) : batch_autotune_t<S, 1, false>(b, reps, out);
-    default: return exact ? batch_autotune_t<S, 2, true>(b, reps, out) : batch_autotune_t<S, 2, false>(b, reps, out);
-    }
 }
 
 }  // namespace
@@ -1308,5 +1280,5 @@ extern "C" int vah_batch_autotune(vah_batch *b, int reps, vah_tune_report *out) 
         const int rc = rebuild_work(b);
         if (rc != VAH_OK) return rc;
     }
-    return b->elem == sizeof(float) ? batch_autotune_s<float>(b, reps, out) : batch_autotune_s<double>(b, reps, out);
+    return batch_autotune(b, reps, out);
 }

@@ -12,14 +12,18 @@ namespace vah {
 template <typename S>
 cudaError_t launch_stage(const StageArgs<S> &a, int physics, cudaStream_t stream);
 
-// ---- face/cell split: launch kinds and their tunable launch configuration --
-// Kinds of launch in one split stage: the face launches per axis, then the
-// cell launch. Each has a block shape (bx x by = kSplitThreads threads, x
-// fastest) and a register-cap variant minb: the compiler must fit minb
-// resident blocks per SM, i.e. at most 65536 / (128 minb) registers per
-// thread (face: 3, 4, 5 -> 168, 128, 96-102; cell: 2, 3, 4 -> 255, 168, 128).
+// ---- flux/cell split: launch kinds and their tunable launch configuration --
+// Kinds of launch in one split stage: the flux launches per axis, then the
+// cell launch, all of 128-thread blocks. Each kind has one register cap: at
+// least minb resident blocks per SM, the fastest of its candidates on the
+// 121x121x81 event (x fluxes: 96 registers without spills, 105 us against 117
+// at 4 blocks; marches: 120 registers, 105 us against 152 at 5 blocks, which
+// spill; cell: 168 registers, 315 us). The cell launch's block shape bx x by
+// (x fastest) is the autotuner's choice; the flux launches' warps index
+// themselves.
 enum SplitKind { kFaceX = 0, kFaceY = 1, kFaceZ = 2, kCell = 3, kNumSplitKinds = 4 };
 constexpr int kSplitThreads = 128;
+constexpr int kFluxXMinb = 5, kMarchMinb = 4, kCellMinb = 3;
 
 struct KindConfig {
     int bx, by, minb;
@@ -28,45 +32,61 @@ struct SplitConfig {
     KindConfig k[kNumSplitKinds];
 };
 
-// The autotuner's search space per kind (block shapes x register caps).
 constexpr int kNumShapes = 2;
 constexpr int kShapes[kNumShapes][2] = {{32, 4}, {64, 2}};
-constexpr int kNumMinb = 3;
-constexpr int kFaceMinb[kNumMinb] = {3, 4, 5};
-constexpr int kCellMinb[kNumMinb] = {2, 3, 4};
-
-inline bool valid_kind_config(int kind, const KindConfig &c) {
-    if (kind < 0 || kind >= kNumSplitKinds || c.bx * c.by != kSplitThreads) return false;
-    bool shape = false, minb = false;
-    for (int s = 0; s < kNumShapes; ++s) shape |= c.bx == kShapes[s][0] && c.by == kShapes[s][1];
-    for (int m = 0; m < kNumMinb; ++m) minb |= c.minb == (kind == kCell ? kCellMinb[m] : kFaceMinb[m]);
-    return shape && minb;
-}
 
 // Candidates of one kind, in a fixed order; returns their number.
 inline int split_candidates(int kind, KindConfig *out, int max) {
+    const int minb = kind == kCell ? kCellMinb : (kind == kFaceX ? kFluxXMinb : kMarchMinb);
     int n = 0;
-    for (int s = 0; s < kNumShapes; ++s)
-        for (int m = 0; m < kNumMinb; ++m)
-            if (n < max) out[n++] = {kShapes[s][0], kShapes[s][1], kind == kCell ? kCellMinb[m] : kFaceMinb[m]};
+    for (int s = 0; s < (kind == kCell ? kNumShapes : 1); ++s)
+        if (n < max) out[n++] = {kShapes[s][0], kShapes[s][1], minb};
     return n;
 }
 
-// Untuned default: the best of the candidates on the 121x121x81 shear+bulk
-// table-EoS event (faces capped at 128 registers, cells at 168).
+inline bool valid_kind_config(int kind, const KindConfig &c) {
+    if (kind < 0 || kind >= kNumSplitKinds) return false;
+    KindConfig ok[kNumShapes];
+    const int n = split_candidates(kind, ok, kNumShapes);
+    for (int k = 0; k < n; ++k)
+        if (ok[k].bx == c.bx && ok[k].by == c.by && ok[k].minb == c.minb) return true;
+    return false;
+}
+
+// Untuned default.
 inline SplitConfig default_split_config() {
     SplitConfig c;
-    for (int k = 0; k < kNumSplitKinds; ++k) c.k[k] = {32, 4, k == kCell ? 3 : 4};
+    for (int k = 0; k < kNumSplitKinds; ++k) split_candidates(k, &c.k[k], 1);
     return c;
 }
 
-// One launch of one split kind (a.H, and a.HR when exact, must point at the
-// face buffers). exact = the reference's per-cell face evaluation.
+// Cells per march segment along an axis of n cells, from the number of warps
+// a segment length makes: the fewest waves (148 SMs x 5 blocks x 4 warps)
+// times the segment's length plus its start-up (one face and its first
+// loads, about 1.5 cells' work).
+template <typename Warps>
+inline int march_segment(int n, Warps warps) {
+    constexpr long long wave = 148 * kMarchMinb * 4;
+    int best = 1;
+    double cost = 1e300;
+    for (int parts = 1; parts <= n; ++parts) {
+        const int len = (n + parts - 1) / parts;
+        const double c = (double)((warps(len) + wave - 1) / wave) * (len + 1.5);
+        if (c < cost) {
+            cost = c;
+            best = len;
+        }
+    }
+    return best;
+}
+
+// One launch of one split kind (a.D must point at the difference buffers).
+// exact = the reference's per-cell face evaluation.
 template <typename S>
 cudaError_t launch_split_kind(const StageArgs<S> &a, int physics, bool exact, int kind, const KindConfig &c,
                               cudaStream_t stream);
 
-// One RK stage on the face/cell split: face launches (x, y[, z]) then the
+// One RK stage on the flux/cell split: flux launches (x, y[, z]) then the
 // cell launch, with the given (or the default) launch configuration.
 template <typename S>
 cudaError_t launch_stage_split(const StageArgs<S> &a, int physics, bool exact, const SplitConfig &c,

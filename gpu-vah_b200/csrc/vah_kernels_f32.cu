@@ -1,6 +1,6 @@
-// vah_kernels_f32.cu -- the step kernels with FP32 state storage (FP64 arithmetic).
+// vah_kernels_f32.cu -- the set-up and validity kernels with FP32 state storage.
 #include "vah_kernels_impl.cuh"
 
 namespace vah {
-VAH_INSTANTIATE(float)
+VAH_INSTANTIATE_SETUP(float)
 }  // namespace vah

@@ -3,18 +3,15 @@
 // and vah_kernels_f32.cu (separate translation units build in parallel).
 //
 // stage_kernel: one thread per interior cell runs the whole RK stage of that
-// cell (vah_stage.cuh). face_kernel + cell_kernel: the same stage split into
-// per-axis face launches and one cell launch (the default path).
-// The step is FP64-arithmetic-bound (13 Newton inversions per cell and stage
-// in the reference-faithful flux mode), so launches favour occupancy:
-// 128-thread blocks, x fastest so that every load of a field is a coalesced
-// row. The split kernels come in register-cap variants (MINB = the minimum
-// number of resident 128-thread blocks per SM the compiler must allow) and
-// take their block shape at run time; the autotuner picks both per launch
-// kind by timing them on the event's own state.
+// cell (vah_stage.cuh). flux_x_kernel + flux_march_kernel + cell_kernel: the
+// same stage split into per-axis flux launches (vah_march.cuh) and one cell
+// launch (the default path). 128-thread blocks, x fastest so that every load
+// of a field is a coalesced row. The cell kernel takes its block shape at run
+// time; the autotuner picks it by timing on the event's own state.
 #pragma once
 
 #include "vah_kernels.cuh"
+#include "vah_march.cuh"
 
 namespace vah {
 
@@ -42,89 +39,34 @@ __global__ void __launch_bounds__(kBX *kBY) stage_kernel(const StageArgs<S> a) {
     stage_cell<S, PHYS, IS3D>(a, i + 2, j + 2, k + 2);
 }
 
-// Faces at +1/2 of the ghosted cells along DIR that bound an interior cell
-// of the planes [k0, k1): left cell index 1 .. n along DIR (ghost layer 1
-// included), interior across.
-template <typename S, int PHYS, int DIR, bool EXACT, int MINB>
-__global__ void __launch_bounds__(kSplitThreads, MINB) face_kernel(const StageArgs<S> a) {
-    const int ext0 = DIR == 0 ? a.nx + 1 : a.nx;
-    const int ext1 = DIR == 1 ? a.ny + 1 : a.ny;
-    const int ext2 = DIR == 2 ? a.k1 - a.k0 + 1 : a.k1 - a.k0;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int r = row_block() * blockDim.y + threadIdx.y;
-    if (i >= ext0 || r >= ext1 * ext2) return;
-    const int j = r % ext1, k = r / ext1 + a.k0;
-    const int gi = i + (DIR == 0 ? 1 : 2), gj = j + (DIR == 1 ? 1 : 2), gk = k + (DIR == 2 ? 1 : 2);
-    const long long st = DIR == 0 ? 1 : (DIR == 1 ? (long long)a.ncx : a.plane);
-    const long long s = gi + (long long)a.ncx * gj + a.plane * gk;
-    const int gl = DIR == 0 ? gi : (DIR == 1 ? gj : gk), n = DIR == 0 ? a.nx : (DIR == 1 ? a.ny : a.nz);
-    const unsigned fails = face_compute<S, PHYS, EXACT>(a, s, DIR, st, gl >= 2, gl <= n);
-    if (a.counters) {
-        if (fails & 255u) count_add(a.counters + 0, fails & 255u);
-        if (fails >> 8) count_add(a.counters + 2, 1ull);
-    }
+// The x flux differences of the planes [k0, k1): a warp per strip.
+template <int PHYS, bool EXACT>
+__global__ void __launch_bounds__(kSplitThreads, kFluxXMinb) flux_x_kernel(const StageArgs<double> a, int strips) {
+    __shared__ HalfPointers hp;
+    set_half_pointers<PHYS>(hp, a, threadIdx.x);
+    __syncthreads();
+    const int strip = blockIdx.x * (kSplitThreads / 32) + threadIdx.x / 32;
+    if (strip < strips) flux_x<PHYS, EXACT>(a, hp, strip);
 }
 
-// Faces along x with the x flux differences taken in the launch (a.Dx set):
-// blocks of 32 x 4 threads, one warp per row segment. Lane L of warp w in its
-// row takes the face at +1/2 of ghosted cell f + 1, f = 31 w + L, so that
-// consecutive warps share one face. Each face is evaluated as in face_kernel,
-// but only the two evaluations' weights are kept, and each field's two fluxes
-// are formed at the exchange: lane L >= 1 owns cell f + 1 (when interior) and
-// writes Dx = H(-1/2) - H(+1/2) as that cell evaluates them, the -1/2 value
-// from lane L - 1 through a shuffle. The face a warp shares with the previous
-// one is evaluated twice and counted once.
-template <typename S, int PHYS, bool EXACT, int MINB>
-__global__ void __launch_bounds__(kSplitThreads, MINB) face_x_diff_kernel(const StageArgs<S> a) {
-    constexpr int NQ = Phys<PHYS>::NQ;
-    const int lane = threadIdx.x;  // blockDim.x == 32: a warp is one row segment
-    const int r = row_block() * blockDim.y + threadIdx.y;
-    if (r >= a.ny * (a.k1 - a.k0)) return;  // whole warps
-    const int j = r % a.ny, k = r / a.ny + a.k0;
-    const int gi = 31 * blockIdx.x + lane + 1;  // the face at +1/2 of ghosted cell gi
-    const bool act = gi <= a.nx + 1;            // faces 1 .. nx + 1 bound the interior cells
-    const long long s = gi + (long long)a.ncx * (j + 2) + a.plane * (k + 2);
-    double qR[NQ], qL[NQ];
-    double wRo = 0.0, wLo = 0.0, wRr = 0.0, wLr = 0.0;  // the left cell's evaluation, the right cell's
-    unsigned fails = 0;
-    if (act) {
-        face_states<S, PHYS>(a, s, 1, qR, qL);
-        InvSetup sR, sL;
-        invert_setup<PHYS>(a.t_src, qR, sR);
-        invert_setup<PHYS>(a.t_src, qL, sL);
-        if (!EXACT || gi >= 2) {
-            const double ux = ld(a.uin[1], s), uy = ld(a.uin[2], s);
-            fails += face_weights(sR, sL, 0, ld(a.ein, s), sqrt(fabs(ux * ux + uy * uy)), wRo, wLo);
-        }
-        if (EXACT && gi <= a.nx) {
-            const double vx = ld(a.uin[1], s + 1), vy = ld(a.uin[2], s + 1);
-            fails += face_weights(sR, sL, 0, ld(a.ein, s + 1), sqrt(fabs(vx * vx + vy * vy)), wRr, wLr);
-        }
-    } else {
-#pragma unroll
-        for (int n = 0; n < NQ; ++n) qR[n] = qL[n] = 0.0;
-    }
-    const bool own = act && lane >= 1 && gi >= 2;  // cell gi is interior, and lane - 1 holds its -1/2 face
-#pragma unroll
-    for (int n = 0; n < NQ; ++n) {
-        const double h = wRo * qR[n] + wLo * qL[n];                 // +1/2 as cell gi evaluates it
-        const double hr = EXACT ? wRr * qR[n] + wLr * qL[n] : h;   // +1/2 as cell gi + 1 evaluates it
-        const double hm = __shfl_up_sync(0xffffffffu, hr, 1);
-        if (own) a.Dx[n][s] = (S)(hm - h);
-    }
-    if (a.counters && act && (lane >= 1 || blockIdx.x == 0)) {
-        if (fails & 255u) count_add(a.counters + 0, fails & 255u);
-        if (fails >> 8) count_add(a.counters + 2, 1ull);
-    }
+// The y or eta flux differences: a warp per strip and segment of `seg` cells.
+template <int PHYS, int DIR, bool EXACT>
+__global__ void __launch_bounds__(kSplitThreads, kMarchMinb) flux_march_kernel(const StageArgs<double> a, int strips, int seg) {
+    extern __shared__ double march_sm[];
+    const int lo = DIR == 1 ? 0 : a.k0, hi = DIR == 1 ? a.ny : a.k1;
+    const int w = blockIdx.x * (kSplitThreads / 32) + threadIdx.x / 32;
+    const int part = w / strips, m0 = lo + part * seg;
+    if (m0 >= hi) return;
+    flux_march<PHYS, DIR, EXACT>(a, HalfSelect<PHYS>{a}, w - part * strips, m0, min(m0 + seg, hi), march_sm + (threadIdx.x / 32) * kMarchDoubles<PHYS>);
 }
 
-template <typename S, int PHYS, bool IS3D, bool EXACT, int MINB>
-__global__ void __launch_bounds__(kSplitThreads, MINB) cell_kernel(const StageArgs<S> a) {
+template <int PHYS, bool IS3D>
+__global__ void __launch_bounds__(kSplitThreads, kCellMinb) cell_kernel(const StageArgs<double> a) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int r = row_block() * blockDim.y + threadIdx.y;
     if (i >= a.nx || r >= a.ny * (a.k1 - a.k0)) return;
     const int j = r % a.ny, k = r / a.ny + a.k0;
-    cell_compute<S, PHYS, IS3D, EXACT>(a, i + 2, j + 2, k + 2);
+    cell_compute<double, PHYS, IS3D, true>(a, i + 2, j + 2, k + 2);
 }
 
 template <typename S, int PHYS>
@@ -208,58 +150,43 @@ cudaError_t stage_dispatch(const StageArgs<S> &a, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
-// One launch of a split kernel kind with the given shape and register-cap variant.
-template <typename S, int PHYS, bool EXACT, int DIR>
-cudaError_t face_launch(const StageArgs<S> &a, const KindConfig &c, cudaStream_t stream) {
-    const int ext0 = DIR == 0 ? a.nx + 1 : a.nx;
-    const int rows = (DIR == 1 ? a.ny + 1 : a.ny) * (DIR == 2 ? a.k1 - a.k0 + 1 : a.k1 - a.k0);
-    const dim3 block(c.bx, c.by), grid = row_grid(ext0, rows, c.bx, c.by);
-    switch (c.minb) {
-    case 3: face_kernel<S, PHYS, DIR, EXACT, 3><<<grid, block, 0, stream>>>(a); break;
-    case 4: face_kernel<S, PHYS, DIR, EXACT, 4><<<grid, block, 0, stream>>>(a); break;
-    case 5: face_kernel<S, PHYS, DIR, EXACT, 5><<<grid, block, 0, stream>>>(a); break;
-    default: return cudaErrorInvalidValue;
-    }
+template <int PHYS, bool EXACT>
+cudaError_t flux_x_launch(const StageArgs<double> &a, cudaStream_t stream) {
+    const int strips = flux_x_strips(a.nx, a.ny, a.k1 - a.k0);
+    flux_x_kernel<PHYS, EXACT><<<(strips + 3) / 4, kSplitThreads, 0, stream>>>(a, strips);
     return cudaGetLastError();
 }
 
-// The x face launch that also differences (a.Dx set): 32 x 4 blocks whatever
-// the tuned shape (a warp must be one row segment); the register cap as tuned.
-template <typename S, int PHYS, bool EXACT>
-cudaError_t face_x_diff_launch(const StageArgs<S> &a, const KindConfig &c, cudaStream_t stream) {
-    const int rows = a.ny * (a.k1 - a.k0);
-    const dim3 block(32, kSplitThreads / 32), grid = row_grid((a.nx + 30) / 31, rows, 1, kSplitThreads / 32);
-    switch (c.minb) {
-    case 3: face_x_diff_kernel<S, PHYS, EXACT, 3><<<grid, block, 0, stream>>>(a); break;
-    case 4: face_x_diff_kernel<S, PHYS, EXACT, 4><<<grid, block, 0, stream>>>(a); break;
-    case 5: face_x_diff_kernel<S, PHYS, EXACT, 5><<<grid, block, 0, stream>>>(a); break;
-    default: return cudaErrorInvalidValue;
-    }
+template <int PHYS, bool EXACT, int DIR>
+cudaError_t flux_march_launch(const StageArgs<double> &a, cudaStream_t stream) {
+    constexpr size_t smem = kSplitThreads / 32 * kMarchDoubles<PHYS> * sizeof(double);
+    auto kernel = flux_march_kernel<PHYS, DIR, EXACT>;
+    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    const int n = DIR == 1 ? a.ny : a.k1 - a.k0;
+    const int strips = march_strips(DIR == 1 ? a.nx * (a.k1 - a.k0) : a.nx * a.ny);
+    const int seg = march_segment(n, [&](int len) { return (long long)strips * ((n + len - 1) / len); });
+    const int warps = strips * ((n + seg - 1) / seg);
+    kernel<<<(warps + 3) / 4, kSplitThreads, smem, stream>>>(a, strips, seg);
     return cudaGetLastError();
 }
 
-template <typename S, int PHYS, bool EXACT, bool IS3D>
-cudaError_t cell_launch(const StageArgs<S> &a, const KindConfig &c, cudaStream_t stream) {
+template <int PHYS, bool IS3D>
+cudaError_t cell_launch(const StageArgs<double> &a, const KindConfig &c, cudaStream_t stream) {
     const dim3 block(c.bx, c.by), grid = row_grid(a.nx, (long long)a.ny * (a.k1 - a.k0), c.bx, c.by);
-    switch (c.minb) {
-    case 2: cell_kernel<S, PHYS, IS3D, EXACT, 2><<<grid, block, 0, stream>>>(a); break;
-    case 3: cell_kernel<S, PHYS, IS3D, EXACT, 3><<<grid, block, 0, stream>>>(a); break;
-    case 4: cell_kernel<S, PHYS, IS3D, EXACT, 4><<<grid, block, 0, stream>>>(a); break;
-    default: return cudaErrorInvalidValue;
-    }
+    cell_kernel<PHYS, IS3D><<<grid, block, 0, stream>>>(a);
     return cudaGetLastError();
 }
 
-template <typename S, int PHYS, bool EXACT>
-cudaError_t split_kind_dispatch(const StageArgs<S> &a, int kind, const KindConfig &c, cudaStream_t stream) {
+template <int PHYS, bool EXACT>
+cudaError_t split_kind_dispatch(const StageArgs<double> &a, int kind, const KindConfig &c, cudaStream_t stream) {
     if (a.k0 < 0 || a.k1 > a.nz || a.k0 > a.k1) return cudaErrorInvalidValue;
     if (a.k0 == a.k1) return cudaSuccess;  // no planes
     switch (kind) {
-    case kFaceX: return a.Dx[0] ? face_x_diff_launch<S, PHYS, EXACT>(a, c, stream) : face_launch<S, PHYS, EXACT, 0>(a, c, stream);
-    case kFaceY: return face_launch<S, PHYS, EXACT, 1>(a, c, stream);
-    case kFaceZ: return a.nz > 1 ? face_launch<S, PHYS, EXACT, 2>(a, c, stream) : cudaSuccess;
-    case kCell:
-        return a.nz > 1 ? cell_launch<S, PHYS, EXACT, true>(a, c, stream) : cell_launch<S, PHYS, EXACT, false>(a, c, stream);
+    case kFaceX: return flux_x_launch<PHYS, EXACT>(a, stream);
+    case kFaceY: return flux_march_launch<PHYS, EXACT, 1>(a, stream);
+    case kFaceZ: return a.nz > 1 ? flux_march_launch<PHYS, EXACT, 2>(a, stream) : cudaSuccess;
+    case kCell: return a.nz > 1 ? cell_launch<PHYS, true>(a, c, stream) : cell_launch<PHYS, false>(a, c, stream);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -289,14 +216,14 @@ cudaError_t launch_split_kind(const StageArgs<S> &a, int physics, bool exact, in
     if (!valid_kind_config(kind, c)) return cudaErrorInvalidValue;
     switch (physics) {
     case kIdeal:
-        return exact ? split_kind_dispatch<S, kIdeal, true>(a, kind, c, stream)
-                     : split_kind_dispatch<S, kIdeal, false>(a, kind, c, stream);
+        return exact ? split_kind_dispatch<kIdeal, true>(a, kind, c, stream)
+                     : split_kind_dispatch<kIdeal, false>(a, kind, c, stream);
     case kPimunu:
-        return exact ? split_kind_dispatch<S, kPimunu, true>(a, kind, c, stream)
-                     : split_kind_dispatch<S, kPimunu, false>(a, kind, c, stream);
+        return exact ? split_kind_dispatch<kPimunu, true>(a, kind, c, stream)
+                     : split_kind_dispatch<kPimunu, false>(a, kind, c, stream);
     case kPimunuPi:
-        return exact ? split_kind_dispatch<S, kPimunuPi, true>(a, kind, c, stream)
-                     : split_kind_dispatch<S, kPimunuPi, false>(a, kind, c, stream);
+        return exact ? split_kind_dispatch<kPimunuPi, true>(a, kind, c, stream)
+                     : split_kind_dispatch<kPimunuPi, false>(a, kind, c, stream);
     default: return cudaErrorInvalidValue;
     }
 }
@@ -379,19 +306,22 @@ cudaError_t launch_ghost_pass(const FieldSet<S> &fields, int nx, int ny, int nz,
     return cudaGetLastError();
 }
 
-#define VAH_INSTANTIATE(S)                                                                                      \
-    template cudaError_t launch_stage<S>(const StageArgs<S> &, int, cudaStream_t);                              \
+// The set-up launches and the validity diagnostics serve both storage types;
+// the stage launches are FP64 (the FP32 form has the tile kernel).
+#define VAH_INSTANTIATE_SETUP(S)                                                                                \
     template cudaError_t launch_validity<S>(const ValidityArgs<S> &, int, cudaStream_t);                        \
-    template cudaError_t launch_split_kind<S>(const StageArgs<S> &, int, bool, int, const KindConfig &,         \
-                                              cudaStream_t);                                                    \
-    template cudaError_t launch_stage_split<S>(const StageArgs<S> &, int, bool, const SplitConfig &,            \
-                                               cudaStream_t);                                                   \
-    template cudaError_t launch_stage_split<S>(const StageArgs<S> &, int, bool, cudaStream_t);                  \
     template cudaError_t launch_set_conserved<S>(const FieldSet<S> &, const FieldSet<S> &, const FieldSet<S> &, \
                                                  const S *, int, int, int, int, int, double, int, cudaStream_t); \
     template cudaError_t launch_init_primitives<S>(const FieldSet<S> &, const FieldSet<S> &, const S *, S *,    \
                                                    const Eos &, int, int, int, int, cudaStream_t);             \
     template cudaError_t launch_ghosts<S>(const FieldSet<S> &, int, int, int, int, cudaStream_t);              \
     template cudaError_t launch_ghost_pass<S>(const FieldSet<S> &, int, int, int, int, int, cudaStream_t);
+#define VAH_INSTANTIATE_STAGE(S)                                                                                \
+    template cudaError_t launch_stage<S>(const StageArgs<S> &, int, cudaStream_t);                              \
+    template cudaError_t launch_split_kind<S>(const StageArgs<S> &, int, bool, int, const KindConfig &,         \
+                                              cudaStream_t);                                                    \
+    template cudaError_t launch_stage_split<S>(const StageArgs<S> &, int, bool, const SplitConfig &,            \
+                                               cudaStream_t);                                                   \
+    template cudaError_t launch_stage_split<S>(const StageArgs<S> &, int, bool, cudaStream_t);
 
 }  // namespace vah

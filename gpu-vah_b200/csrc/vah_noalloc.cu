@@ -164,12 +164,9 @@ extern "C" int vah_stage_noalloc(const vah_lattice *lat, double eta_over_s, int 
     a.eout = buf->e_out;
     a.pout = buf->p_out;
     a.counters = (unsigned long long *)base;
-    double *faces = (double *)(base + kCounterBytes);
+    double *diffs = (double *)(base + kCounterBytes);
     for (int d = 0; d < ndir; ++d)
-        for (int n = 0; n < nq; ++n) {
-            a.H[d][n] = faces + ((size_t)(d * nq + n) * 2) * ncell;
-            a.HR[d][n] = faces + ((size_t)(d * nq + n) * 2 + 1) * ncell;
-        }
+        for (int n = 0; n < nq; ++n) a.D[d][n] = diffs + (size_t)(d * nq + n) * ncell;
 
     vah::finish_args(a);
     if (cudaMemsetAsync(base, 0, kCounterBytes, s) != cudaSuccess) return VAH_ERR_CUDA;

@@ -14,8 +14,10 @@
 
 #ifdef __CUDACC__
 #define VAH_HD __host__ __device__ __forceinline__
+#define VAH_COLD __host__ __device__ __forceinline__
 #else
 #define VAH_HD inline
+#define VAH_COLD inline
 #endif
 
 namespace vah {
@@ -40,12 +42,6 @@ VAH_HD double quotient_fast(double f, double d) {
     return f / d;
 #endif
 }
-
-}  // namespace vah
-
-#include "vah_closure_polys.h"
-
-namespace vah {
 
 constexpr int kIdeal = 0, kPimunu = 1, kPimunuPi = 2;
 
@@ -95,6 +91,58 @@ VAH_HD float rsqrt_r(float x) {
     return 1.0f / sqrtf(x);
 #endif
 }
+
+// 1/d and f/d to rounding level for d of ordinary magnitude. On the device: the
+// hardware reciprocal estimate (about 2^-20) refined by two Newton-Raphson
+// steps y += y (1 - d y), and for the quotient one residual correction
+// q += y (f - d q); outside |d| in [2^-1000, 2^1001), where the estimate
+// flushes or overflows, the IEEE quotient. On the host: IEEE.
+VAH_HD double recip_d(double d) {
+#ifdef __CUDA_ARCH__
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(d));
+    y = fma(y, fma(-d, y, 1.0), y);
+    y = fma(y, fma(-d, y, 1.0), y);
+    return y;
+#else
+    return 1.0 / d;
+#endif
+}
+VAH_HD double quotient_d(double f, double d) {
+#ifdef __CUDA_ARCH__
+    const unsigned biased = ((unsigned)__double2hiint(d) >> 20) & 0x7ffu;
+    if (biased - 23u > 2000u) return f / d;
+    const double y = recip_d(d), q = f * y;
+    return fma(y, fma(-d, q, f), q);
+#else
+    return f / d;
+#endif
+}
+
+// sqrt(x) for the root's admission tests only: on the device the hardware
+// 1/sqrt estimate times x (about 1e-6 relative); 0 for x = 0.
+VAH_HD double sqrt_estimate(double x) {
+#ifdef __CUDA_ARCH__
+    double y;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(x));
+    return x > 0.0 ? x * y : 0.0;
+#else
+    return sqrt(x);
+#endif
+}
+
+// f / d in the arithmetic type of the caller; and with 1/d at hand: the FP64
+// form multiplies, the FP32 form keeps the quotient's single rounding.
+VAH_HD double quot(double f, double d) { return quotient_d(f, d); }
+VAH_HD float quot(float f, float d) { return f / d; }
+VAH_HD double quot(double f, double, double inv_d) { return f * inv_d; }
+VAH_HD float quot(float f, float d, float) { return f / d; }
+
+}  // namespace vah
+
+#include "vah_closure_polys.h"
+
+namespace vah {
 
 VAH_HD uint32_t float_bits(float x) {
 #ifdef __CUDA_ARCH__
@@ -244,6 +292,17 @@ VAH_HD R zeta_over_s(const Eos &eos, R T) {
     return -R(13.77) * x * x + R(27.55) * x - R(13.45);
 }
 
+// x / (zeta/s): in FP64 the crossover's Lorentzian inverted without a division.
+VAH_HD double over_zeta(const Eos &eos, double T, double x) {
+    if (eos.zeta == 1) {
+        constexpr double tp = 0.155 / kHbarc, inv_w = kHbarc / 0.050;
+        const double d = (T - tp) * inv_w;
+        return x * ((1.0 / 0.05) * (1.0 + d * d));
+    }
+    return x / zeta_over_s(eos, T);
+}
+VAH_HD float over_zeta(const Eos &eos, float T, float x) { return x / zeta_over_s(eos, T); }
+
 // --------------------------------------------------------------- limiter --
 // FluxLimiter.cpp:28-33, theta = 1.1: minmod(l, minmod(c, r)) with
 // minmod(x, y) = (sign x + sign y) min(|x|,|y|) / 2, sign(0) = +1
@@ -280,18 +339,19 @@ struct InvSetup {
     double G0, G1;
 };
 
-template <int PHYS, bool FAST = false>
-VAH_HD void invert_setup(double t, const double *q, InvSetup &s) {
-    double pitt = 0, pitx = 0, pity = 0, pitn = 0, bulk = 0;
-    if (Phys<PHYS>::PIMUNU) {
-        pitt = q[5];
-        pitx = q[6];
-        pity = q[7];
-        pitn = q[8];
-    }
-    if (Phys<PHYS>::BULK) bulk = q[kSlotPi];
-    const double pl = q[kSlotPL];
-    const double m0 = q[0] - pitt, m1 = q[1] - pitx, m2 = q[2] - pity, m3 = q[3] - pitn;
+// What an inversion takes from a state: m = T^{tau mu} - pi^{tau mu}, P_L, Pi.
+struct InvIn {
+    double m0, m1, m2, m3, pl, bulk;
+};
+template <int PHYS>
+VAH_HD InvIn inv_in(const double *q) {
+    if (!Phys<PHYS>::PIMUNU) return {q[0], q[1], q[2], q[3], q[kSlotPL], 0.0};
+    return {q[0] - q[5], q[1] - q[6], q[2] - q[7], q[3] - q[8], q[kSlotPL], Phys<PHYS>::BULK ? q[kSlotPi] : 0.0};
+}
+
+template <bool FAST = false>
+VAH_HD void invert_setup(double t, const InvIn &q, InvSetup &s) {
+    const double m0 = q.m0, m1 = q.m1, m2 = q.m2, m3 = q.m3, pl = q.pl, bulk = q.bulk;
     double m0pl = m0 + pl;
     if (m0pl == 0.0) m0pl = 1.e-16;
     const double F = FAST ? quotient_fast(m3, m0pl) : m3 / m0pl;  // W off: F = A
@@ -349,77 +409,139 @@ VAH_HD int newton_uT(const InvSetup &s, double uT0, double &uT) {
     return 1;
 }
 
-// One Newton iteration from w, straight-line (the exits are tested after the
-// arithmetic, so that two independent iterations can be interleaved by the
-// scheduler): 0 = converged to next, 1 = the reference falls back, 2 = go on
-// from next. The same operations as newton_uT's loop body.
-VAH_HD int newton_step(const InvSetup &s, double w, double &next) {
-    const double w2 = 1 + w * w;
-    const double r = rsqrt_d(w2);
-    const double v = w * r;
-    const double e = s.c0 - v * s.x * s.mbt;  // the reference's energy, for its exit test
-    const double g = s.G0 - s.G1 * v;          // bL + b (0.5 (e - pl) + 1.5 Pi), one operation after v
-    const double r3 = r * r * r;
-    const double f = v * g - s.bT;
-    double fp = r3 * (s.G0 - 2 * s.G1 * v);   // r3 g + v b (0.5 (-bT r3))
-    if (fabs(fp) == 0.0) fp = 1.e-16;
-    next = w - newton_correction(f, fp);
-    if (e < 0.0) return 1;
-    if (!(next >= 0.0 && next <= 9.0072e+15)) return 1;  // NaN, +-inf, negative or too large
-    return fabs(next - w) <= 1.e-7 * fabs(next) ? 0 : 2;
+// -------------------------------------------- the root without iterating --
+// With the closure P_T = (e - P_L)/2 + 3/2 Pi the equation Newton's iteration
+// solves is a quadratic in v = u_T / sqrt(1 + u_T^2):
+//   f(v) = v (G0 - G1 v) - bT = 0,  G1 = b bT / 2,
+// whose smaller root is v = 2 bT / (G0 + sqrt(G0^2 - 2 b bT^2)), bT = x |m_T|.
+// Neither x nor |m_T| is needed by itself: v^x = v m1 x / |m_T| =
+// 2 x^2 m1 / (G0 + sqrt(G0^2 - 2 b x^2 m_T^2)).
+// The iteration's answer is this root, up to its stopping error (the square
+// of its 1e-7 tolerance), or the reference's fallback; which of the two
+// follows without running it: in w = u_T >= 0 the function f(v(w)) is concave
+// and increasing while v < G0 / (2 G1). From a guess below the root the
+// iterates increase to it; from one above, the first step lands at or below
+// the root, so the iteration goes on from there unless that step is negative
+// (a fallback). The energy e = c0 - v bT falls with v, so its test e < 0 can
+// only fire at the guess or beyond the root. InvRoot admits a state when the
+// root is well inside this picture (margins far above rounding), and
+// newton_reaches tests a guess; everything else runs the iteration itself,
+// so every fallback decision near a boundary is the iteration's own.
+// Cost: one square root, two quotients per state and a few products per
+// guess, instead of 3-4 iterations of a square root and a quotient per state
+// and guess, one after the other.
+// (Products and sums that could contract either way are written as fma, so that
+// every compiled variant of a kernel rounds them alike.)
+struct InvRoot {
+    double F, x2, c0, inv;  // inv = 1 / (G0 + sqrt(G0^2 - 2 b bT^2)); v^x = 2 x2 inv m1
+    double G0, G1, bT, s2;  // s2 = v bT, so e = c0 - s2; G0 = NaN: not admitted
+};
+
+template <bool FAST = false>
+VAH_HD void invert_root(double t, const InvIn &q, InvRoot &r) {
+    const double m0 = q.m0, m1 = q.m1, m2 = q.m2, m3 = q.m3, pl = q.pl, bulk = q.bulk;
+    double m0pl = m0 + pl;
+    if (m0pl == 0.0) m0pl = 1.e-16;
+    r.F = FAST ? quotient_fast(m3, m0pl) : quotient_d(m3, m0pl);
+    const double Ft = t * r.F;
+    const double Ft2 = Ft * Ft;
+    r.x2 = fabs(fma(-Ft, Ft, 1.));
+    const double b = r.x2 + Ft2;
+    r.c0 = fma(-(t * Ft), m3, m0);
+    r.G0 = fma(b, fma(1.5, bulk, 0.5 * (r.c0 - pl)), fma(r.x2, m0, -(Ft2 * pl)));
+    const double bT2 = r.x2 * fma(m1, m1, m2 * m2);
+    const double G02 = r.G0 * r.G0, disc = fma(-2 * b, bT2, G02);
+    r.inv = recip_d(fma(disc, rsqrt_d(disc), r.G0));
+    r.s2 = 2 * bT2 * r.inv;
+    r.bT = sqrt_estimate(bT2);
+    r.G1 = 0.5 * b * r.bT;
+    // a root well below the parabola's top, u_T < 31, e > 0, and magnitudes
+    // at which the estimates above hold (b >= 1, so bT2 < G0^2 / 2)
+    const bool in = r.G0 > 1e-100 && r.G0 < 1e100 && disc > 1e-4 * G02 && r.s2 < (1 - 1e-5) * r.c0 &&
+                    2 * r.s2 * r.inv < 1 - 1e-3 && r.x2 > 1e-6;
+    if (!in) r.G0 = NAN;
 }
 
-// Two independent Newton solves in lockstep (same iterates as two newton_uT
-// calls, one loop): st = 0 converged (root in u), 1 fallback.
-VAH_HD void newton_uT2(const InvSetup &A, const InvSetup &B, double g0, double g1, double &u0, double &u1, int &st0,
-                       int &st1) {
-    double w0 = g0, w1 = g1;
-    st0 = st1 = 2;
-    for (int it = 0; it < 10000; ++it) {
-        double n0 = w0, n1 = w1;
-        const int c0 = newton_step(A, w0, n0);
-        const int c1 = newton_step(B, w1, n1);
-        if (st0 == 2) {
-            st0 = c0;
-            w0 = n0;
-        }
-        if (st1 == 2) {
-            st1 = c1;
-            w1 = n1;
-        }
-        if (st0 != 2 && st1 != 2) break;
-    }
-    if (st0 == 2) st0 = 1;  // 10^4 iterations without convergence
-    if (st1 == 2) st1 = 1;
-    u0 = w0;
-    u1 = w1;
+// A guess w0 as the test takes it: v0 = w0 / sqrt(1 + w0^2), r2 = 1 / (1 +
+// w0^2), to the hardware estimate's 1e-6 (the margins are wider).
+struct Guess {
+    double v0, r2;
+};
+VAH_HD Guess newton_guess(double ux, double uy) {
+    const double w2 = fma(ux, ux, uy * uy);
+#ifdef __CUDA_ARCH__
+    double g;
+    asm("rsqrt.approx.ftz.f64 %0, %1;" : "=d"(g) : "d"(1 + w2));
+#else
+    const double g = 1.0 / sqrt(1 + w2);
+#endif
+    return {sqrt_estimate(w2) * g, g * g};
+}
+
+// Whether the iteration from the guess ends at the admitted state's root.
+VAH_HD bool newton_reaches(const InvRoot &r, const Guess &w) {
+    const double s = r.G1 * w.v0, f = w.v0 * (r.G0 - s) - r.bT, h = r.G0 - 2 * s;
+    return h > 1e-3 * r.G0 && (f <= 0.0 || (f < 0.999 * (w.v0 * w.r2) * h && w.v0 * r.bT < (1 - 1e-5) * r.c0));
+}
+
+// The velocity v_dir = u^dir / u^tau of an admitted, converged state.
+VAH_HD double root_velocity(const InvRoot &r, double m_dir, int dir) {
+    return dir == 2 ? r.F : 2 * r.x2 * r.inv * m_dir;
 }
 
 // The full inversion. Returns 0 (converged), 1 (fallback) or 2 (a NaN
 // reached e or u). out = {e, p, ut, ux, uy, un}. PF32 (the FP32 form): the
 // pressure from the EoS in FP32 arithmetic (the form stores p in FP32).
-template <int PHYS, bool PF32 = false>
-VAH_HD int invert(const Eos &eos, double t, const double *q, double ePrev, double uT0, double *out) {
+// Its iterated form: (e, u^mu) by Newton's iteration or the fallback; the
+// status without the NaN test. Out of line on the device: seldom run, and its
+// registers stay out of the callers.
+VAH_COLD int invert_iterated(double t, InvIn q, double ePrev, double uT0, double *out) {
     InvSetup s;
-    invert_setup<PHYS>(t, q, s);
+    invert_setup(t, q, s);
     double uT;
     const int status = newton_uT(s, uT0, uT);
-    double e, ut, ux, uy, un;
     if (status == 0) {
         const double C = sqrt(1.0 + uT * uT);
         const double U = uT / C;
         const double inv_mbt = 1.0 / s.mbt, inv_x = 1.0 / s.x;
-        ux = uT * s.m1 * inv_mbt;
-        uy = uT * s.m2 * inv_mbt;
-        un = s.F * C * inv_x;
-        ut = C * inv_x;
-        e = s.c0 - U * s.x * s.mbt;
+        out[0] = s.c0 - U * s.x * s.mbt;
+        out[1] = C * inv_x;
+        out[2] = uT * s.m1 * inv_mbt;
+        out[3] = uT * s.m2 * inv_mbt;
+        out[4] = s.F * C * inv_x;
     } else {
-        e = ePrev * .999;
-        ux = 0.0;
-        uy = 0.0;
-        un = 0.0;
-        ut = 1.0;
+        out[0] = ePrev * .999;
+        out[1] = 1.0;
+        out[2] = out[3] = out[4] = 0.0;
+    }
+    return status;
+}
+
+// ux0, uy0: the guess's velocity (|u_T| starts the iteration).
+template <int PHYS, bool PF32 = false>
+VAH_HD int invert(const Eos &eos, double t, const double *q, double ePrev, double ux0, double uy0, double *out) {
+    const InvIn in = inv_in<PHYS>(q);
+    InvRoot s;
+    invert_root(t, in, s);
+    double e, ut, ux, uy, un;
+    int status = 0;
+    if (newton_reaches(s, newton_guess(ux0, uy0))) {
+        const double C = rsqrt_d(fma(-2 * s.s2, s.inv, 1.0));  // 1 / sqrt(1 - v^2), v^2 = 4 bT^2 inv^2
+        const double ix = rsqrt_d(s.x2);
+        const double k = 2 * s.x2 * ix * s.inv * C;  // u_T / |m_T|
+        ux = k * in.m1;
+        uy = k * in.m2;
+        ut = C * ix;
+        un = s.F * ut;
+        e = s.c0 - s.s2;
+    } else {
+        double r[5];
+        status = invert_iterated(t, in, ePrev, sqrt(fabs(ux0 * ux0 + uy0 * uy0)), r);
+        e = r[0];
+        ut = r[1];
+        ux = r[2];
+        uy = r[3];
+        un = r[4];
     }
     out[0] = e;
     out[1] = PF32 ? (double)eos_pressure_f(eos, (float)e) : eos_pressure(eos, e);
@@ -431,39 +553,24 @@ VAH_HD int invert(const Eos &eos, double t, const double *q, double ePrev, doubl
     return status;
 }
 
-// What a face needs of an inversion: the velocity v_dir = u^dir / u^tau
-// (u^tau = C/x, u^x = uT m1/mbt, u^y = uT m2/mbt, u^eta = F C/x with
-// C = sqrt(1 + uT^2), so v_x = uT m1 x / (mbt C), v_eta = F), 0 after a
-// fallback (u = (1,0,0,0)). Same statuses as invert; a fallback's NaN check
-// is on e = 0.999 ePrev, a converged one's on v and the energy offset.
-VAH_HD int face_velocity(const InvSetup &s, double ePrev, double uT0, int dir, double *v) {
-    double uT;
-    if (newton_uT(s, uT0, uT) != 0) {
-        *v = 0.0;
-        return isnan(ePrev) ? 2 : 1;
-    }
-    double vv;
-    if (dir == 2) {
-        vv = s.F;
-    } else {
-        // uT m x / (mbt C), C = sqrt(1 + uT^2), with 1/C from rsqrt_d
-        vv = uT * (dir == 0 ? s.m1 : s.m2) * s.x * rsqrt_d(1.0 + uT * uT) / s.mbt;
-    }
-    *v = vv;
-    return (isnan(vv) || isnan(s.c0)) ? 2 : 0;
-}
-
 // ------------------------------------------------------------ face flux --
 // Kurganov-Tadmor central flux at one face from the reconstructed states
 // (SemiDiscreteKurganovTadmorScheme.cpp:13-57, SpectralRadius.cpp:14-24,
 // LocalPropagationSpeed.cpp:14-22, FluxFunctions.cpp:15-25):
 // H = (F(qR) + F(qL) - a (qR - qL)) / 2, F = v_dir q, a = max |v_dir|.
-// sR/sL: the inversion set-ups of qR/qL; ePrev, uT: the evaluating cell's
-// fallback energy and Newton guess.
+// ePrev, ux0, uy0: the evaluating cell's fallback energy and guess velocity.
 // Returns the number of the two inversions that fell back; bit 8 flags a NaN.
-// The velocity of a converged solve, as face_velocity (status 0 or 2).
-template <bool FAST = false>
-VAH_HD int face_velocity_of(const InvSetup &s, double uT, int dir, double *v) {
+// The velocity of one face state by the iteration (u^dir / u^tau of its root,
+// 0 after a fallback): 0 converged, 1 fallback, 2 NaN. Seldom run.
+template <bool FAST>
+VAH_COLD int face_velocity_iterated(double t, InvIn q, int dir, double ePrev, double ux0, double uy0, double *v) {
+    InvSetup s;
+    invert_setup<FAST>(t, q, s);
+    double uT;
+    if (newton_uT(s, sqrt(fabs(ux0 * ux0 + uy0 * uy0)), uT) != 0) {
+        *v = 0.0;
+        return isnan(ePrev) ? 2 : 1;
+    }
     double vv;
     if (dir == 2) {
         vv = s.F;
@@ -476,65 +583,66 @@ VAH_HD int face_velocity_of(const InvSetup &s, double uT, int dir, double *v) {
     return (isnan(vv) || isnan(s.c0)) ? 2 : 0;
 }
 
-// The weights of one evaluation, H = wR qR + wL qL (the same statuses).
-VAH_HD int face_weights(const InvSetup &sR, const InvSetup &sL, int dir, double ePrev, double uT, double &wR,
-                        double &wL) {
-    // both states' Newton solves from this guess, in lockstep
-    double uR, uL, vR = 0.0, vL = 0.0;
-    int nR, nL;
-    newton_uT2(sR, sL, uT, uT, uR, uL, nR, nL);
-    const int stR = nR != 0 ? (isnan(ePrev) ? 2 : 1) : face_velocity_of(sR, uR, dir, &vR);
-    const int stL = nL != 0 ? (isnan(ePrev) ? 2 : 1) : face_velocity_of(sL, uL, dir, &vL);
+// The velocity of one face state as a cell evaluates it, with that cell's
+// guess velocity and fallback energy; the iteration's status.
+template <bool FAST = false>
+VAH_HD int face_velocity(double t, const InvIn &q, const InvRoot &r, int dir, double ePrev, double ux0, double uy0,
+                         double *v) {
+    if (newton_reaches(r, newton_guess(ux0, uy0))) {
+        *v = root_velocity(r, dir == 1 ? q.m2 : q.m1, dir);
+        return 0;
+    }
+    return face_velocity_iterated<FAST>(t, q, dir, ePrev, ux0, uy0, v);
+}
+
+// (vR qR + vL qL - a (qR - qL)) / 2 = wR qR + wL qL; the halving is exact
+VAH_HD void face_weights_of(double vR, double vL, double &wR, double &wL) {
     const double a = fmax(fabs(vL), fabs(vR));
-    // (vR qR + vL qL - a (qR - qL)) / 2 = wR qR + wL qL; the halving is exact
     wR = 0.5 * (vR - a);
     wL = 0.5 * (vL + a);
+}
+
+// One face's two states, ready for the evaluations from either side.
+struct FaceRoots {
+    InvIn qR, qL;
+    InvRoot R, L;
+};
+template <int PHYS, bool FAST = false>
+VAH_HD void face_roots(double t, const double *qR, const double *qL, FaceRoots &f) {
+    f.qR = inv_in<PHYS>(qR);
+    f.qL = inv_in<PHYS>(qL);
+    invert_root<FAST>(t, f.qR, f.R);
+    invert_root<FAST>(t, f.qL, f.L);
+}
+
+// The weights of one evaluation, H = wR qR + wL qL (the face flux's status word).
+template <bool FAST = false>
+VAH_HD int face_weights(double t, const FaceRoots &f, int dir, double ePrev, double ux0, double uy0, double &wR,
+                        double &wL) {
+    double vR, vL;
+    const int stR = face_velocity<FAST>(t, f.qR, f.R, dir, ePrev, ux0, uy0, &vR);
+    const int stL = face_velocity<FAST>(t, f.qL, f.L, dir, ePrev, ux0, uy0, &vL);
+    face_weights_of(vR, vL, wR, wL);
     return (stR != 0) + (stL != 0) + ((stR == 2 || stL == 2) ? 256 : 0);
 }
 
 template <int PHYS>
-VAH_HD int face_flux_setup(const InvSetup &sR, const InvSetup &sL, const double *qR, const double *qL, int dir,
-                           double ePrev, double uT, double *H) {
+VAH_HD int face_flux_roots(double t, const FaceRoots &f, const double *qR, const double *qL, int dir, double ePrev,
+                           double ux0, double uy0, double *H) {
     constexpr int NQ = Phys<PHYS>::NQ;
     double wR, wL;
-    const int st = face_weights(sR, sL, dir, ePrev, uT, wR, wL);
+    const int st = face_weights(t, f, dir, ePrev, ux0, uy0, wR, wL);
 #pragma unroll
-    for (int n = 0; n < NQ; ++n) H[n] = wR * qR[n] + wL * qL[n];
+    for (int n = 0; n < NQ; ++n) H[n] = fma(wR, qR[n], wL * qL[n]);
     return st;
 }
 
 template <int PHYS>
-VAH_HD int face_flux(double t, const double *qR, const double *qL, int dir, double ePrev, double uT, double *H) {
-    InvSetup sR, sL;
-    invert_setup<PHYS>(t, qR, sR);
-    invert_setup<PHYS>(t, qL, sL);
-    return face_flux_setup<PHYS>(sR, sL, qR, qL, dir, ePrev, uT, H);
-}
-
-// ------------------------------------------------------- axis sources --
-// pi/Pi gradient terms of the T^{tau mu} equations along one axis
-// (SourceTerms.cpp:46-176). d[n] = (q[+1] - q[-1]) / (2h) for the pi fields.
-template <int PHYS, typename R>
-VAH_HD void axis_sources(const R *d, int dir, R ucomp, R ut, R t, R *S) {
-    const R v = ucomp / ut;
-    const R dPi = Phys<PHYS>::BULK ? d[kSlotPi] * R(1.5) : R(0.0);
-    if (dir == 0) {
-        S[0] = d[5] * v - d[6] - v * dPi;
-        S[1] = d[6] * v - d[9] - dPi;
-        S[2] = d[7] * v - d[10];
-        S[3] = d[8] * v - d[11];
-    } else if (dir == 1) {
-        S[0] = d[5] * v - d[7] - v * dPi;
-        S[2] = d[7] * v - d[12] - dPi;
-        S[1] = d[6] * v - d[10];
-        S[3] = d[8] * v - d[13];
-    } else {
-        const float tf = (float)t;  // SourceTerms.cpp:172: powf(t, 2)
-        S[0] = d[5] * v - d[8] - v * dPi;
-        S[3] = d[8] * v - d[14] - dPi / (R)(tf * tf);
-        S[1] = d[6] * v - d[11];
-        S[2] = d[7] * v - d[13];
-    }
+VAH_HD int face_flux(double t, const double *qR, const double *qL, int dir, double ePrev, double ux0, double uy0,
+                     double *H) {
+    FaceRoots f;
+    face_roots<PHYS>(t, qR, qL, f);
+    return face_flux_roots<PHYS>(t, f, qR, qL, dir, ePrev, ux0, uy0, H);
 }
 
 // x / d for a constant d with its rounded reciprocal inv_d: the product and
@@ -546,7 +654,6 @@ VAH_HD R div_const(R x, R d, R inv_d) {
     return fma(fma(-q, d, x), inv_d, q);
 }
 
-// ----------------------------------------------------------- cell sources --
 // Inputs of the local source terms at one cell: stage-input conserved values,
 // primitives, previous-stage velocity and central differences (q(+1)-q(-1))/(2h).
 template <typename R>
@@ -562,6 +669,8 @@ struct CellGradT {
 template <typename R>
 struct StepConstsT {
     R t, dt, etabar, inv_t, inv_t2, inv_dt;
+    R inv_etabar;
+    R tf2, inv_tf2;  // powf(t, 2) of the eta axis sources (SourceTerms.cpp:172) and 1 / it
 };
 
 using CellGrad = CellGradT<double>;
@@ -576,13 +685,43 @@ VAH_HD StepConstsT<R> step_consts(R t, R dt, R etabar) {
     k.inv_t = R(1.0) / t;
     k.inv_t2 = R(1.0) / (t * t);
     k.inv_dt = R(1.0) / dt;
+    k.inv_etabar = R(1.0) / etabar;
+    const float tf = (float)t;
+    k.tf2 = (R)(tf * tf);
+    k.inv_tf2 = R(1.0) / k.tf2;
     return k;
 }
 
+// ------------------------------------------------------- axis sources --
+// pi/Pi gradient terms of the T^{tau mu} equations along one axis
+// (SourceTerms.cpp:46-176). d[n] = (q[+1] - q[-1]) / (2h) for the pi fields;
+// v = u^dir / u^tau.
+template <int PHYS, typename R>
+VAH_HD void axis_sources(const R *d, int dir, R v, const StepConstsT<R> &k, R *S) {
+    const R dPi = Phys<PHYS>::BULK ? d[kSlotPi] * R(1.5) : R(0.0);
+    if (dir == 0) {
+        S[0] = d[5] * v - d[6] - v * dPi;
+        S[1] = d[6] * v - d[9] - dPi;
+        S[2] = d[7] * v - d[10];
+        S[3] = d[8] * v - d[11];
+    } else if (dir == 1) {
+        S[0] = d[5] * v - d[7] - v * dPi;
+        S[2] = d[7] * v - d[12] - dPi;
+        S[1] = d[6] * v - d[10];
+        S[3] = d[8] * v - d[13];
+    } else {
+        S[0] = d[5] * v - d[8] - v * dPi;
+        S[3] = d[8] * v - d[14] - quot(dPi, k.tf2, k.inv_tf2);
+        S[1] = d[6] * v - d[11];
+        S[2] = d[7] * v - d[13];
+    }
+}
+
+// ----------------------------------------------------------- cell sources --
 // Geometric and relaxation sources S[n] (SourceTerms.cpp:178-1044), W off.
 template <int PHYS, typename R>
 VAH_HD int cell_sources(const Eos &eos, const R *Q, const CellGradT<R> &g, const StepConstsT<R> &k, R *S) {
-    const R t = k.t, etabar = k.etabar;
+    const R t = k.t;
     constexpr bool PIM = Phys<PHYS>::PIMUNU, BULK = Phys<PHYS>::BULK;
     const R ttt = Q[0], ttx = Q[1], tty = Q[2], ttn = Q[3], pl = Q[4];
     R pitt = 0, pitx = 0, pity = 0, pitn = 0, pixx = 0, pixy = 0, pixn = 0, piyy = 0, piyn = 0, pinn = 0,
@@ -598,11 +737,11 @@ VAH_HD int cell_sources(const Eos &eos, const R *Q, const CellGradT<R> &g, const
     const R dyut = g.dyut, dyux = g.dyux, dyuy = g.dyuy, dyun = g.dyun;
     const R dnut = g.dnut, dnux = g.dnux, dnuy = g.dnuy, dnun = g.dnun;
 
-    const R inv_ut = R(1.0) / ut, inv_t = k.inv_t;
+    const R inv_ut = quot(R(1.0), ut), inv_t = k.inv_t;
     const R vx = ux * inv_ut, vy = uy * inv_ut, vn = un * inv_ut;
     const R dkvk = (dxux - vx * dxut) * inv_ut + (dyuy - vy * dyut) * inv_ut + (dnun - vn * dnut) * inv_ut;
 
-    const R t2 = t * t, t3 = t * t2, un2 = un * un, ut2 = ut * ut;
+    const R t2 = t * t, un2 = un * un, ut2 = ut * ut;
     const R inv_t2 = k.inv_t2;
 
     // velocity gradients (SourceTerms.cpp:301-334)
@@ -629,7 +768,7 @@ VAH_HD int cell_sources(const Eos &eos, const R *Q, const CellGradT<R> &g, const
     const R sxn = -ut * ux * un * inv_t - (dxun + dnux * inv_t2) * R(0.5) - (un * dux + ux * dun) * R(0.5) + ux * un * th3;
     const R syy = -(dyuy + uy * duy) + (1 + uy * uy) * th3;
     const R syn = -ut * uy * un * inv_t - (dyun + dnuy * inv_t2) * R(0.5) - (un * duy + uy * dun) * R(0.5) + uy * un * th3;
-    const R snn = -ut * (1 + 2 * t2 * un2) / t3 - dnun * inv_t2 - un * dun + (inv_t2 + un2) * th3;
+    const R snn = quot(-ut * (1 + 2 * t2 * un2), t * t2, inv_t * inv_t2) - dnun * inv_t2 - un * dun + (inv_t2 + un2) * th3;
 
     // transverse / longitudinal split (SourceTerms.cpp:355-426)
     const R uT2 = ux * ux + uy * uy;
@@ -638,8 +777,7 @@ VAH_HD int cell_sources(const Eos &eos, const R *Q, const CellGradT<R> &g, const
     const R uTdnuT = ux * dnux + uy * dnuy;
     const R uTduT = ut * (ux * dtux + uy * dtuy) + ux * uTdxuT + uy * uTdyuT + un * uTdnuT;
     const R F = 1 + uT2;
-    const R inv_F = R(1.0) / F;
-    const R F2 = F * F;
+    const R inv_F = quot(R(1.0), F);
     const R inv_sF = rsqrt_r(F);
     const R z0 = t * un * inv_sF;
     const R z3 = ut * inv_t * inv_sF;
@@ -670,20 +808,16 @@ VAH_HD int cell_sources(const Eos &eos, const R *Q, const CellGradT<R> &g, const
     if (e == 0) e = R(1.e-7);
     R T, cs2;
     eos_T_cs2(eos, e, &T, &cs2);
-    const R inv_e = R(1.0) / e;
+    const R inv_e = quot(R(1.0), e);
     // The closure fits are evaluated in FP64 whatever R is: their monomial
     // coefficients (up to ~1e7, alternating in sign) cancel to results of
     // O(1e-3), and in FP32 several lose every digit (Rbar0P turns infinite).
-    double ap[16];
-    ap[0] = 1.0;
-    ap[1] = (double)pl * (double)inv_e;
-#pragma unroll
-    for (int k = 2; k < 16; ++k) ap[k] = ap[k - 1] * ap[1];
-    const R a = R(ap[1]);
-    const R Rtilde = R(poly::Rtilde<double, kFastQuot<R>>(ap));
-    const R Rbar0 = R(poly::Rbar0<double, kFastQuot<R>>(ap));
-    const R Rgamma = R(poly::Rgamma<double, kFastQuot<R>>(ap));
-    const R Rbar0P = R(poly::Rbar0P<double, kFastQuot<R>>(ap));
+    const double ap = (double)pl * (double)inv_e;
+    const R a = R(ap);
+    const R Rtilde = R(poly::Rtilde<kFastQuot<R>>(ap));
+    const R Rbar0 = R(poly::Rbar0<kFastQuot<R>>(ap));
+    const R Rgamma = R(poly::Rgamma<kFastQuot<R>>(ap));
+    const R Rbar0P = R(poly::Rbar0P<kFastQuot<R>>(ap));
 
     const R e3p = e - 3 * p;
     const R ptHat = (e - pl - Rbar0 * e3p) * R(0.5);
@@ -713,14 +847,13 @@ VAH_HD int cell_sources(const Eos &eos, const R *Q, const CellGradT<R> &g, const
     const R dnLtn = (DP * dnut * un) * inv_F + (DP * dnun * ut) * inv_F + (dnDP * un * ut) * inv_F -
                          (2 * DP * uTdnuT * un * ut) * inv_F2;
     const R dnLnn = ((2 * DP * dnut * ut) * inv_F + (dnDP * ut2) * inv_F - (2 * DP * uTdnuT * ut2) * inv_F2) * inv_t2;
-    (void)F2;
 
     const R zeta_zz = Rtilde * e - 3 * pl;
     const R zeta_zT = (Rtilde * e + pl) * R(0.5);
     const R delta_pipi = (3 + Rgamma) * R(0.5);
     const R tau_pipi = div_const(4 * delta_pipi, R(3.0), R(1.0) / R(3.0));  // SourceTerms.cpp:634, 1/2 -> 0
     const R lambda_pipi = Rgamma - 1;
-    const R taupiInv = R(0.2) * T / etabar;
+    const R taupiInv = quot(R(0.2) * T, k.etabar, k.inv_etabar);
 
     const R psT = pitt * sttT - 2 * pitx * stxT - 2 * pity * styT + pixx * sxxT + 2 * pixy * sxyT + piyy * syyT -
                        2 * pitn * stnT * t2 + 2 * pixn * sxnT * t2 + 2 * piyn * synT * t2 + pinn * snnT * t2 * t2;
@@ -732,16 +865,17 @@ VAH_HD int cell_sources(const Eos &eos, const R *Q, const CellGradT<R> &g, const
         if (third == R(0.0)) third = R(1.e-16);
         const R meq2 = 36 * third;
         const R z2logz = -2 * (1 + R(0.02536) * meq2);
-        const R g40 = (R(poly::g0m2040DividedBym2LogZTerm<double, kFastQuot<R>>(ap)) * z2logz + R(poly::g0m2040DividedBym2Zm2Term<double, kFastQuot<R>>(ap))) /
-                          meq2 +
-                      R(poly::g0m2040DividedBym2ConstantTerm<double, kFastQuot<R>>(ap));
-        const R g20c = R(poly::g0m2020ConstantTerm<double, kFastQuot<R>>(ap));
-        const R g20 = g20c + R(poly::g0m2020Z2LogZTerm<double, kFastQuot<R>>(ap)) * z2logz + R(poly::g0m2020Z2Term<double, kFastQuot<R>>(ap)) * meq2;
+        const R g40 = quot(R(poly::g0m2040DividedBym2LogZTerm<kFastQuot<R>>(ap)) * z2logz +
+                               R(poly::g0m2040DividedBym2Zm2Term<kFastQuot<R>>(ap)),
+                           meq2) +
+                      R(poly::g0m2040DividedBym2ConstantTerm<kFastQuot<R>>(ap));
+        const R g20c = R(poly::g0m2020ConstantTerm<kFastQuot<R>>(ap));
+        const R g20 = g20c + R(poly::g0m2020Z2LogZTerm<kFastQuot<R>>(ap)) * z2logz + R(poly::g0m2020Z2Term<kFastQuot<R>>(ap)) * meq2;
         beta_lPi = 3 * g40;
         delta_lPi = g20 + g40;
         beta_PiPi = 1 - g20c;
         delta_PiPi = R(0.5) * (1 + g20c);
-        lambda_Pipi = div_const(3 * R(poly::G_G1<double, kFastQuot<R>>(ap)), R(5.0), R(1.0) / R(5.0)) * (0 - cs2);
+        lambda_Pipi = div_const(3 * R(poly::G_G1<kFastQuot<R>>(ap)), R(5.0), R(1.0) / R(5.0)) * (0 - cs2);
     }
 
     const R dPL = -(pl - p) * taupiInv + zeta_zz * zDzu - zeta_zT * thetaT - beta_lPi * Pi * zDzu -
@@ -821,9 +955,9 @@ VAH_HD int cell_sources(const Eos &eos, const R *Q, const CellGradT<R> &g, const
     }
     if (BULK) {
         // SourceTerms.cpp:1030-1042
-        const R Rhat = R(poly::Rhat<double, kFastQuot<R>>(ap));
+        const R Rhat = R(poly::Rhat<kFastQuot<R>>(ap));
         const R bb = R(1.0) / R(3.0) - cs2;
-        const R tauPiInv = 15 * bb * bb * T / zeta_over_s(eos, T);
+        const R tauPiInv = over_zeta(eos, T, 15 * bb * bb * T);
         const R zeta_z = div_const((Rhat - Rbar0) * e3p, R(3.0), R(1.0) / R(3.0));
         const R zeta_T = div_const(-(Rbar0 + Rhat) * e3p, R(6.0), R(1.0) / R(6.0));
         const R dPi = -(div_const((1 - Rbar0) * e3p, R(3.0), R(1.0) / R(3.0)) + Pi) * tauPiInv - zeta_z * zDzu - zeta_T * thetaT -
@@ -848,24 +982,21 @@ VAH_HD void regulate(R t, R &e, R &p, R *q, const R *u, R *maps = nullptr) {
     if (q[kSlotPL] < R(0.0)) q[kSlotPL] = R(1.e-7);
     if (!Phys<PHYS>::PIMUNU) return;
     const R pl = q[kSlotPL];
-    double ap[9];  // FP64 closure fit, as in cell_sources
-    ap[0] = 1.0;
-    ap[1] = kFastQuot<R> ? quotient_fast((double)pl, (double)e) : (double)pl / (double)e;
-#pragma unroll
-    for (int k = 2; k < 9; ++k) ap[k] = ap[k - 1] * ap[1];
-    const R ptHat = (e - pl - R(poly::Rbar0<double, kFastQuot<R>>(ap)) * (e - 3 * p)) * R(0.5);
+    // FP64 closure fit, as in cell_sources
+    const double ap = kFastQuot<R> ? quotient_fast((double)pl, (double)e) : quotient_d((double)pl, (double)e);
+    const R ptHat = (e - pl - R(poly::Rbar0<kFastQuot<R>>(ap)) * (e - 3 * p)) * R(0.5);
     const R pitt = q[5], pitx = q[6], pity = q[7], pitn = q[8], pixx = q[9];
     const R pixy = q[10], pixn = q[11], piyy = q[12], piyn = q[13], pinn = q[14];
     const R ut = u[0], ux = u[1], uy = u[2], un = u[3];
     const R inv_sF = rsqrt_r(1 + (ux * ux + uy * uy));
     const R z0 = t * un * inv_sF;
-    const R z3 = ut / t * inv_sF;
+    const R z3 = quot(ut, t) * inv_sF;
     const R t2 = t * t;
     const R sTrsTrs = sqrt(fabs(e * e + pl * pl + 2 * ptHat * ptHat));
     const R pipi = pitt * pitt - 2 * pitx * pitx - 2 * pity * pity + pixx * pixx + 2 * pixy * pixy + piyy * piyy -
                         2 * pitn * pitn * t2 + 2 * pixn * pixn * t2 + 2 * piyn * piyn * t2 + pinn * pinn * t2 * t2;
     const R spipi = sqrt(fabs(pipi));
-    R rho = spipi / sTrsTrs;
+    R rho = quot(spipi, sTrsTrs);
     const R den = spipi;
     const R num[9] = {pitt - pixx - piyy - pinn * t2,
                            -pitn * t2 * un + pitt * ut - pitx * ux - pity * uy,
@@ -893,10 +1024,10 @@ VAH_HD void regulate(R t, R &e, R &p, R *q, const R *u, R *maps = nullptr) {
 #pragma unroll
         for (int m = 0; m < 9; ++m)
             if (num[m] > top) top = num[m];
-        const R c = top / den;
+        const R c = quot(top, den);
         if (c > rho) rho = c;
     }
-    R fac = tanh(rho) / rho;
+    R fac = quot(tanh(rho), rho);
     if (rho < R(1.e-7)) fac = R(1.0);
 #pragma unroll
     for (int n = 5; n < 15; ++n) q[n] *= fac;

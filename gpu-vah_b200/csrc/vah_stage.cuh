@@ -51,16 +51,15 @@ struct StageArgs {
     unsigned char *hot;
     double e_freeze;
     unsigned long long *crossings;
-    // face/cell split: flux through the face at +1/2 of ghosted cell s along
-    // axis d, field n, as cell s evaluates it (H) and as cell s+1 does (HR,
-    // reference face semantics only); scratch of ncell entries per field
+    // the plain form (face_compute): flux through the face at +1/2 of ghosted
+    // cell s along axis d, field n, as cell s evaluates it (H) and as cell s+1
+    // does (HR, reference face semantics only)
     S *H[3][16];
     S *HR[3][16];
-    // optional (FP64 event launches): the x flux difference of each interior
-    // cell, H(-1/2) - H(+1/2) as the cell evaluates both faces, written by the
-    // x face launch (face_x_diff_kernel) and read by the cell launch instead of
-    // H[0] / HR[0]; null: the cell launch differences H[0] / HR[0] itself
-    S *Dx[16];
+    // flux differences of each interior cell per axis, H(-1/2) - H(+1/2) as the
+    // cell evaluates both faces, written by the flux launches (vah_march.cuh)
+    // and read by the cell launch; null: it differences H / HR itself
+    S *D[3][16];
 };
 
 VAH_HD void count_add(unsigned long long *c, unsigned long long v) {
@@ -83,8 +82,8 @@ VAH_HD void finish_args(StageArgs<S> &a) {
     }
 }
 
-template <typename S>
-VAH_HD double ld(const S *p, long long i) {
+template <typename S, typename I>
+VAH_HD double ld(const S *p, I i) {
     return (double)ldg(p + i);
 }
 
@@ -92,8 +91,8 @@ VAH_HD double ld(const S *p, long long i) {
 // (evict-first) cache policy, so that they do not push the state's neighbour
 // reuse out of L1 and L2 (cell launch 3% faster; streaming stores in the face
 // launches cost those 2%, so they store normally).
-template <typename S>
-VAH_HD double ld_stream(const S *p, long long i) {
+template <typename S, typename I>
+VAH_HD double ld_stream(const S *p, I i) {
 #ifdef __CUDA_ARCH__
     return (double)__ldcs(p + i);
 #else
@@ -102,9 +101,9 @@ VAH_HD double ld_stream(const S *p, long long i) {
 }
 
 // Gradients and centre values the source terms need (SourceTerms.cpp:239-280, 484-486).
-template <typename S, bool IS3D>
-VAH_HD void load_cell_grad(const StageArgs<S> &a, long long s, CellGrad &g) {
-    const long long sx = 1, sy = a.ncx, sz = a.plane;
+template <typename S, bool IS3D, typename I>
+VAH_HD void load_cell_grad(const StageArgs<S> &a, I s, CellGrad &g) {
+    const I sx = 1, sy = a.ncx, sz = (I)a.plane;
     const double fx = a.inv2h[0], fy = a.inv2h[1], fz = a.inv2h[2];
     const S *UT = a.uin[0], *UX = a.uin[1], *UY = a.uin[2], *UN = a.uin[3];
     g.e = ld(a.ein, s);
@@ -139,7 +138,7 @@ VAH_HD void load_cell_grad(const StageArgs<S> &a, long long s, CellGrad &g) {
 // val += dt * ((H(-1/2) - H(+1/2)) / h + S_axis).
 template <typename S, int PHYS>
 VAH_HD unsigned axis_update(const StageArgs<S> &a, long long s, int dir, long long st, double h, const double *qc,
-                            double ePrev, double uT, double ucomp, double ut, double *val) {
+                            const CellGrad &g, double ucomp, double *val) {
     constexpr int NQ = Phys<PHYS>::NQ;
     double qR[NQ], qL[NQ], H[NQ];
     unsigned fails = 0;
@@ -151,7 +150,7 @@ VAH_HD unsigned axis_update(const StageArgs<S> &a, long long s, int dir, long lo
         qR[n] = qp - approx_derivative(qc[n], qp, qpp) * 0.5;
         qL[n] = qc[n] + approx_derivative(qm, qc[n], qp) * 0.5;
     }
-    fails += face_flux<PHYS>(a.t_src, qR, qL, dir, ePrev, uT, H);
+    fails += face_flux<PHYS>(a.t_src, qR, qL, dir, g.e, g.ux, g.uy, H);
 #pragma unroll
     for (int n = 0; n < NQ; ++n) val[n] -= c * H[n];
     // face at -1/2: right state from this cell, left state from cell -1
@@ -161,7 +160,7 @@ VAH_HD unsigned axis_update(const StageArgs<S> &a, long long s, int dir, long lo
         qR[n] = qc[n] - approx_derivative(qm, qc[n], qp) * 0.5;
         qL[n] = qm + approx_derivative(qmm, qm, qc[n]) * 0.5;
     }
-    fails += face_flux<PHYS>(a.t_src, qR, qL, dir, ePrev, uT, H);
+    fails += face_flux<PHYS>(a.t_src, qR, qL, dir, g.e, g.ux, g.uy, H);
 #pragma unroll
     for (int n = 0; n < NQ; ++n) val[n] += c * H[n];
     if (Phys<PHYS>::PIMUNU) {
@@ -170,15 +169,15 @@ VAH_HD unsigned axis_update(const StageArgs<S> &a, long long s, int dir, long lo
 #pragma unroll
         for (int n = 5; n < NQ; ++n) d[n] = (ld(a.qin[n], s + st) - ld(a.qin[n], s - st)) * f;
         double Sa[4];
-        axis_sources<PHYS>(d, dir, ucomp, ut, a.t_src, Sa);
+        axis_sources<PHYS>(d, dir, quotient_d(ucomp, g.ut), a.ksrc, Sa);
 #pragma unroll
         for (int n = 0; n < 4; ++n) val[n] += a.dt * Sa[n];
     }
     return fails;
 }
 
-template <typename S>
-VAH_HD void store_cell(const StageArgs<S> &a, long long s, int NQ, const double *val, const double *u, double e,
+template <typename S, typename I>
+VAH_HD void store_cell(const StageArgs<S> &a, I s, int NQ, const double *val, const double *u, double e,
                        double p) {
     for (int n = 0; n < NQ; ++n) a.qout[n][s] = (S)val[n];
     for (int m = 0; m < 4; ++m) a.uout[m][s] = (S)u[m];
@@ -203,11 +202,10 @@ VAH_HD void stage_cell(const StageArgs<S> &a, int i, int j, int k) {
     for (int n = 0; n < NQ; ++n) val[n] = qc[n] + a.dt * Sv[n];
 
     // X, Y, Z flux sweeps; Newton guess = |u_T| of this cell, fallback = its e
-    const double uT = sqrt(fabs(g.ux * g.ux + g.uy * g.uy));
     unsigned fails = 0;
-    fails += axis_update<S, PHYS>(a, s, 0, 1, a.dx, qc, g.e, uT, g.ux, g.ut, val);
-    fails += axis_update<S, PHYS>(a, s, 1, a.ncx, a.dy, qc, g.e, uT, g.uy, g.ut, val);
-    if (IS3D) fails += axis_update<S, PHYS>(a, s, 2, a.plane, a.dz, qc, g.e, uT, g.un, g.ut, val);
+    fails += axis_update<S, PHYS>(a, s, 0, 1, a.dx, qc, g, g.ux, val);
+    fails += axis_update<S, PHYS>(a, s, 1, a.ncx, a.dy, qc, g, g.uy, val);
+    if (IS3D) fails += axis_update<S, PHYS>(a, s, 2, a.plane, a.dz, qc, g, g.un, val);
 
     // stage 2: Q = (q + Q) / 2 (convexCombinationEulerStepKernel, :465-521)
     if (a.stage2) {
@@ -221,7 +219,7 @@ VAH_HD void stage_cell(const StageArgs<S> &a, int i, int j, int k) {
     double qfull[16];
 #pragma unroll
     for (int n = 0; n < 16; ++n) qfull[n] = n < NQ ? val[n] : 0.0;
-    const int st = invert<PHYS>(a.eos, a.t_inv, qfull, g.e, sqrt(fabs(gx * gx + gy * gy)), prim);
+    const int st = invert<PHYS>(a.eos, a.t_inv, qfull, g.e, gx, gy, prim);
     double e = prim[0], p = prim[1];
     double u[4] = {prim[2], prim[3], prim[4], prim[5]};
     double rmap[11];
@@ -247,10 +245,11 @@ VAH_HD void stage_cell(const StageArgs<S> &a, int i, int j, int k) {
     }
 }
 
-// ------------------------------------------------------- face/cell split --
-// The face fluxes of a stage are computed by their own launch (face_compute)
-// into scratch buffers, and the cell launch (cell_compute) takes flux
-// differences from them. Two face modes:
+// ------------------------------------------------------- flux/cell split --
+// The flux differences of a stage are computed by their own launches
+// (vah_march.cuh) into scratch buffers, and the cell launch (cell_compute)
+// reads them. face_compute is the same evaluation in its plain form, one face
+// at a time into H / HR, which the host build runs. Two face modes:
 //   EXACT (reference semantics, VAH_FLUX_PER_CELL): the reference evaluates
 //     each face twice, once from each neighbour, with that neighbour's Newton
 //     guess and fallback energy (FullyDiscreteKurganovTadmorScheme.cpp:179,183);
@@ -286,19 +285,18 @@ VAH_HD unsigned face_compute(const StageArgs<S> &a, long long s, int dir, long l
     constexpr int NQ = Phys<PHYS>::NQ;
     double qR[NQ], qL[NQ], H[NQ];
     face_states<S, PHYS>(a, s, st, qR, qL);
-    InvSetup sR, sL;  // set up once, inverted from one guess (shared) or both (reference faces)
-    invert_setup<PHYS>(a.t_src, qR, sR);
-    invert_setup<PHYS>(a.t_src, qL, sL);
+    FaceRoots f;  // once, tested from one guess (shared) or both (reference faces)
+    face_roots<PHYS>(a.t_src, qR, qL, f);
     unsigned fails = 0;
     if (!EXACT || left_in) {
         const double ux = ld(a.uin[1], s), uy = ld(a.uin[2], s);
-        fails += face_flux_setup<PHYS>(sR, sL, qR, qL, dir, ld(a.ein, s), sqrt(fabs(ux * ux + uy * uy)), H);
+        fails += face_flux_roots<PHYS>(a.t_src, f, qR, qL, dir, ld(a.ein, s), ux, uy, H);
 #pragma unroll
         for (int n = 0; n < NQ; ++n) a.H[dir][n][s] = (S)H[n];
     }
     if (EXACT && right_in) {
         const double vx = ld(a.uin[1], s + st), vy = ld(a.uin[2], s + st);
-        fails += face_flux_setup<PHYS>(sR, sL, qR, qL, dir, ld(a.ein, s + st), sqrt(fabs(vx * vx + vy * vy)), H);
+        fails += face_flux_roots<PHYS>(a.t_src, f, qR, qL, dir, ld(a.ein, s + st), vx, vy, H);
 #pragma unroll
         for (int n = 0; n < NQ; ++n) a.HR[dir][n][s] = (S)H[n];
     }
@@ -309,7 +307,8 @@ VAH_HD unsigned face_compute(const StageArgs<S> &a, long long s, int dir, long l
 template <typename S, int PHYS, bool IS3D, bool EXACT>
 VAH_HD void cell_compute(const StageArgs<S> &a, int i, int j, int k) {
     constexpr int NQ = Phys<PHYS>::NQ;
-    const long long s = i + (long long)a.ncx * j + a.plane * k;
+    const int ncx = a.ncx, plane = (int)a.plane;
+    const int s = i + ncx * j + plane * k;  // 32-bit: 2^31 cells of any form exceed the device memory
     double qc[NQ], val[NQ], Sv[NQ];
 #pragma unroll
     for (int n = 0; n < NQ; ++n) qc[n] = ld(a.qin[n], s);
@@ -318,17 +317,17 @@ VAH_HD void cell_compute(const StageArgs<S> &a, int i, int j, int k) {
     int bad = cell_sources<PHYS>(a.eos, qc, g, a.ksrc, Sv);
 #pragma unroll
     for (int n = 0; n < NQ; ++n) val[n] = qc[n] + a.dt * Sv[n];
-    const long long strides[3] = {1, a.ncx, a.plane};
+    const int strides[3] = {1, ncx, plane};
     const double hs[3] = {a.dx, a.dy, a.dz};
-    const double ucomp[3] = {g.ux, g.uy, g.un};
+    const double ucomp[3] = {g.ux, g.uy, g.un}, inv_ut = quotient_d(1.0, g.ut);
 #pragma unroll
     for (int dir = 0; dir < (IS3D ? 3 : 2); ++dir) {
-        const long long st = strides[dir];
+        const int st = strides[dir];
         const double c = a.c_h[dir];
         const S *const *Hm = EXACT ? a.HR[dir] : a.H[dir];  // face -1/2 as this cell evaluates it
-        if (dir == 0 && a.Dx[0]) {
+        if (a.D[0][0]) {
 #pragma unroll
-            for (int n = 0; n < NQ; ++n) val[n] += c * ld_stream(a.Dx[n], s);
+            for (int n = 0; n < NQ; ++n) val[n] += c * ld_stream(a.D[dir][n], s);
         } else {
 #pragma unroll
             for (int n = 0; n < NQ; ++n) val[n] += c * (ld_stream(Hm[n], s - st) - ld_stream(a.H[dir][n], s));
@@ -339,7 +338,7 @@ VAH_HD void cell_compute(const StageArgs<S> &a, int i, int j, int k) {
 #pragma unroll
             for (int n = 5; n < NQ; ++n) d[n] = (ld(a.qin[n], s + st) - ld(a.qin[n], s - st)) * f;
             double Sa[4];
-            axis_sources<PHYS>(d, dir, ucomp[dir], g.ut, a.t_src, Sa);
+            axis_sources<PHYS>(d, dir, ucomp[dir] * inv_ut, a.ksrc, Sa);
 #pragma unroll
             for (int n = 0; n < 4; ++n) val[n] += a.dt * Sa[n];
         }
@@ -352,7 +351,7 @@ VAH_HD void cell_compute(const StageArgs<S> &a, int i, int j, int k) {
     double prim[6], qfull[16];
 #pragma unroll
     for (int n = 0; n < 16; ++n) qfull[n] = n < NQ ? val[n] : 0.0;
-    const int st = invert<PHYS>(a.eos, a.t_inv, qfull, g.e, sqrt(fabs(gx * gx + gy * gy)), prim);
+    const int st = invert<PHYS>(a.eos, a.t_inv, qfull, g.e, gx, gy, prim);
     double e = prim[0], p = prim[1];
     double u[4] = {prim[2], prim[3], prim[4], prim[5]};
     double rmap[11];
@@ -370,7 +369,7 @@ VAH_HD void cell_compute(const StageArgs<S> &a, int i, int j, int k) {
         }
     }
     store_cell(a, s, NQ, val, u, e, p);
-    const long long sy = a.ncx, sz = a.plane;
+    const int sy = ncx, sz = plane;
     if (i == 2) { store_cell(a, s - 1, NQ, val, u, e, p); store_cell(a, s - 2, NQ, val, u, e, p); }
     if (i == a.nx + 1) { store_cell(a, s + 1, NQ, val, u, e, p); store_cell(a, s + 2, NQ, val, u, e, p); }
     if (j == 2) { store_cell(a, s - sy, NQ, val, u, e, p); store_cell(a, s - 2 * sy, NQ, val, u, e, p); }

@@ -108,16 +108,11 @@ VAH_TILE_FACE unsigned tile_face(const QA q, long long L, long long st, int dir,
         dR[n] = n < NQ ? (double)qR[n] : 0.0;
         dL[n] = n < NQ ? (double)qL[n] : 0.0;
     }
-    InvSetup sR, sL;
-    invert_setup<PHYS, true>(t, dR, sR);
-    invert_setup<PHYS, true>(t, dL, sL);
-    double uR, uL, vR = 0.0, vL = 0.0;
-    int nR, nL;
-    newton_uT2(sR, sL, uT, uT, uR, uL, nR, nL);
-    const int stR = nR != 0 ? (isnan(ePrev) ? 2 : 1) : face_velocity_of<true>(sR, uR, dir, &vR);
-    const int stL = nL != 0 ? (isnan(ePrev) ? 2 : 1) : face_velocity_of<true>(sL, uL, dir, &vL);
-    const double a = fmax(fabs(vL), fabs(vR));
-    const float wR = (float)(0.5 * (vR - a)), wL = (float)(0.5 * (vL + a));
+    FaceRoots f;
+    face_roots<PHYS, true>(t, dR, dL, f);
+    double wRd, wLd;
+    const unsigned st_word = face_weights<true>(t, f, dir, ePrev, uT, 0.0, wRd, wLd);
+    const float wR = (float)wRd, wL = (float)wLd;
 #pragma unroll
     for (int n = 0; n + 1 < NQ; n += 2) {  // wR qR + wL qL, two fields at a time
         const Pair h = pfma(Pair{wR, wR}, Pair{qR[n], qR[n + 1]}, pmul(Pair{wL, wL}, Pair{qL[n], qL[n + 1]}));
@@ -125,7 +120,7 @@ VAH_TILE_FACE unsigned tile_face(const QA q, long long L, long long st, int dir,
         H[(n + 1) * hs] = h.b;
     }
     if (NQ % 2) H[(NQ - 1) * hs] = fmaf(wR, qR[NQ - 1], wL * qL[NQ - 1]);
-    return (stR != 0) + (stL != 0) + ((stR == 2 || stL == 2) ? 256u : 0u);
+    return st_word;
 }
 
 // Stage-input primitives: e, p, u read at the cell and its +-1 neighbours
@@ -199,7 +194,7 @@ VAH_HD void tile_cell_explicit(const QA &q, long long b, long long bsy, long lon
 #pragma unroll
             for (int n = 5; n < NQ; ++n) dd[n] = (q(n, b + sts[dir]) - q(n, b - sts[dir])) * fh[dir];
             float Sa[4];
-            axis_sources<PHYS>(dd, dir, ucomp[dir], g.ut, (float)t_src, Sa);
+            axis_sources<PHYS>(dd, dir, ucomp[dir] / g.ut, k, Sa);
 #pragma unroll
             for (int n = 0; n < 4; ++n) val[n] += dtf * Sa[n];
         }
@@ -226,7 +221,7 @@ VAH_HD int tile_cell_invert(const TilePrims &pr, long long s, const QV &qavg, bo
     double qd[16], prim[6];
 #pragma unroll
     for (int n = 0; n < 16; ++n) qd[n] = n < NQ ? (double)val[n] : 0.0;
-    const int st = invert<PHYS, true>(eos, t_inv, qd, (double)e_prev, sqrt(fabs(gx * gx + gy * gy)), prim);
+    const int st = invert<PHYS, true>(eos, t_inv, qd, (double)e_prev, gx, gy, prim);
     e = (float)prim[0];
     p = (float)prim[1];
     for (int m = 0; m < 4; ++m) u[m] = (float)prim[2 + m];

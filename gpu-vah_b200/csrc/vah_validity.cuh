@@ -107,11 +107,7 @@ VAH_HD void validity_cell(const ValidityArgs<S> &a, long long s) {
     const double pixy = pi[5], pixn = pi[6], piyy = pi[7], piyn = pi[8], pinn = pi[9];
     const double pipi = pitt * pitt - 2 * pitx * pitx - 2 * pity * pity + pixx * pixx + 2 * pixy * pixy + piyy * piyy -
                         2 * pitn * pitn * t2 + 2 * pixn * pixn * t2 + 2 * piyn * piyn * t2 + pinn * pinn * t2 * t2;
-    double ap[16];
-    ap[0] = 1.0;
-    ap[1] = pl / e_s;
-#pragma unroll
-    for (int k = 2; k < 16; ++k) ap[k] = ap[k - 1] * ap[1];
+    const double ap = pl / e_s;
     const double Rtilde = poly::Rtilde(ap), Rhat = poly::Rhat(ap), Rbar0 = poly::Rbar0(ap), Rgamma = poly::Rgamma(ap);
     const double ptHat = (e_s - pl - Rbar0 * (e_s - 3 * p_s)) / 2;
     a.v[4][s] = sqrt(fabs(pipi)) / fabs(ptHat);
