@@ -50,6 +50,8 @@ struct vah_event {
     unsigned char *d_fb;             // optional: per ghosted cell, stage-1 then stage-2 inversion fallback flags
     long long steps;
     double last_t, last_dt;          // time and step of the latest vah_rk2_step (autotuning state)
+    double *d_fstage;                // staging of the field reads and writes ...
+    size_t fstage;                   // ... of this many values
     double *d_stage64;               // FP32 storage: one FP64 field of staging for the host-buffer step ...
     double *d_stage_all;             // ... and every field, host layout, for its overlapped form (3+1D)
     bool validity;                   // fill the validity diagnostics every step
@@ -135,6 +137,7 @@ void free_all(vah_event *ev) {
     cudaFree(ev->d_exc);
     cudaFree(ev->d_counters);
     cudaFree(ev->d_fb);
+    cudaFree(ev->d_fstage);
     cudaFree(ev->d_stage64);
     cudaFree(ev->d_stage_all);
     for (int m = 0; m < VAH_NUM_VALIDITY; ++m) cudaFree(ev->vd[m]);
@@ -433,6 +436,8 @@ extern "C" int vah_event_create(const vah_lattice *lat, const vah_hydro *hydro, 
     ev->timing = false;
     ev->steps = 0;
     ev->last_t = hydro->t0;
+    ev->d_fstage = nullptr;
+    ev->fstage = std::max(vah::field_stage_values(ev->ncell), (size_t)lat->nx + 4);  // at least one row
     ev->d_stage64 = nullptr;
     ev->d_stage_all = nullptr;
     ev->d_fb = nullptr;
@@ -510,6 +515,7 @@ extern "C" int vah_event_create(const vah_lattice *lat, const vah_hydro *hydro, 
     if (opt->flux != VAH_FLUX_PER_CELL_FUSED && !ev->tile)
         for (int d = 0; d < (lat->nz > 1 ? 3 : 2); ++d)
             for (int n = 0; n < ev->nq; ++n) alloc(&ev->D[d][n]);
+    if (rc == VAH_OK && cudaMalloc((void **)&ev->d_fstage, ev->fstage * sizeof(double)) != cudaSuccess) rc = VAH_ERR_NOMEM;
     if (rc == VAH_OK && cudaMalloc((void **)&ev->d_counters, 4 * sizeof(unsigned long long)) != cudaSuccess)
         rc = VAH_ERR_NOMEM;
     if (rc == VAH_OK) cudaMemset(ev->d_counters, 0, 4 * sizeof(unsigned long long));
@@ -551,42 +557,17 @@ extern "C" int vah_event_destroy(vah_event *ev) {
 namespace {
 
 // Copy interior or full arrays between double host memory and the event's
-// storage type; FP32 storage converts through a host staging buffer.
+// storage type.
 int copy_field(vah_event *ev, void *d, double *host_out, const double *host_in, int with_ghosts) {
     const int nx = ev->lat.nx, ny = ev->lat.ny, nz = ev->lat.nz;
-    const size_t full = (size_t)(nx + 4) * ev->ncy * ev->ncz, inner = (size_t)nx * ny * nz;  // host layouts
-    const size_t n = with_ghosts ? full : inner;
-    const bool to_dev = host_in != nullptr;
-    std::vector<float> stage;
-    if (ev->elem == sizeof(float)) {
-        stage.resize(n);
-        if (to_dev)
-            for (size_t k = 0; k < n; ++k) stage[k] = (float)host_in[k];
-    }
-    const void *src_h = ev->elem == sizeof(float) ? (const void *)stage.data() : (const void *)host_in;
-    void *dst_h = ev->elem == sizeof(float) ? (void *)stage.data() : (void *)host_out;
-    const size_t es = ev->elem;
-    if (with_ghosts) {  // rows of nx + 4 on the host, of the device pitch on the device
-        const size_t w = (size_t)(nx + 4) * es, rows = (size_t)ev->ncy * ev->ncz;
-        if (to_dev)
-            VAH_TRY(cudaMemcpy2DAsync(d, ev->ncx * es, src_h, w, w, rows, cudaMemcpyHostToDevice, ev->stream));
-        else
-            VAH_TRY(cudaMemcpy2DAsync(dst_h, w, d, ev->ncx * es, w, rows, cudaMemcpyDeviceToHost, ev->stream));
-    } else {
-        for (int k = 0; k < nz; ++k) {
-            char *dev_row = (char *)d + es * (2 + (size_t)ev->ncx * (2 + (size_t)ev->ncy * (k + 2)));
-            const size_t off = es * (size_t)nx * ny * k;
-            if (to_dev)
-                VAH_TRY(cudaMemcpy2DAsync(dev_row, ev->ncx * es, (const char *)src_h + off, nx * es, nx * es, ny,
-                                          cudaMemcpyHostToDevice, ev->stream));
-            else
-                VAH_TRY(cudaMemcpy2DAsync((char *)dst_h + off, nx * es, dev_row, ev->ncx * es, nx * es, ny,
-                                          cudaMemcpyDeviceToHost, ev->stream));
-        }
-    }
+    const bool gh = with_ghosts != 0;
+    if (ev->elem == sizeof(float))
+        VAH_TRY(host_in ? vah::write_field<float>((float *)d, host_in, nx, ny, nz, ev->ncx, gh, ev->d_fstage, ev->fstage, ev->stream)
+                        : vah::read_field<float>((const float *)d, host_out, nx, ny, nz, ev->ncx, gh, ev->d_fstage, ev->fstage, ev->stream));
+    else
+        VAH_TRY(host_in ? vah::write_field<double>((double *)d, host_in, nx, ny, nz, ev->ncx, gh, ev->d_fstage, ev->fstage, ev->stream)
+                        : vah::read_field<double>((const double *)d, host_out, nx, ny, nz, ev->ncx, gh, ev->d_fstage, ev->fstage, ev->stream));
     VAH_TRY(cudaStreamSynchronize(ev->stream));
-    if (!to_dev && ev->elem == sizeof(float))
-        for (size_t k = 0; k < n; ++k) host_out[k] = (double)stage[k];
     return VAH_OK;
 }
 

@@ -20,6 +20,7 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <type_traits>
 #include <vector>
 
 #include "vah.h"
@@ -356,11 +357,15 @@ struct vah_batch {
         vah_hydro hydro{};
         double dt = 0;
         size_t bytes = 0;
+        long long admitted = 0;  // the batch's step count at admission: the velocity buffers' parity since
         void *mem = nullptr;
         std::vector<void *> field;  // VAH_F_* -> device array (current roles resolved at query time)
     };
     std::vector<Slot> slots;
+    long long steps;                       // queued since the batch was created
     std::vector<unsigned char> desc_host;  // host mirror of the descriptor array
+    double *d_fstage;  // staging of the field reads ...
+    size_t fstage;     // ... of this many values
     WorkItem *d_work[vah::K_NUM];
     // FP32 form: tile descriptors per slot, tile work-lists (2+1D, 3+1D), launch counter and error flags
     bool tile;
@@ -866,6 +871,8 @@ extern "C" int vah_batch_create(const vah_options *opt, const double *eos_table,
     chk(cudaMalloc((void **)&b->d_counters, sizeof(unsigned long long) * 4 * vah::kMaxSlots));
     chk(cudaMalloc((void **)&b->d_maxbits, sizeof(unsigned long long) * vah::kMaxSlots));
     chk(cudaMalloc((void **)&b->d_wcount, sizeof(unsigned) * vah::K_NUM));
+    b->fstage = vah::kFieldStageValues;
+    chk(cudaMalloc((void **)&b->d_fstage, sizeof(double) * b->fstage));
     if (b->tile) {
         chk(cudaMalloc((void **)&b->d_tdesc, sizeof(vah::TileSlot) * vah::kMaxSlots));
         chk(cudaMalloc((void **)&b->d_tcount, 2 * sizeof(unsigned)));
@@ -927,6 +934,7 @@ extern "C" int vah_batch_destroy(vah_batch *b) {
     cudaFree(b->d_counters);
     cudaFree(b->d_maxbits);
     cudaFree(b->d_wcount);
+    cudaFree(b->d_fstage);
     cudaFree(b->d_tdesc);
     cudaFree(b->d_tcount);
     cudaFree(b->d_tab);
@@ -963,6 +971,14 @@ int add_slot(vah_batch *b, const vah_lattice *lat, const vah_hydro *hydro, doubl
         }
     if (slot < 0) return VAH_ERR_FULL;
     VAH_TRY(cudaSetDevice(b->opt.device));
+    if ((size_t)lat->nx + 4 > b->fstage) {  // the staging holds a row of any event
+        double *wider = nullptr;
+        VAH_TRY(cudaStreamSynchronize(b->stream));
+        VAH_TRY(cudaMalloc((void **)&wider, sizeof(double) * ((size_t)lat->nx + 4)));
+        cudaFree(b->d_fstage);
+        b->d_fstage = wider;
+        b->fstage = (size_t)lat->nx + 4;
+    }
     vah_batch::Slot &sl = b->slots[slot];
     VAH_TRY(cudaMallocFromPoolAsync(&sl.mem, bytes, b->pool, b->stream));
     VAH_TRY(cudaMemsetAsync(sl.mem, 0, bytes, b->stream));
@@ -971,6 +987,7 @@ int add_slot(vah_batch *b, const vah_lattice *lat, const vah_hydro *hydro, doubl
     sl.hydro = *hydro;
     sl.dt = dt;
     sl.bytes = bytes;
+    sl.admitted = b->steps;
     b->used += bytes;
     int rc = b->elem == sizeof(float) ? fill_slot<float>(b, slot) : fill_slot<double>(b, slot);
     if (rc == VAH_OK)
@@ -1023,7 +1040,10 @@ extern "C" int vah_batch_step(vah_batch *b, int nsteps) {
         if ((rc = capture_graph(b)) != VAH_OK) return rc;
     }
     if (b->timing) VAH_TRY(cudaEventRecord(b->t0, b->stream));
-    for (int n = 0; n < nsteps; ++n) VAH_TRY(cudaGraphLaunch(b->graph, b->stream));
+    for (int n = 0; n < nsteps; ++n) {
+        VAH_TRY(cudaGraphLaunch(b->graph, b->stream));
+        ++b->steps;
+    }
     if (b->timing) {
         VAH_TRY(cudaEventRecord(b->t1, b->stream));
         VAH_TRY(cudaEventSynchronize(b->t1));
@@ -1067,47 +1087,24 @@ const unsigned char *slot_fallback(vah_batch *b, int slot) {
 extern "C" int vah_batch_get_field(vah_batch *b, int slot, int field, double *host, int with_ghosts) {
     if (!b || !host || slot < 0 || slot >= vah::kMaxSlots || !b->slots[slot].used) return VAH_ERR_ARG;
     VAH_TRY(cudaSetDevice(b->opt.device));
-    SlotClock c;
-    VAH_TRY(cudaMemcpyAsync(&c, b->d_clk + slot, sizeof(c), cudaMemcpyDeviceToHost, b->stream));
-    VAH_TRY(cudaStreamSynchronize(b->stream));
     const vah_lattice &lat = b->slots[slot].lat;
-    const size_t ncx = slot_pitch(b, lat.nx), ncy = lat.ny + 4, hx = lat.nx + 4;
-    const size_t ncell = hx * ncy * (lat.nz + 4);  // host layout
-    const size_t n = with_ghosts ? ncell : (size_t)lat.nx * lat.ny * lat.nz;
-    std::vector<float> f32;
-    void *src = b->elem == sizeof(float) ? (void *)slot_field<float>(b, slot, field, c.parity)
-                                         : (void *)slot_field<double>(b, slot, field, c.parity);
-    if (!src) return VAH_ERR_ARG;
-    const size_t es = b->elem;
-    if (es == sizeof(float)) f32.resize(n);
-    void *dst = es == sizeof(float) ? (void *)f32.data() : (void *)host;
-    if (with_ghosts && lat.nz == 1) {  // 2+1D steps leave the eta ghost layers to the reader
-        if (es == sizeof(float)) {
-            vah::FieldSet<float> f{};
-            f.f[0] = (float *)src;
+    const int ncx = slot_pitch(b, lat.nx), parity = (int)((b->steps - b->slots[slot].admitted) & 1);
+    auto read = [&](auto *src) -> int {
+        using S = std::remove_reference_t<decltype(*src)>;
+        if (!src) return VAH_ERR_ARG;
+        if (with_ghosts && lat.nz == 1) {  // 2+1D steps leave the eta ghost layers to the reader
+            vah::FieldSet<S> f{};
+            f.f[0] = src;
             f.n = 1;
-            VAH_TRY(vah::launch_ghost_pass<float>(f, lat.nx, lat.ny, lat.nz, (int)ncx, 2, b->stream));
-        } else {
-            vah::FieldSet<double> f{};
-            f.f[0] = (double *)src;
-            f.n = 1;
-            VAH_TRY(vah::launch_ghost_pass<double>(f, lat.nx, lat.ny, lat.nz, (int)ncx, 2, b->stream));
+            VAH_TRY(vah::launch_ghost_pass<S>(f, lat.nx, lat.ny, lat.nz, ncx, 2, b->stream));
         }
-    }
-    if (with_ghosts) {
-        VAH_TRY(cudaMemcpy2DAsync(dst, hx * es, src, ncx * es, hx * es, ncy * (lat.nz + 4), cudaMemcpyDeviceToHost,
-                                  b->stream));
-    } else {
-        for (int k = 0; k < lat.nz; ++k) {
-            const char *row = (const char *)src + es * (2 + ncx * (2 + ncy * (k + 2)));
-            VAH_TRY(cudaMemcpy2DAsync((char *)dst + es * (size_t)lat.nx * lat.ny * k, lat.nx * es, row, ncx * es,
-                                      lat.nx * es, lat.ny, cudaMemcpyDeviceToHost, b->stream));
-        }
-    }
-    VAH_TRY(cudaStreamSynchronize(b->stream));
-    if (es == sizeof(float))
-        for (size_t k = 0; k < n; ++k) host[k] = (double)f32[k];
-    return VAH_OK;
+        VAH_TRY(vah::read_field<S>(src, host, lat.nx, lat.ny, lat.nz, ncx, with_ghosts != 0, b->d_fstage, b->fstage,
+                                   b->stream));
+        VAH_TRY(cudaStreamSynchronize(b->stream));
+        return VAH_OK;
+    };
+    return b->elem == sizeof(float) ? read(slot_field<float>(b, slot, field, parity))
+                                    : read(slot_field<double>(b, slot, field, parity));
 }
 
 extern "C" int vah_batch_fallback_mask(vah_batch *b, int slot, unsigned char *host) {

@@ -60,6 +60,22 @@ __global__ void __launch_bounds__(kSplitThreads, kMarchMinb) flux_march_kernel(c
     flux_march<PHYS, DIR, EXACT>(a, HalfSelect<PHYS>{a}, w - part * strips, m0, min(m0 + seg, hi), march_sm + (threadIdx.x / 32) * kMarchDoubles<PHYS>);
 }
 
+// One warp per row at a time; PACK: device layout -> packed, else back.
+template <typename S, bool PACK>
+__global__ void pack_kernel(S *__restrict__ field, double *__restrict__ packed, int w, int nyr, int pitch, int ncy,
+                            int off, long long row0, long long rows) {
+    for (long long r = blockIdx.x * (long long)blockDim.y + threadIdx.y; r < rows; r += (long long)gridDim.x * blockDim.y) {
+        const long long k = (row0 + r) / nyr;
+        const int j = (int)((row0 + r) - k * nyr);
+        S *f = field + off + pitch * ((j + off) + (long long)ncy * (k + off));
+        double *p = packed + r * w;
+        for (int i = threadIdx.x; i < w; i += 32) {
+            if (PACK) p[i] = (double)f[i];
+            else f[i] = (S)p[i];
+        }
+    }
+}
+
 template <int PHYS, bool IS3D>
 __global__ void __launch_bounds__(kSplitThreads, kCellMinb) cell_kernel(const StageArgs<double> a) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -295,6 +311,26 @@ cudaError_t launch_ghosts(const FieldSet<S> &fields, int nx, int ny, int nz, int
     return cudaSuccess;
 }
 
+template <typename S, bool PACK>
+cudaError_t pack_dispatch(S *field, double *packed, int nx, int ny, int pitch, bool ghosts, long long row0,
+                          long long rows, cudaStream_t stream) {
+    if (rows <= 0) return cudaSuccess;
+    const int off = ghosts ? 0 : 2, grid = grid_for(rows, 8);
+    pack_kernel<S, PACK><<<grid, dim3(32, 8), 0, stream>>>(field, packed, ghosts ? nx + 4 : nx, ghosts ? ny + 4 : ny,
+                                                           pitch, ny + 4, off, row0, rows);
+    return cudaGetLastError();
+}
+template <typename S>
+cudaError_t launch_pack(const S *field, double *packed, int nx, int ny, int pitch, bool ghosts, long long row0,
+                        long long rows, cudaStream_t stream) {
+    return pack_dispatch<S, true>(const_cast<S *>(field), packed, nx, ny, pitch, ghosts, row0, rows, stream);
+}
+template <typename S>
+cudaError_t launch_unpack(S *field, const double *packed, int nx, int ny, int pitch, bool ghosts, long long row0,
+                          long long rows, cudaStream_t stream) {
+    return pack_dispatch<S, false>(field, const_cast<double *>(packed), nx, ny, pitch, ghosts, row0, rows, stream);
+}
+
 // One pass of the ghost fill (0: x, 1: y, 2: eta), as launch_ghosts runs it.
 template <typename S>
 cudaError_t launch_ghost_pass(const FieldSet<S> &fields, int nx, int ny, int nz, int pitch, int pass,
@@ -314,6 +350,10 @@ cudaError_t launch_ghost_pass(const FieldSet<S> &fields, int nx, int ny, int nz,
                                                  const S *, int, int, int, int, int, double, int, cudaStream_t); \
     template cudaError_t launch_init_primitives<S>(const FieldSet<S> &, const FieldSet<S> &, const S *, S *,    \
                                                    const Eos &, int, int, int, int, cudaStream_t);             \
+    template cudaError_t launch_pack<S>(const S *, double *, int, int, int, bool, long long, long long,         \
+                                        cudaStream_t);                                                          \
+    template cudaError_t launch_unpack<S>(S *, const double *, int, int, int, bool, long long, long long,       \
+                                          cudaStream_t);                                                        \
     template cudaError_t launch_ghosts<S>(const FieldSet<S> &, int, int, int, int, cudaStream_t);              \
     template cudaError_t launch_ghost_pass<S>(const FieldSet<S> &, int, int, int, int, int, cudaStream_t);
 #define VAH_INSTANTIATE_STAGE(S)                                                                                \
