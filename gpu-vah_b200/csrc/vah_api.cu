@@ -3,11 +3,9 @@
 // An event owns its device state: conserved q (current) and qS (intermediate
 // stage), two (e, p) buffers used ping-pong across the two stages, and the
 // three velocity sets u (current), up (previous step) and uS (intermediate).
-// FP64 storage runs the face/cell split (or fused) kernels on the reference
-// layout. VAH_FP32 runs the FP32 form through the TMA-tiled stage kernel
-// (vah_tile.cuh): q and qS are then each one block of N_q fields, and every
-// field uses a row pitch padded to a multiple of 4 floats; the host-facing
-// copies convert to and from the reference layout.
+// Both storage types keep the reference layout and run the flux/cell split
+// (FP64 also the fused kernel); the host-facing copies widen and narrow FP32
+// fields.
 // No call ever exits or traps; failures come back as status codes.
 #include <cuda_runtime.h>
 
@@ -22,7 +20,6 @@
 #include "vah_ic_device.cuh"
 #include "vah_kernels.cuh"
 #include "vah_powf_exc.h"
-#include "vah_tile.cuh"
 
 using vah::FieldSet;
 using vah::StageArgs;
@@ -38,11 +35,13 @@ struct vah_event {
     cudaStream_t stream;
     bool own_stream;
     size_t elem;       // bytes per stored value: 8 (VAH_FP64) or 4 (VAH_FP32)
+    void *block;       // the state and the flux differences: one allocation
     void *q[16], *qS[16];
     void *ep[2][2];    // [buffer][0 = e, 1 = p]
     int cur;           // current (e, p) buffer
     void *u[4], *up[4], *uS[4];
-    void *D[3][16];    // flux differences per axis (scratch of a stage)
+    void *D[3][16];    // flux differences per axis of d_planes planes (scratch of a stage)
+    int d_planes;
     double *d_tab;
     uint32_t *d_exc;
     int nexc;
@@ -57,7 +56,6 @@ struct vah_event {
     bool validity;                   // fill the validity diagnostics every step
     double *vd[VAH_NUM_VALIDITY];    // validity fields (FP64, ghosted layout)
     void *vq[16];                    // P_L, pi, Pi at the start of the step (validity input)
-    vah::SplitConfig split;          // launch configuration of the face/cell kernels
     bool timing;
     std::vector<cudaEvent_t> tev;  // start/stop pairs of timed launches
     int tev_used;
@@ -65,16 +63,6 @@ struct vah_event {
     long long kernel_launches;
     cudaStream_t s_in, s_out;         // copy streams of the pipelined host-buffer step (created on first use)
     std::vector<cudaEvent_t> pev;     // its slab events
-    // FP32 form (tile layout)
-    bool tile;
-    void *qblock[2];                  // q and qS: nq fields each, ncell floats apart
-    void *pblock;                     // e, p of both buffers, then u, up, uS: 16 fields, ncell floats apart
-    vah::TileSlot h_tslot;            // the event's tile descriptor (host copy) ...
-    vah::TileSlot *d_tslot;           // ... and on the device
-    vah::TileItem *d_titems;
-    int ntitems;
-    unsigned *d_tcount, *d_terr;      // tile counter of a launch; kernel error flags
-    int tparity;                      // 0: u^n in the descriptor's uA; 1: in uB
 };
 
 namespace {
@@ -107,32 +95,7 @@ void *field_ptr(vah_event *ev, int id) {
 }
 
 void free_all(vah_event *ev) {
-    if (ev->tile) {
-        cudaFree(ev->qblock[0]);
-        cudaFree(ev->qblock[1]);
-        cudaFree(ev->pblock);
-        cudaFree(ev->d_tslot);
-        cudaFree(ev->d_titems);
-        cudaFree(ev->d_tcount);  // d_terr lives in the same allocation
-    } else {
-        for (int n = 0; n < 16; ++n) {
-            cudaFree(ev->q[n]);
-            cudaFree(ev->qS[n]);
-        }
-    }
-    if (!ev->tile) {
-        for (int b = 0; b < 2; ++b)
-            for (int m = 0; m < 2; ++m) cudaFree(ev->ep[b][m]);
-        for (int m = 0; m < 4; ++m) {
-            cudaFree(ev->u[m]);
-            cudaFree(ev->up[m]);
-            cudaFree(ev->uS[m]);
-        }
-    }
-    for (int d = 0; d < 3; ++d)
-        for (int n = 0; n < 16; ++n) {
-            cudaFree(ev->D[d][n]);
-        }
+    cudaFree(ev->block);
     cudaFree(ev->d_tab);
     cudaFree(ev->d_exc);
     cudaFree(ev->d_counters);
@@ -183,6 +146,7 @@ void fill_common(const vah_event *ev, StageArgs<S> &a) {
     a.counters = ev->d_counters;
     for (int d = 0; d < 3; ++d)
         for (int n = 0; n < 16; ++n) a.D[d][n] = (S *)ev->D[d][n];
+    a.d_planes = ev->d_planes;
     if (ev->validity)
         for (int m = 0; m < 11; ++m) a.regmap[m] = ev->vd[VAH_V_REGULATIONS + m];
 }
@@ -209,87 +173,13 @@ int timed(vah_event *ev, F launch) {
     return VAH_OK;
 }
 
-int timed_launch(vah_event *ev, const StageArgs<double> &a) {
+template <typename S>
+int timed_launch(vah_event *ev, const StageArgs<S> &a) {
     return timed(ev, [&]() {
-        if (ev->opt.flux == VAH_FLUX_PER_CELL_FUSED) return vah::launch_stage<double>(a, ev->opt.physics, ev->stream);
-        return vah::launch_stage_split<double>(a, ev->opt.physics, ev->opt.flux == VAH_FLUX_PER_CELL, ev->split,
-                                               ev->stream);
+        if constexpr (sizeof(S) == sizeof(double))
+            if (ev->opt.flux == VAH_FLUX_PER_CELL_FUSED) return vah::launch_stage<S>(a, ev->opt.physics, ev->stream);
+        return vah::launch_stage_split<S>(a, ev->opt.physics, ev->opt.flux == VAH_FLUX_PER_CELL, ev->stream);
     });
-}
-
-// One stage of the FP32 form: the persistent tile launch over the event's tiles.
-int tile_stage(vah_event *ev, int stage, double t, double dt) {
-    const vah::TileClock clk0{t, ev->tparity, 1, ev->steps};
-    const vah::Eos eos = make_eos(ev);
-    return timed(ev, [&]() {
-        return vah::tile_launch(ev->d_tslot, nullptr, clk0, dt, ev->d_titems, ev->ntitems, ev->lat.nz > 1,
-                                ev->d_tcount, stage, ev->opt.physics, eos, ev->d_terr, ev->stream);
-    });
-}
-
-}  // namespace
-
-namespace {
-
-// Copy the host tile descriptor to the device (after a buffer role changes).
-int tile_sync_desc(vah_event *ev) {
-    VAH_TRY(cudaMemcpyAsync(ev->d_tslot, &ev->h_tslot, sizeof(vah::TileSlot), cudaMemcpyHostToDevice, ev->stream));
-    VAH_TRY(cudaStreamSynchronize(ev->stream));  // the host copy may change again
-    return VAH_OK;
-}
-
-// The tile descriptor, tensor maps and work-list of an FP32 event.
-int tile_setup(vah_event *ev) {
-    vah::TileSlot &d = ev->h_tslot;
-    memset(&d, 0, sizeof(d));
-    for (int b = 0; b < 2; ++b) {
-        d.Q[b] = (float *)ev->qblock[b];
-        const int rc = vah::tile_encode_q(&d.tmQ[b], d.Q[b], ev->lat.nx, ev->lat.ny, ev->lat.nz, ev->ncx,
-                                          (long long)ev->ncell, ev->nq);
-        if (rc != VAH_OK) return rc;
-    }
-    for (int b = 0; b < 2; ++b)
-        for (int m = 0; m < 2; ++m) d.ep[b][m] = (float *)ev->ep[b == 0 ? ev->cur : 1 - ev->cur][m];
-    for (int m = 0; m < 4; ++m) {
-        d.uA[m] = (float *)ev->u[m];
-        d.uB[m] = (float *)ev->up[m];
-        d.uS[m] = (float *)ev->uS[m];
-    }
-    const int nx = ev->lat.nx, ny = ev->lat.ny, nz = ev->lat.nz;
-    const long long fs = (long long)ev->ncell;
-    for (int b = 0; b < 2; ++b) {
-        const int rc = vah::tile_encode_p(&d.tmEP[b], d.ep[b][0], nx, ny, nz, ev->ncx, fs, 2);
-        if (rc != VAH_OK) return rc;
-    }
-    float *const *us[3] = {d.uA, d.uB, d.uS};
-    for (int b = 0; b < 3; ++b) {
-        const int rc = vah::tile_encode_p(&d.tmU[b], us[b][0], nx, ny, nz, ev->ncx, fs, 4);
-        if (rc != VAH_OK) return rc;
-    }
-    d.fstride = (long long)ev->ncell;
-    d.nx = ev->lat.nx;
-    d.ny = ev->lat.ny;
-    d.nz = ev->lat.nz;
-    d.pitch = ev->ncx;
-    d.ncy = ev->ncy;
-    d.nq = ev->nq;
-    d.dx = ev->lat.dx;
-    d.dy = ev->lat.dy;
-    d.dz = ev->lat.dz;
-    d.dt = 0.0;  // events pass their step with each launch
-    d.etabar = ev->hydro.eta_over_s;
-    d.counters = ev->d_counters;
-    d.zghosts = zghosts_eager(ev);
-    VAH_TRY(cudaMalloc((void **)&ev->d_tslot, sizeof(vah::TileSlot)));
-    std::vector<vah::TileItem> items;
-    vah::tile_items(items, 0, ev->lat.nx, ev->lat.ny, ev->lat.nz);
-    ev->ntitems = (int)items.size();
-    VAH_TRY(cudaMalloc((void **)&ev->d_titems, items.size() * sizeof(vah::TileItem)));
-    VAH_TRY(cudaMemcpy(ev->d_titems, items.data(), items.size() * sizeof(vah::TileItem), cudaMemcpyHostToDevice));
-    VAH_TRY(cudaMalloc((void **)&ev->d_tcount, 2 * sizeof(unsigned)));
-    ev->d_terr = ev->d_tcount + 1;
-    VAH_TRY(cudaMemset(ev->d_tcount, 0, 2 * sizeof(unsigned)));
-    return tile_sync_desc(ev);
 }
 
 }  // namespace
@@ -423,8 +313,7 @@ extern "C" int vah_event_create(const vah_lattice *lat, const vah_hydro *hydro, 
     ev->hydro = *hydro;
     ev->opt = *opt;
     ev->nq = nq_of(opt->physics);
-    ev->tile = opt->precision == VAH_FP32;
-    ev->ncx = ev->tile ? vah::tile_pitch(lat->nx) : lat->nx + 4;  // row pitch of the device arrays
+    ev->ncx = lat->nx + 4;
     ev->ncy = lat->ny + 4;
     ev->ncz = lat->nz + 4;
     ev->ncell = (size_t)ev->ncx * ev->ncy * ev->ncz;
@@ -447,74 +336,51 @@ extern "C" int vah_event_create(const vah_lattice *lat, const vah_hydro *hydro, 
     memset(ev->vd, 0, sizeof(ev->vd));
     memset(ev->vq, 0, sizeof(ev->vq));
     ev->last_dt = 0.005;
-    ev->split = vah::default_split_config();
     ev->nexc = 0;
-    ev->qblock[0] = ev->qblock[1] = nullptr;
-    ev->pblock = nullptr;
-    ev->d_tslot = nullptr;
-    ev->d_titems = nullptr;
-    ev->d_tcount = ev->d_terr = nullptr;
-    ev->ntitems = 0;
-    ev->tparity = 0;
     ev->own_stream = opt->stream == nullptr;
     int rc = VAH_OK;
-    auto alloc = [&](void **p) {
-        if (rc != VAH_OK) return;
-        cudaError_t e = cudaMalloc(p, ev->ncell * ev->elem);
-        if (e == cudaSuccess) e = cudaMemset(*p, 0, ev->ncell * ev->elem);
-        if (e != cudaSuccess) rc = cuda_status(e);
-    };
     if (ev->own_stream) {
         if (cudaStreamCreateWithFlags(&ev->stream, cudaStreamNonBlocking) != cudaSuccess) rc = VAH_ERR_CUDA;
     } else {
         ev->stream = (cudaStream_t)opt->stream;
     }
-    if (ev->tile) {  // q and qS as blocks of nq fields (one tensor map each)
-        for (int b = 0; b < 2 && rc == VAH_OK; ++b) {
-            cudaError_t e = cudaMalloc(&ev->qblock[b], ev->nq * ev->ncell * sizeof(float));
-            if (e == cudaSuccess) e = cudaMemset(ev->qblock[b], 0, ev->nq * ev->ncell * sizeof(float));
-            if (e != cudaSuccess) rc = cuda_status(e);
-        }
-        if (rc == VAH_OK)
-            for (int n = 0; n < ev->nq; ++n) {
-                ev->q[n] = (float *)ev->qblock[0] + n * ev->ncell;
-                ev->qS[n] = (float *)ev->qblock[1] + n * ev->ncell;
-            }
-    } else {
-        for (int n = 0; n < 16; ++n)
-            if (n < ev->nq || (n == VAH_F_PI && ev->nq == 16)) {
-                alloc(&ev->q[n]);
-                alloc(&ev->qS[n]);
-            }
+    // one allocation: the state (2 N_q + 16 arrays), then the flux differences
+    // of as many planes as 1 GB holds (at least one; a stage runs slab by slab)
+    const bool split = opt->flux != VAH_FLUX_PER_CELL_FUSED || ev->elem == sizeof(float);
+    const int ndir = lat->nz > 1 ? 3 : 2;
+    const size_t plane = (size_t)ev->ncx * ev->ncy * ev->elem;
+    ev->d_planes = (int)std::min<size_t>(lat->nz, std::max<size_t>(1, ((size_t)1 << 30) / (plane * ndir * ev->nq)));
+    auto padded = [](size_t n) { return (n + 255) / 256 * 256; };
+    const size_t field = padded(ev->ncell * ev->elem), diff = padded(plane * ev->d_planes);
+    const size_t state = field * (2 * ev->nq + 16);
+    char *at = nullptr;
+    if (rc == VAH_OK) {
+        cudaError_t e = cudaMalloc(&ev->block, state + (split ? diff * ndir * ev->nq : 0));
+        if (e == cudaSuccess) e = cudaMemset(ev->block, 0, state);
+        if (e != cudaSuccess) rc = cuda_status(e);
+        at = (char *)ev->block;
     }
-    if (ev->tile) {  // the primitives as one block: (e, p) pairs and u quads are TMA boxes
-        if (rc == VAH_OK) {
-            cudaError_t e = cudaMalloc(&ev->pblock, 16 * ev->ncell * sizeof(float));
-            if (e == cudaSuccess) e = cudaMemset(ev->pblock, 0, 16 * ev->ncell * sizeof(float));
-            if (e != cudaSuccess) rc = cuda_status(e);
+    if (rc == VAH_OK) {
+        auto next = [&](size_t n) {
+            void *p = at;
+            at += n;
+            return p;
+        };
+        for (int n = 0; n < ev->nq; ++n) {
+            ev->q[n] = next(field);
+            ev->qS[n] = next(field);
         }
-        if (rc == VAH_OK) {
-            float *pb = (float *)ev->pblock;
-            for (int b = 0; b < 2; ++b)
-                for (int m = 0; m < 2; ++m) ev->ep[b][m] = pb + (2 * b + m) * ev->ncell;
-            for (int m = 0; m < 4; ++m) {
-                ev->u[m] = pb + (4 + m) * ev->ncell;
-                ev->up[m] = pb + (8 + m) * ev->ncell;
-                ev->uS[m] = pb + (12 + m) * ev->ncell;
-            }
-        }
-    } else {
         for (int b = 0; b < 2; ++b)
-            for (int m = 0; m < 2; ++m) alloc(&ev->ep[b][m]);
+            for (int m = 0; m < 2; ++m) ev->ep[b][m] = next(field);
         for (int m = 0; m < 4; ++m) {
-            alloc(&ev->u[m]);
-            alloc(&ev->up[m]);
-            alloc(&ev->uS[m]);
+            ev->u[m] = next(field);
+            ev->up[m] = next(field);
+            ev->uS[m] = next(field);
         }
+        if (split)
+            for (int d = 0; d < ndir; ++d)
+                for (int n = 0; n < ev->nq; ++n) ev->D[d][n] = next(diff);
     }
-    if (opt->flux != VAH_FLUX_PER_CELL_FUSED && !ev->tile)
-        for (int d = 0; d < (lat->nz > 1 ? 3 : 2); ++d)
-            for (int n = 0; n < ev->nq; ++n) alloc(&ev->D[d][n]);
     if (rc == VAH_OK && cudaMalloc((void **)&ev->d_fstage, ev->fstage * sizeof(double)) != cudaSuccess) rc = VAH_ERR_NOMEM;
     if (rc == VAH_OK && cudaMalloc((void **)&ev->d_counters, 4 * sizeof(unsigned long long)) != cudaSuccess)
         rc = VAH_ERR_NOMEM;
@@ -535,7 +401,6 @@ extern "C" int vah_event_create(const vah_lattice *lat, const vah_hydro *hydro, 
                 rc = VAH_ERR_CUDA;
         }
     }
-    if (rc == VAH_OK && ev->tile) rc = tile_setup(ev);
     if (rc != VAH_OK) {
         free_all(ev);
         delete ev;
@@ -821,18 +686,12 @@ int rk2_step_t(vah_event *ev, double t, double dt) {
     if (ev->validity)  // the diagnostics read P_L, pi, Pi as they are at the start of the step
         for (int n = VAH_F_PL; n < ev->nq; ++n)
             VAH_TRY(cudaMemcpyAsync(ev->vq[n], ev->q[n], ev->ncell * sizeof(S), cudaMemcpyDeviceToDevice, ev->stream));
-    int rc;
-    if (ev->tile) {
-        rc = tile_stage(ev, 1, t, dt);
-        if (rc == VAH_OK) rc = tile_stage(ev, 2, t, dt);
-    } else {
-        StageArgs<double> a;
-        stage1_args(ev, t, dt, a);
-        rc = timed_launch(ev, a);
-        if (rc != VAH_OK) return rc;
-        stage2_args(ev, t, dt, a);
-        rc = timed_launch(ev, a);
-    }
+    StageArgs<S> a;
+    stage1_args(ev, t, dt, a);
+    int rc = timed_launch(ev, a);
+    if (rc != VAH_OK) return rc;
+    stage2_args(ev, t, dt, a);
+    rc = timed_launch(ev, a);
     if (rc != VAH_OK || !ev->validity) return rc;
     ValidityArgs<S> v;
     memset(&v, 0, sizeof(v));
@@ -873,7 +732,6 @@ extern "C" int vah_rk2_step(vah_event *ev, double t, double dt) {
         ev->u[m] = ev->up[m];
         ev->up[m] = tmp;
     }
-    ev->tparity ^= 1;  // the tile descriptor keeps its buffers; the parity follows the swap
     ev->steps++;
     ev->last_t = t + dt;
     ev->last_dt = dt;
@@ -882,10 +740,10 @@ extern "C" int vah_rk2_step(vah_event *ev, double t, double dt) {
 
 namespace {
 
-// Time every candidate launch configuration of each split kind on the
-// event's current state, in stage-1 buffer roles (their outputs -- the face
-// buffers, qS, uS and the other (e, p) pair -- are scratch that the next step
-// rewrites), and keep the fastest. The device counters are restored after.
+// Time each split kind (`reps` launches after a warm-up) on the event's current
+// state, in stage-1 buffer roles (their outputs -- the difference buffers, qS,
+// uS and the other (e, p) pair -- are scratch that the next step rewrites).
+// Each kind has one launch configuration. The device counters are restored.
 int autotune_split(vah_event *ev, int reps, vah_tune_report *out) {
     StageArgs<double> a;
     stage1_args(ev, ev->last_t, ev->last_dt, a);
@@ -896,43 +754,22 @@ int autotune_split(vah_event *ev, int reps, vah_tune_report *out) {
     cudaEvent_t e0, e1;
     VAH_TRY(cudaEventCreate(&e0));
     VAH_TRY(cudaEventCreate(&e1));
+    auto launch = [&](int kind) {
+        return vah::launch_split_kind<double>(a, ev->opt.physics, exact, kind, ev->stream) == cudaSuccess;
+    };
     int rc = VAH_OK;
-    auto launch = [&](int kind, const vah::KindConfig &c) {
-        return vah::launch_split_kind<double>(a, ev->opt.physics, exact, kind, c, ev->stream);
-    };
-    auto time_one = [&](int kind, const vah::KindConfig &c, double *ms) -> int {
-        if (launch(kind, c) != cudaSuccess) return VAH_ERR_CUDA;  // warm-up
-        if (cudaEventRecord(e0, ev->stream) != cudaSuccess) return VAH_ERR_CUDA;
-        for (int r = 0; r < reps; ++r)
-            if (launch(kind, c) != cudaSuccess) return VAH_ERR_CUDA;
-        if (cudaEventRecord(e1, ev->stream) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess)
-            return VAH_ERR_CUDA;
-        float f = 0;
-        if (cudaEventElapsedTime(&f, e0, e1) != cudaSuccess) return VAH_ERR_CUDA;
-        *ms = f / reps;
-        return VAH_OK;
-    };
     out->nkinds = vah::kNumSplitKinds;
     for (int kind = 0; kind < vah::kNumSplitKinds && rc == VAH_OK; ++kind) {
-        vah_launch_choice &r = out->kind[kind];
-        const vah::KindConfig def = ev->split.k[kind];
-        r = {def.bx, def.by, def.minb, 0.0, 0.0};
+        // as 128-thread blocks: 4 flux blocks, 7 cell blocks of 64 per SM
+        out->kind[kind] = {32, 4, kind == vah::kCell ? 3 : 4, 0.0, 0.0};
         if (kind == vah::kFaceZ && ev->lat.nz == 1) continue;  // no eta faces in 2+1D
-        vah::KindConfig cand[16];
-        const int n = vah::split_candidates(kind, cand, 16);
-        double best = 1e300;
-        for (int i = 0; i < n && rc == VAH_OK; ++i) {
-            double ms = 0;
-            rc = time_one(kind, cand[i], &ms);
-            if (rc != VAH_OK) break;
-            if (cand[i].bx == def.bx && cand[i].by == def.by && cand[i].minb == def.minb) r.ms_default = ms;
-            if (ms < best) {
-                best = ms;
-                ev->split.k[kind] = cand[i];
-            }
-        }
-        const vah::KindConfig &b = ev->split.k[kind];
-        r = {b.bx, b.by, b.minb, r.ms_default, best};
+        bool ok = launch(kind) && cudaEventRecord(e0, ev->stream) == cudaSuccess;
+        for (int r = 0; r < reps && ok; ++r) ok = launch(kind);
+        float ms = 0;
+        if (!ok || cudaEventRecord(e1, ev->stream) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
+            cudaEventElapsedTime(&ms, e0, e1) != cudaSuccess)
+            rc = VAH_ERR_CUDA;
+        out->kind[kind].ms_default = out->kind[kind].ms_best = ms / reps;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -946,7 +783,7 @@ int autotune_split(vah_event *ev, int reps, vah_tune_report *out) {
 extern "C" int vah_event_autotune(vah_event *ev, int reps, vah_tune_report *out) {
     if (!ev || !out || reps < 1) return VAH_ERR_ARG;
     memset(out, 0, sizeof(*out));
-    if (ev->opt.flux == VAH_FLUX_PER_CELL_FUSED || ev->tile) return VAH_OK;  // one launch shape: nothing to tune
+    if (ev->opt.flux == VAH_FLUX_PER_CELL_FUSED || ev->elem == sizeof(float)) return VAH_OK;  // one launch shape: nothing to tune
     VAH_TRY(cudaSetDevice(ev->opt.device));
     return autotune_split(ev, reps, out);
 }
@@ -973,11 +810,6 @@ extern "C" int vah_event_set_validity(vah_event *ev, int on) {
         if (rc != VAH_OK) return rc;
     }
     ev->validity = on != 0;
-    if (ev->tile) {  // the tile kernel writes the regulator maps through its descriptor
-        for (int m = 0; m < 11; ++m) ev->h_tslot.regmap[m] = ev->validity ? ev->vd[VAH_V_REGULATIONS + m] : nullptr;
-        ev->h_tslot.zghosts = zghosts_eager(ev);
-        return tile_sync_desc(ev);
-    }
     return VAH_OK;
 }
 
@@ -1015,11 +847,6 @@ extern "C" int vah_event_sync(vah_event *ev) {
     VAH_TRY(cudaStreamSynchronize(ev->stream));
     unsigned long long c[4];
     VAH_TRY(cudaMemcpy(c, ev->d_counters, sizeof(c), cudaMemcpyDeviceToHost));
-    if (ev->tile) {  // a tile launch that gave up waiting for its copy (never expected)
-        unsigned err = 0;
-        VAH_TRY(cudaMemcpy(&err, ev->d_terr, sizeof(err), cudaMemcpyDeviceToHost));
-        if (err) return VAH_ERR_CUDA;
-    }
     return c[2] ? VAH_ERR_NAN : VAH_OK;
 }
 
@@ -1046,11 +873,6 @@ extern "C" int vah_event_track_fallbacks(vah_event *ev, int on) {
         VAH_TRY(cudaStreamSynchronize(ev->stream));
         VAH_TRY(cudaFree(ev->d_fb));
         ev->d_fb = nullptr;
-    }
-    if (ev->tile) {
-        ev->h_tslot.fallback1 = ev->d_fb;
-        ev->h_tslot.fallback2 = ev->d_fb ? ev->d_fb + ev->ncell : nullptr;
-        return tile_sync_desc(ev);
     }
     return VAH_OK;
 }
@@ -1223,13 +1045,13 @@ int step_host_pipelined(vah_event *ev, double t, double dt, double *const *field
             VAH_TRY(cudaStreamWaitEvent(ev->stream, in_ready[m], 0));
             a1.k0 = bound[m];
             a1.k1 = hi;
-            VAH_TRY(vah::launch_stage_split<double>(a1, ev->opt.physics, exact, ev->split, ev->stream));
+            VAH_TRY(vah::launch_stage_split<double>(a1, ev->opt.physics, exact, ev->stream));
         }
         if (m >= 1) {
             const int k = m - 1, lo = bound[k], hi = bound[k + 1];
             a2.k0 = lo;
             a2.k1 = hi;
-            VAH_TRY(vah::launch_stage_split<double>(a2, ev->opt.physics, exact, ev->split, ev->stream));
+            VAH_TRY(vah::launch_stage_split<double>(a2, ev->opt.physics, exact, ev->stream));
             VAH_TRY(cudaEventRecord(done[k], ev->stream));
             VAH_TRY(cudaStreamWaitEvent(ev->s_out, done[k], 0));
             const size_t p0 = k == 0 ? 0 : (size_t)lo + 2, p1 = k == nslab - 1 ? (size_t)nz + 4 : (size_t)hi + 2;
@@ -1275,33 +1097,15 @@ __global__ void widen_rows_kernel(FieldRows f, int hx, int pitch, size_t r0, siz
         dst[k] = (double)src[(k / hx) * pitch + k % hx];
 }
 
-// Slabs of whole tile layers along eta for the FP32 form's overlapped
-// host-buffer step: about `thick` planes each (rounded to tile layers, at
-// least one), as in slab_bounds. Returns the bounds in tile layers.
-std::vector<int> tile_slab_layers(int nz, int thick) {
-    constexpr int TZ = vah::TileShape<true>::TZ;
-    const int nlayer = (nz + TZ - 1) / TZ, per = std::max(1, (thick + TZ / 2) / TZ);
-    const int n = std::max(1, nlayer / per);
-    std::vector<int> b = {0};
-    for (int m = 0; m < n; ++m) b.push_back(b.back() + nlayer / n + (m < nlayer % n ? 1 : 0));
-    return b;
-}
-
 // Host-buffer step of the FP32 form (3+1D) with its copies overlapped, in the
-// slab order of step_host_pipelined. A slab is a run of whole tile layers, so
-// its tiles are one run of the k-major work-list, and its stage 1 or 2 is one
-// tile launch over that run. Its FP64 planes cross PCIe into a device copy of
-// the host layout (d_stage_all) and are narrowed into the FP32 fields on the
-// event's stream before its stage 1; after its stage 2 they are widened there
-// and copied back. Every slab but possibly the last has at least 4 planes, so
-// the 2-plane stencil halo of a slab lies in its neighbours, which is what the
-// order relies on.
+// slabs and the order of step_host_pipelined. A slab's FP64 planes cross PCIe
+// into a device copy of the host layout (d_stage_all) and are narrowed into
+// the FP32 fields on the event's stream before its stage 1; after its stage 2
+// they are widened there and copied back.
 int step_host_fp32_pipelined(vah_event *ev, double t, double dt, double *const *fields, int thick) {
-    constexpr int TZ = vah::TileShape<true>::TZ, TX = vah::TileShape<true>::TX, TY = vah::TileShape<true>::TY;
-    const int nx = ev->lat.nx, ny = ev->lat.ny, nz = ev->lat.nz, hx = nx + 4;
-    const std::vector<int> lb = tile_slab_layers(nz, thick);
-    const int nslab = (int)lb.size() - 1, per_layer = ((nx + TX - 1) / TX) * ((ny + TY - 1) / TY);
-    auto plane_of = [&](int layer) { return std::min(layer * TZ, nz); };  // interior plane of a slab bound
+    const int nz = ev->lat.nz, hx = ev->lat.nx + 4;
+    const std::vector<int> bound = slab_bounds(nz, thick);
+    const int nslab = (int)bound.size() - 1;
     const size_t hplane = (size_t)hx * ev->ncy, hn = hplane * ev->ncz;  // doubles per host plane, field
     if (!ev->d_stage_all) VAH_TRY(cudaMalloc((void **)&ev->d_stage_all, VAH_NUM_FIELDS * hn * sizeof(double)));
     if (!ev->s_in) VAH_TRY(cudaStreamCreateWithFlags(&ev->s_in, cudaStreamNonBlocking));
@@ -1353,12 +1157,13 @@ int step_host_fp32_pipelined(vah_event *ev, double t, double dt, double *const *
         VAH_TRY(cudaGetLastError());
         return VAH_OK;
     };
-    const vah::TileClock clk0{t, ev->tparity, 1, ev->steps};
-    const vah::Eos eos = make_eos(ev);
-    auto stage = [&](int st, int m) {
-        return vah::tile_launch(ev->d_tslot, nullptr, clk0, dt, ev->d_titems + (size_t)lb[m] * per_layer,
-                                (lb[m + 1] - lb[m]) * per_layer, true, ev->d_tcount, st, ev->opt.physics, eos,
-                                ev->d_terr, ev->stream);
+    StageArgs<float> a1, a2;
+    stage1_args(ev, t, dt, a1);
+    stage2_args(ev, t, dt, a2);
+    auto stage = [&](StageArgs<float> &a, int m) {
+        a.k0 = bound[m];
+        a.k1 = bound[m + 1];
+        return vah::launch_stage_split<float>(a, ev->opt.physics, false, ev->stream);
     };
     VAH_TRY(cudaEventRecord(start, ev->stream));  // after the work queued before this step
     VAH_TRY(cudaStreamWaitEvent(ev->s_in, start, 0));
@@ -1367,7 +1172,7 @@ int step_host_fp32_pipelined(vah_event *ev, double t, double dt, double *const *
     int rc = VAH_OK;
     for (int m = 0; m <= nslab && rc == VAH_OK; ++m) {
         if (m < nslab) {
-            const size_t need = m == nslab - 1 ? (size_t)nz + 4 : (size_t)plane_of(lb[m + 1]) + 4;
+            const size_t need = m == nslab - 1 ? (size_t)nz + 4 : (size_t)bound[m + 1] + 4;
             rc = copy_planes(true, loaded, need, ev->s_in);
             if (rc != VAH_OK) break;
             VAH_TRY(cudaEventRecord(in_ready[m], ev->s_in));
@@ -1375,11 +1180,11 @@ int step_host_fp32_pipelined(vah_event *ev, double t, double dt, double *const *
             rc = convert(true, loaded, need);
             if (rc != VAH_OK) break;
             loaded = need;
-            VAH_TRY(stage(1, m));
+            VAH_TRY(stage(a1, m));
         }
         if (m >= 1) {
-            const int k = m - 1, lo = plane_of(lb[k]), hi = plane_of(lb[k + 1]);
-            VAH_TRY(stage(2, k));
+            const int k = m - 1, lo = bound[k], hi = bound[k + 1];
+            VAH_TRY(stage(a2, k));
             const size_t p0 = k == 0 ? 0 : (size_t)lo + 2, p1 = k == nslab - 1 ? (size_t)nz + 4 : (size_t)hi + 2;
             rc = convert(false, p0, p1);
             if (rc != VAH_OK) break;
@@ -1397,7 +1202,6 @@ int step_host_fp32_pipelined(vah_event *ev, double t, double dt, double *const *
         ev->u[m] = ev->up[m];
         ev->up[m] = tmp;
     }
-    ev->tparity ^= 1;
     ev->steps++;
     ev->last_t = t + dt;
     ev->last_dt = dt;
@@ -1412,15 +1216,14 @@ extern "C" int vah_rk2_step_host(vah_event *ev, double t, double dt, double *con
     int rc;
     // overlapped copies where the lattice has enough planes along eta (at
     // least 3 slabs); slab thickness from VAH_HOST_SLAB_PLANES (>= 2) when
-    // set, else nz / 6 (6 slabs: the best of 3 to 40 on the 121x121x81 event;
-    // the FP32 form rounds it to whole tile layers)
+    // set, else nz / 6 (6 slabs: the best of 3 to 40 on the 121x121x81 event)
     static const int slab_env = [] {
         const char *v = getenv("VAH_HOST_SLAB_PLANES");
         return v ? atoi(v) : 0;
     }();
     const int slab = slab_env >= 2 ? slab_env : std::max(2, ev->lat.nz / 6);
     if (ev->elem != sizeof(double)) {
-        if (ev->lat.nz > 1 && !ev->validity && tile_slab_layers(ev->lat.nz, slab).size() >= 4) {
+        if (!ev->validity && ev->lat.nz >= 3 * slab) {
             if (!(dt > 0) || !(t > 0)) return VAH_ERR_ARG;
             return step_host_fp32_pipelined(ev, t, dt, fields, slab);
         }

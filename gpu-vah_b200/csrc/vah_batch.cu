@@ -1,20 +1,18 @@
 // vah_batch.cu -- many events, one persistent launch per kernel kind.
 //
 // A batch holds up to kMaxSlots events of independent grid sizes. Every
-// launch of a step covers all events: a persistent grid of blocks walks a
-// work-list of 32x4 tiles (event slot, tile origin), each block a contiguous
-// run of it, so events of uneven sizes share one launch and the GPU is filled
-// even by many small events.
+// launch of a step covers all events: a block takes an item of a work-list
+// (event slot, part of it), largest event first, so events of uneven sizes
+// share one launch and the GPU is filled even by many small events.
 // The per-event state lives in one device allocation per event (stream-
 // ordered, from the batch's memory pool); per-event descriptors (buffer
 // pointers, geometry) and clocks (time, u/u_prev parity, step count) live in
 // device arrays, so a whole RK2 step -- face and cell launches of both stages
 // plus the clock advance -- is captured once as a CUDA graph and replayed.
 // The graph is re-captured only when events are added or removed.
-// VAH_FP32 batches run the FP32 form on the TMA-tiled stage kernel
-// (vah_tile.cuh): one persistent launch per stage and tile shape (2+1D and
-// 3+1D events), each slot with a row pitch padded to 4 floats and a tile
-// descriptor (tensor maps over its q and qS blocks) admitted with it.
+// The flux differences of a stage are scratch that events share: where one
+// scratch of kScratchBytes does not hold every event's, the events are stepped
+// in groups that it holds.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -28,7 +26,7 @@
 #include "vah_kernels.cuh"
 #include "vah_march.cuh"
 #include "vah_powf_exc.h"
-#include "vah_tile.cuh"
+#include "vah_tile_cell.cuh"
 
 namespace vah {
 namespace {
@@ -42,7 +40,7 @@ struct SlotDesc {
     long long plane;
     double dx, dy, dz, dt, etabar;
     S *q[16], *qS[16], *ep[2][2], *uA[4], *uB[4], *uS[4];
-    S *D[3][16];  // flux differences per axis (FP64 form)
+    S *D[3][16];  // flux differences per axis, in the shared scratch
     unsigned char *fallback;  // per ghosted cell: 1 where the latest cell inversion fell back
     unsigned char *hot;       // per ghosted cell: 1 while e > e_freeze (freeze-out crossings)
     double e_freeze;
@@ -56,130 +54,124 @@ struct SlotClock {
     int active;
     long long steps;
 };
-// the tile kernel reads the batch's clocks as TileClock
-static_assert(sizeof(SlotClock) == sizeof(TileClock) && offsetof(SlotClock, parity) == offsetof(TileClock, parity) &&
-                  offsetof(SlotClock, t) == offsetof(TileClock, t),
-              "SlotClock and TileClock share a layout");
 
-// One block's piece of work: a 32x4 tile of cells (cell kinds: its origin i0
-// and row r0), four strips of flux_x (from strip i0) or four strips of
-// flux_march (from strip i0) over the cells [r0, r1) along its axis.
+// One block's piece of work: four strips (from strip i0) of flux_x (kind 0) or
+// of flux_march along y or eta (kind 1, 2) over the cells [r0, r1) along it; or
+// the 128 interior cells from i0 (cell lists).
 struct WorkItem {
-    int slot, i0, r0, r1;
+    int slot, kind, i0, r0, r1;
 };
+constexpr int kCellItem = kTX * kTY;
 
-enum { K_FX = 0, K_FY = 1, K_FZ = 2, K_C2 = 3, K_C3 = 4, K_NUM = 5 };
+// The work-lists: fluxes, 2+1D cells, 3+1D cells.
+enum { K_FLUX = 0, K_C2 = 1, K_C3 = 2, K_NUM = 3 };
 
-// StageArgs of one slot and stage (the buffer roles of vah_rk2_step).
+// StageArgs of one slot and stage (the buffer roles of vah_rk2_step), filled by
+// 96 threads together (tid 0 to 95).
 template <typename S>
-__device__ void make_args(StageArgs<S> &a, const SlotDesc<S> &d, const SlotClock &c, int stage, const Eos &eos) {
-    a.nx = d.nx;
-    a.ny = d.ny;
-    a.nz = d.nz;
-    a.k0 = 0;
-    a.k1 = d.nz;
-    a.ncx = d.ncx;
-    a.ncy = d.ncy;
-    a.plane = d.plane;
-    a.dx = d.dx;
-    a.dy = d.dy;
-    a.dz = d.dz;
-    a.dt = d.dt;
-    a.etabar = d.etabar;
-    a.t_src = stage == 1 ? c.t : c.t + d.dt;
-    a.t_inv = c.t + d.dt;
-    a.stage2 = stage == 2;
-    a.zghosts = d.nz > 1;  // 2+1D: the eta ghost layers are filled when a caller reads them
-    a.eos = eos;
-    a.counters = d.counters;
-    a.fallback = d.fallback;
-    for (int m = 0; m < 11; ++m) a.regmap[m] = nullptr;  // validity diagnostics are an event-path option
-    a.hot = d.hot;
-    a.e_freeze = d.e_freeze;
-    a.crossings = d.crossings;
-    S *const *u = c.parity ? d.uB : d.uA;
-    S *const *up = c.parity ? d.uA : d.uB;
-    for (int n = 0; n < 16; ++n) {
-        a.qin[n] = stage == 1 ? d.q[n] : d.qS[n];
-        a.qout[n] = stage == 1 ? d.qS[n] : d.q[n];
-        a.qavg[n] = d.q[n];
+__device__ void make_args(StageArgs<S> &a, const SlotDesc<S> &d, const SlotClock &c, int stage, const Eos &eos, int tid) {
+    const int warp = tid >> 5, n = tid & 31;
+    if (warp == 0) {
+        if (n < 16) {
+            a.qin[n] = stage == 1 ? d.q[n] : d.qS[n];
+            a.qout[n] = stage == 1 ? d.qS[n] : d.q[n];
+            a.qavg[n] = d.q[n];
+            for (int k = 0; k < 3; ++k) a.D[k][n] = d.D[k][n];
+        } else if (n < 20) {
+            const int m = n - 16;
+            S *u = c.parity ? d.uB[m] : d.uA[m], *up = c.parity ? d.uA[m] : d.uB[m];
+            a.uin[m] = stage == 1 ? u : d.uS[m];
+            a.upin[m] = stage == 1 ? up : u;
+            a.guess[m] = u;
+            a.uout[m] = stage == 1 ? d.uS[m] : up;
+        } else if (n < 31) {
+            a.regmap[n - 20] = nullptr;  // validity diagnostics are an event-path option
+        }
+    } else if (tid == 32) {
+        a.nx = d.nx;
+        a.ny = d.ny;
+        a.nz = d.nz;
+        a.k0 = 0;
+        a.k1 = d.nz;
+        a.ncx = d.ncx;
+        a.ncy = d.ncy;
+        a.plane = d.plane;
+        a.stage2 = stage == 2;
+        a.zghosts = d.nz > 1;  // 2+1D: the eta ghost layers are filled when a caller reads them
+        a.d_planes = 0;
+        a.eos = eos;
+        a.counters = d.counters;
+        a.fallback = d.fallback;
+        a.hot = d.hot;
+        a.e_freeze = d.e_freeze;
+        a.crossings = d.crossings;
+        a.ein = d.ep[stage == 1 ? 0 : 1][0];
+        a.pin = d.ep[stage == 1 ? 0 : 1][1];
+        a.eout = d.ep[stage == 1 ? 1 : 0][0];
+        a.pout = d.ep[stage == 1 ? 1 : 0][1];
+    } else if (tid == 64) {
+        a.dx = d.dx;
+        a.dy = d.dy;
+        a.dz = d.dz;
+        a.dt = d.dt;
+        a.etabar = d.etabar;
+        a.t_inv = c.t + d.dt;
+        a.t_src = stage == 1 ? c.t : c.t + d.dt;
+        finish_args(a);
     }
-    for (int m = 0; m < 4; ++m) {
-        a.uin[m] = stage == 1 ? u[m] : d.uS[m];
-        a.upin[m] = stage == 1 ? up[m] : u[m];
-        a.guess[m] = u[m];
-        a.uout[m] = stage == 1 ? d.uS[m] : up[m];
-    }
-    a.ein = d.ep[stage == 1 ? 0 : 1][0];
-    a.pin = d.ep[stage == 1 ? 0 : 1][1];
-    a.eout = d.ep[stage == 1 ? 1 : 0][0];
-    a.pout = d.ep[stage == 1 ? 1 : 0][1];
-    for (int k = 0; k < 3; ++k)
-        for (int n = 0; n < 16; ++n) a.D[k][n] = d.D[k][n];
-    finish_args(a);
 }
 
-// Items are taken from the work-list in chunks through an atomic counter
-// (reset before each launch): blocks that finish early take more, so uneven
-// events do not leave a tail; the list runs largest event first. A march item
-// is a whole segment of four strips, so those go one by one.
-template <int KIND>
-constexpr int kChunk = KIND == K_FY || KIND == K_FZ ? 1 : 4;
+// Both stages' arguments of every active slot, once per step (block: a slot,
+// threadIdx.y: the stage): the stage launches' blocks copy theirs from there.
+template <typename S>
+__global__ void args_kernel(const SlotDesc<S> *__restrict__ descs, const SlotClock *__restrict__ clk, const Eos eos,
+                            StageArgs<S> *args) {
+    const int slot = blockIdx.x;
+    if (clk[slot].active) make_args(args[2 * slot + threadIdx.y], descs[slot], clk[slot], threadIdx.y + 1, eos, threadIdx.x);
+}
 
-// The register caps of the event launches (vah_kernels.cuh).
-template <int KIND>
-constexpr int kKindMinb = KIND == K_FX ? kFluxXMinb : (KIND <= K_FZ ? kMarchMinb : kCellMinb);
+// A block's copy of its item's arguments into shared memory; a barrier before use.
+template <typename S>
+__device__ __forceinline__ void copy_args(StageArgs<S> &sa, const StageArgs<S> *from, int tid) {
+    static_assert(sizeof(StageArgs<S>) % 8 == 0, "copied by 8-byte words");
+    const double *src = (const double *)from;
+    for (int k = tid; k < (int)(sizeof(StageArgs<S>) / 8); k += kTX * kTY) ((double *)&sa)[k] = __ldg(src + k);
+}
 
-template <int PHYS, int KIND, bool EXACT>
-__global__ void __launch_bounds__(kTX *kTY, kKindMinb<KIND>) batch_kernel(const SlotDesc<double> *__restrict__ descs,
-                                                               const SlotClock *__restrict__ clk,
-                                                               const WorkItem *__restrict__ work, int nwork, int stage,
-                                                               const Eos eos, unsigned *next) {
-    extern __shared__ double march_sm[];  // march kinds: each warp's columns
-    __shared__ StageArgs<double> sa;
-    __shared__ HalfPointers hp;
-    __shared__ int sa_slot, s_w0;
-    const bool lead = threadIdx.x == 0 && threadIdx.y == 0;
-    const int warp = threadIdx.y;  // blockDim.x == 32
-    if (lead) sa_slot = -1;
-    for (;;) {
-        __syncthreads();  // s_w0 of the previous chunk has been read
-        if (lead) s_w0 = (int)atomicAdd(next, (unsigned)kChunk<KIND>);
-        __syncthreads();
-        const int w0 = s_w0, w1 = min(nwork, w0 + kChunk<KIND>);
-        if (w0 >= nwork) break;
-        // the per-event arguments in shared memory change only at event boundaries
-        for (int w = w0; w < w1; ++w) {
-            const WorkItem it = work[w];
-            __syncthreads();
-            const bool changed = it.slot != sa_slot;
-            __syncthreads();
-            if (changed) {
-                if (lead) {
-                    make_args(sa, descs[it.slot], clk[it.slot], stage, eos);
-                    sa_slot = it.slot;
-                }
-                __syncthreads();
-                if (KIND <= K_FZ) {
-                    set_half_pointers<PHYS>(hp, sa, threadIdx.y * kTX + threadIdx.x);
-                    __syncthreads();
-                }
-            }
-            if (KIND == K_FX) {
-                if (it.i0 + warp < flux_x_strips(sa.nx, sa.ny, sa.nz)) flux_x<PHYS, EXACT>(sa, hp, it.i0 + warp);
-            } else if (KIND <= K_FZ) {
-                if (it.i0 + warp < march_strips(sa.nx * (KIND == K_FY ? sa.nz : sa.ny)))
-                    flux_march<PHYS, KIND == K_FY ? 1 : 2, EXACT>(sa, hp, it.i0 + warp, it.r0, it.r1,
-                                                                  march_sm + warp * kMarchDoubles<PHYS>);
-            } else {
-                const int i = it.i0 + threadIdx.x, r = it.r0 + threadIdx.y;
-                if (i < sa.nx && r < sa.ny * sa.nz) {
-                    const int j = r % sa.ny, k = r / sa.ny;
-                    cell_compute<double, PHYS, KIND == K_C3, true>(sa, i + 2, j + 2, k + 2);
-                }
-            }
-        }
+template <typename S, int PHYS, bool EXACT>
+__global__ void __launch_bounds__(kTX *kTY, kFluxMinb<S>)
+    batch_flux_kernel(const StageArgs<S> *__restrict__ args, const WorkItem *__restrict__ work, int stage) {
+    extern __shared__ __align__(16) unsigned char march_sm[];  // marches: each warp's columns
+    __shared__ StageArgs<S> sa;
+    __shared__ TablePointers<S> tab;
+    const WorkItem it = work[blockIdx.x];
+    const StageArgs<S> *from = args + 2 * it.slot + stage - 1;
+    const int warp = threadIdx.x / 32, strip = it.i0 + warp;
+    copy_args(sa, from, threadIdx.x);
+    set_table_pointers<PHYS>(tab, *from, threadIdx.x);
+    __syncthreads();
+    S *sm = (S *)march_sm + warp * kMarchValues<S, PHYS>;
+    if (it.kind == 0) {
+        if (strip < flux_x_strips<S>(sa.nx, sa.ny, sa.nz)) flux_x<PHYS, EXACT>(sa, tab, strip);
+    } else if (it.kind == 1) {
+        if (strip < march_strips<S>(sa.nx * sa.nz)) flux_march<PHYS, 1, EXACT>(sa, tab, strip, it.r0, it.r1, sm);
+    } else {
+        if (strip < march_strips<S>(sa.nx * sa.ny)) flux_march<PHYS, 2, EXACT>(sa, tab, strip, it.r0, it.r1, sm);
     }
+}
+
+template <typename S, int PHYS, bool IS3D>
+__global__ void __launch_bounds__(kTX *kTY, kCellMinb<S, IS3D> / 2)
+    batch_cell_kernel(const StageArgs<S> *__restrict__ args, const WorkItem *__restrict__ work, int stage) {
+    __shared__ StageArgs<S> sa;
+    const WorkItem it = work[blockIdx.x];
+    copy_args(sa, args + 2 * it.slot + stage - 1, threadIdx.x);
+    __syncthreads();
+    const int c = it.i0 + threadIdx.x;
+    if (c >= sa.nx * sa.ny * sa.nz) return;
+    const int r = c / sa.nx, i = c - r * sa.nx, k = r / sa.ny, j = r - k * sa.ny;
+    if constexpr (sizeof(S) == 4) cell_compute_f32<PHYS, IS3D>(sa, i + 2, j + 2, k + 2);
+    else cell_compute<S, PHYS, IS3D, true>(sa, i + 2, j + 2, k + 2);
 }
 
 // End of a step: the clock moves on, and the freeze-out surface volume takes
@@ -220,10 +212,10 @@ __global__ void max_e_kernel(const SlotDesc<S> *__restrict__ descs, const WorkIt
     for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
         const WorkItem it = work[w];
         const SlotDesc<S> &d = descs[it.slot];
-        const int i = it.i0 + threadIdx.x, r = it.r0 + threadIdx.y;
+        const int cell = it.i0 + threadIdx.y * kTX + threadIdx.x;
         double v = 0.0;
-        if (i < d.nx && r < d.ny * d.nz) {
-            const int j = r % d.ny, k = r / d.ny;
+        if (cell < d.nx * d.ny * d.nz) {
+            const int r = cell / d.nx, i = cell - r * d.nx, j = r % d.ny, k = r / d.ny;
             const long long s = (i + 2) + (long long)d.ncx * (j + 2) + d.plane * (k + 2);
             v = (double)d.ep[cur_ep][0][s];
             if (!(v > 0.0) || d.fallback[s]) v = 0.0;
@@ -237,10 +229,10 @@ __global__ void max_e_kernel(const SlotDesc<S> *__restrict__ descs, const WorkIt
     }
 }
 
-// Per-tile partial sums of the event observables (tau T^tt, T^xx - T^yy,
+// Per-item partial sums of the event observables (tau T^tt, T^xx - T^yy,
 // T^xx + T^yy, e u^t u_T, e u^t) in FP64 over the cells whose latest
 // inversion converged (a fallback cell's state is not a solution), one row
-// per cell tile; the host adds the rows of each slot in a fixed order.
+// per cell item; the host adds the rows of each slot in a fixed order.
 template <typename S, int PHYS>
 __global__ void observables_kernel(const SlotDesc<S> *__restrict__ descs, const SlotClock *__restrict__ clk,
                                    const WorkItem *__restrict__ work, int nwork, double *partial) {
@@ -250,10 +242,10 @@ __global__ void observables_kernel(const SlotDesc<S> *__restrict__ descs, const 
         const WorkItem it = work[w];
         const SlotDesc<S> &d = descs[it.slot];
         const SlotClock c = clk[it.slot];
-        const int i = it.i0 + threadIdx.x, r = it.r0 + threadIdx.y;
+        const int cell = it.i0 + tid;
         double acc[5] = {0, 0, 0, 0, 0};
-        const bool in = i < d.nx && r < d.ny * d.nz;
-        const int j = in ? r % d.ny : 0, k = in ? r / d.ny : 0;
+        const bool in = cell < d.nx * d.ny * d.nz;
+        const int r = in ? cell / d.nx : 0, i = in ? cell - r * d.nx : 0, j = r % d.ny, k = r / d.ny;
         const long long s = (i + 2) + (long long)d.ncx * (j + 2) + d.plane * (k + 2);
         if (in && !d.fallback[s]) {  // converged cells only
             S *const *u = c.parity ? d.uB : d.uA;
@@ -286,41 +278,6 @@ __global__ void observables_kernel(const SlotDesc<S> *__restrict__ descs, const 
             partial[(size_t)w * 5 + tid] = s;
         }
     }
-}
-
-template <int PHYS, int KIND>
-constexpr size_t kBatchSmem = KIND == K_FY || KIND == K_FZ ? kTY * kMarchDoubles<PHYS> * sizeof(double) : 0;
-
-template <int PHYS, int KIND, bool EXACT>
-int blocks_per_sm() {
-    static int cached = 0;
-    if (!cached) {
-        int n = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, batch_kernel<PHYS, KIND, EXACT>, kTX * kTY,
-                                                          kBatchSmem<PHYS, KIND>) != cudaSuccess ||
-            n < 1)
-            n = 1;
-        cached = n;
-    }
-    return cached;
-}
-
-// A persistent grid of (SMs x resident blocks) walks the work-list.
-template <int PHYS, int KIND, bool EXACT>
-cudaError_t launch_kind(const SlotDesc<double> *descs, const SlotClock *clk, const WorkItem *work, int nwork, int stage,
-                        const Eos &eos, int sms, unsigned *next, cudaStream_t stream) {
-    if (nwork <= 0) return cudaSuccess;
-    constexpr size_t smem = kBatchSmem<PHYS, KIND>;
-    cudaError_t e = cudaSuccess;
-    if (smem)
-        e = cudaFuncSetAttribute(batch_kernel<PHYS, KIND, EXACT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)smem);
-    if (e != cudaSuccess) return e;
-    const int grid = std::min((nwork + kChunk<KIND> - 1) / kChunk<KIND>, sms * blocks_per_sm<PHYS, KIND, EXACT>());
-    if ((e = cudaMemsetAsync(next, 0, sizeof(unsigned), stream)) != cudaSuccess) return e;
-    batch_kernel<PHYS, KIND, EXACT><<<grid, dim3(kTX, kTY), smem, stream>>>(descs, clk, work, nwork, stage, eos,
-                                                                                  next);
-    return cudaGetLastError();
 }
 
 }  // namespace
@@ -367,16 +324,19 @@ struct vah_batch {
     double *d_fstage;  // staging of the field reads ...
     size_t fstage;     // ... of this many values
     WorkItem *d_work[vah::K_NUM];
-    // FP32 form: tile descriptors per slot, tile work-lists (2+1D, 3+1D), launch counter and error flags
-    bool tile;
-    vah::TileSlot *d_tdesc;  // [kMaxSlots]
-    vah::TileItem *d_titems[2];
-    int ntitems[2], cap_titems[2];
-    unsigned *d_tcount;      // [0]: tile counter, [1]: error flags
-    unsigned *d_wcount;      // [K_NUM] work-list counters of the face/cell launches
-    int nwork[vah::K_NUM], cap_work[vah::K_NUM];
+    void *d_args;        // StageArgs<S>[cap_args]: both stages' arguments by slot
+    size_t cap_args;     // in StageArgs
+    int nslots;          // slots up to the last one in use
+    char *d_scratch;     // the flux differences of one group of events
+    size_t cap_scratch;
+    struct Group {
+        int first[vah::K_NUM], count[vah::K_NUM];  // its runs of the work-lists
+    };
+    std::vector<Group> groups;
+    int nwork[vah::K_NUM];
+    size_t cap_work[vah::K_NUM];
     double *d_partial;
-    int cap_partial;
+    size_t cap_partial;
     bool dirty;
     cudaGraphExec_t graph;
     bool has_graph;
@@ -404,20 +364,17 @@ int cuda_status(cudaError_t e) {
 int nq_of(int physics) { return physics == VAH_IDEAL ? 5 : (physics == VAH_PIMUNU ? 15 : 16); }
 
 // Arrays of one event in its allocation: 16 q, 16 qS, 4 e/p, 4 uA, 4 uB,
-// 4 uS, and the flux differences per axis; then one byte per cell of fallback flags and one of freeze-out state.
-int arrays_per_event(const vah_batch *b, const vah_lattice *lat) {
-    if (b->tile) return 48;  // the tile kernel keeps its face fluxes on chip
-    const int ndir = lat->nz > 1 ? 3 : 2;
-    return 48 + ndir * b->nq;
-}
+// 4 uS; then one byte per cell of fallback flags and one of freeze-out state.
+constexpr int kArraysPerEvent = 48;
 
-// Row pitch of a slot's arrays: nx + 4, padded to 4 floats for the tile form.
-int slot_pitch(const vah_batch *b, int nx) { return b->tile ? vah::tile_pitch(nx) : nx + 4; }
+// The scratch that a group's flux differences share; an event that needs more
+// is a group of its own. With 1 GB the 256-event batch is one group.
+constexpr size_t kScratchBytes = (size_t)1 << 30;
 
 size_t event_bytes(const vah_batch *b, const vah_lattice *lat) {
-    const size_t ncell = (size_t)slot_pitch(b, lat->nx) * (lat->ny + 4) * (lat->nz + 4);
+    const size_t ncell = (size_t)(lat->nx + 4) * (lat->ny + 4) * (lat->nz + 4);
     const size_t per = (ncell * b->elem + 255) / 256 * 256;
-    return per * arrays_per_event(b, lat) + 2 * ((ncell + 255) / 256 * 256) + 256;
+    return per * kArraysPerEvent + 2 * ((ncell + 255) / 256 * 256) + 256;
 }
 
 vah::Eos batch_eos(const vah_batch *b) {
@@ -462,7 +419,7 @@ int fill_slot(vah_batch *b, int slot) {
     d.nx = sl.lat.nx;
     d.ny = sl.lat.ny;
     d.nz = sl.lat.nz;
-    d.ncx = slot_pitch(b, sl.lat.nx);
+    d.ncx = sl.lat.nx + 4;
     d.ncy = sl.lat.ny + 4;
     d.plane = (long long)d.ncx * d.ncy;
     d.dx = sl.lat.dx;
@@ -487,10 +444,6 @@ int fill_slot(vah_batch *b, int slot) {
     for (int m = 0; m < 4; ++m) d.uA[m] = next();
     for (int m = 0; m < 4; ++m) d.uB[m] = next();
     for (int m = 0; m < 4; ++m) d.uS[m] = next();
-    const int ndir = sl.lat.nz > 1 ? 3 : 2;
-    if (!b->tile)
-        for (int k = 0; k < ndir; ++k)
-            for (int n = 0; n < b->nq; ++n) d.D[k][n] = next();
     d.fallback = (unsigned char *)(base + off);
     d.hot = (unsigned char *)(base + off + (ncell + 255) / 256 * 256);
     d.e_freeze = energy_at_temperature(b, sl.hydro.freezeout_T_GeV / 0.197326938);
@@ -498,207 +451,183 @@ int fill_slot(vah_batch *b, int slot) {
     *desc_host<S>(b, slot) = d;
     VAH_TRY(cudaMemcpyAsync((char *)b->d_desc + sizeof(SlotDesc<S>) * slot, &d, sizeof(d), cudaMemcpyHostToDevice,
                             b->stream));
-    if (b->tile) {  // the FP32 form's tile descriptor: the same buffers, q and qS as blocks of per-byte fields
-        vah::TileSlot t;
-        memset(&t, 0, sizeof(t));
-        t.Q[0] = (float *)d.q[0];
-        t.Q[1] = (float *)d.qS[0];
-        t.fstride = (long long)(per / sizeof(float));
-        for (int bb = 0; bb < 2; ++bb) {
-            const int rc = vah::tile_encode_q(&t.tmQ[bb], t.Q[bb], sl.lat.nx, sl.lat.ny, sl.lat.nz, d.ncx, t.fstride,
-                                              b->nq);
-            if (rc != VAH_OK) return rc;
-        }
-        for (int x = 0; x < 2; ++x)
-            for (int y = 0; y < 2; ++y) t.ep[x][y] = (float *)d.ep[x][y];
-        for (int m = 0; m < 4; ++m) {
-            t.uA[m] = (float *)d.uA[m];
-            t.uB[m] = (float *)d.uB[m];
-            t.uS[m] = (float *)d.uS[m];
-        }
-        // the slot's arrays follow one another `per` bytes apart: (e, p) pairs and u quads are blocks
-        for (int bb = 0; bb < 2; ++bb) {
-            const int rc = vah::tile_encode_p(&t.tmEP[bb], t.ep[bb][0], sl.lat.nx, sl.lat.ny, sl.lat.nz, d.ncx,
-                                              t.fstride, 2);
-            if (rc != VAH_OK) return rc;
-        }
-        float *const *us[3] = {t.uA, t.uB, t.uS};
-        for (int bb = 0; bb < 3; ++bb) {
-            const int rc = vah::tile_encode_p(&t.tmU[bb], us[bb][0], sl.lat.nx, sl.lat.ny, sl.lat.nz, d.ncx,
-                                              t.fstride, 4);
-            if (rc != VAH_OK) return rc;
-        }
-        t.nx = d.nx;
-        t.ny = d.ny;
-        t.nz = d.nz;
-        t.pitch = d.ncx;
-        t.ncy = d.ncy;
-        t.nq = b->nq;
-        t.dx = d.dx;
-        t.dy = d.dy;
-        t.dz = d.dz;
-        t.dt = d.dt;
-        t.etabar = d.etabar;
-        t.counters = d.counters;
-        t.zghosts = d.nz > 1;      // 2+1D: the eta ghost layers are filled when a caller reads them
-        t.fallback2 = d.fallback;  // the batch keeps the latest (stage-2) flags
-        t.hot = d.hot;
-        t.e_freeze = d.e_freeze;
-        t.crossings = d.crossings;
-        // a pageable source: the copy is staged before the call returns (the slot's next use is stream-ordered)
-        VAH_TRY(cudaMemcpy(b->d_tdesc + slot, &t, sizeof(t), cudaMemcpyHostToDevice));
-    }
     return VAH_OK;
 }
 
-int rebuild_tiles(vah_batch *b) {
-    std::vector<vah::TileItem> lists[2];  // 2+1D, 3+1D events
-    for (int s = 0; s < (int)b->slots.size(); ++s) {
-        const vah_batch::Slot &sl = b->slots[s];
-        if (sl.used) vah::tile_items(lists[sl.lat.nz > 1 ? 1 : 0], s, sl.lat.nx, sl.lat.ny, sl.lat.nz);
-    }
-    for (int k = 0; k < 2; ++k) {
-        const int n = (int)lists[k].size();
-        if (n > b->cap_titems[k]) {
-            if (b->d_titems[k]) VAH_TRY(cudaFreeAsync(b->d_titems[k], b->stream));
-            const int cap = std::max(n, 2 * b->cap_titems[k]);
-            VAH_TRY(cudaMallocFromPoolAsync((void **)&b->d_titems[k], cap * sizeof(vah::TileItem), b->pool, b->stream));
-            b->cap_titems[k] = cap;
-        }
-        if (n) VAH_TRY(cudaMemcpyAsync(b->d_titems[k], lists[k].data(), n * sizeof(vah::TileItem),
-                                       cudaMemcpyHostToDevice, b->stream));
-        b->ntitems[k] = n;
-    }
-    VAH_TRY(cudaStreamSynchronize(b->stream));  // the lists die here
+template <typename T>
+int grow(vah_batch *b, T *&p, size_t &cap, size_t n) {  // device memory for n values; contents lost
+    if (n <= cap) return VAH_OK;
+    if (p) VAH_TRY(cudaFreeAsync(p, b->stream));
+    p = nullptr;
+    cap = 0;
+    VAH_TRY(cudaMallocFromPoolAsync((void **)&p, n * sizeof(T), b->pool, b->stream));
+    cap = n;
     return VAH_OK;
 }
 
+// The work-lists, groups and scratch of the admitted events.
+template <typename S>
 int rebuild_work(vah_batch *b) {
-    if (b->tile) {  // the reductions still walk the cell work-lists below
-        const int rc = rebuild_tiles(b);
-        if (rc != VAH_OK) return rc;
-    }
     std::vector<WorkItem> lists[vah::K_NUM];
-    std::vector<int> order;  // largest event first: its tiles start first, small ones fill the tail
+    std::vector<int> order;  // largest event first: its items start first, small ones fill the tail
+    b->nslots = 0;
     for (int s = 0; s < (int)b->slots.size(); ++s)
-        if (b->slots[s].used) order.push_back(s);
+        if (b->slots[s].used) {
+            order.push_back(s);
+            b->nslots = s + 1;
+        }
     auto cells = [&](int s) {
         const vah_lattice &l = b->slots[s].lat;
         return (long long)l.nx * l.ny * l.nz;
     };
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cells(x) > cells(y); });
-    int seg[vah::K_NUM] = {};  // march segments, from the whole batch's warps
-    for (int kind : {vah::K_FY, vah::K_FZ}) {
-        int longest = 1;
-        for (int s : order) longest = std::max(longest, kind == vah::K_FY ? b->slots[s].lat.ny : b->slots[s].lat.nz);
-        seg[kind] = vah::march_segment(longest, [&](int len) {
-            long long w = 0;
-            for (int s : order) {
-                const vah_lattice &l = b->slots[s].lat;
-                if (kind == vah::K_FZ && l.nz == 1) continue;
-                const long long strips = vah::march_strips(kind == vah::K_FY ? l.nx * l.nz : l.nx * l.ny);
-                const int n = kind == vah::K_FY ? l.ny : l.nz;
-                w += (strips + 3) / 4 * 4 * ((n + len - 1) / len);
-            }
-            return w;
-        });
-    }
+    // groups of events whose differences the scratch holds
+    auto per_field = [&](int s) {  // bytes of one field of differences
+        const vah_lattice &l = b->slots[s].lat;
+        return ((size_t)(l.nx + 4) * (l.ny + 4) * (l.nz + 4) * sizeof(S) + 255) / 256 * 256;
+    };
+    auto scratch_of = [&](int s) { return per_field(s) * (b->slots[s].lat.nz > 1 ? 3 : 2) * b->nq; };
+    std::vector<std::vector<int>> members;
+    size_t held = 0, need = 0;
     for (int s : order) {
-        const vah_batch::Slot &sl = b->slots[s];
-        const int nx = sl.lat.nx, ny = sl.lat.ny, nz = sl.lat.nz;
-        auto march = [&](int kind, int strips, int n) {
-            for (int r0 = 0; r0 < n; r0 += seg[kind])
-                for (int i0 = 0; i0 < strips; i0 += vah::kTY)
-                    lists[kind].push_back({s, i0, r0, std::min(r0 + seg[kind], n)});
-        };
-        if (!b->tile) {
-            const int xs = vah::flux_x_strips(nx, ny, nz);
-            for (int i0 = 0; i0 < xs; i0 += vah::kTY) lists[vah::K_FX].push_back({s, i0, 0, 0});
-            march(vah::K_FY, vah::march_strips(nx * nz), ny);
-            if (nz > 1) march(vah::K_FZ, vah::march_strips(nx * ny), nz);
+        if (members.empty() || held + scratch_of(s) > kScratchBytes) {
+            members.emplace_back();
+            held = 0;
         }
-        for (int r0 = 0; r0 < ny * nz; r0 += vah::kTY)
-            for (int i0 = 0; i0 < nx; i0 += vah::kTX) lists[nz > 1 ? vah::K_C3 : vah::K_C2].push_back({s, i0, r0, 0});
+        members.back().push_back(s);
+        held += scratch_of(s);
+        need = std::max(need, held);
     }
-    for (int k = 0; k < vah::K_NUM; ++k) {
-        const int n = (int)lists[k].size();
-        if (n > b->cap_work[k]) {
-            if (b->d_work[k]) VAH_TRY(cudaFreeAsync(b->d_work[k], b->stream));
-            const int cap = std::max(n, 2 * b->cap_work[k]);
-            VAH_TRY(cudaMallocFromPoolAsync((void **)&b->d_work[k], cap * sizeof(WorkItem), b->pool, b->stream));
-            b->cap_work[k] = cap;
+    int rc = grow(b, b->d_scratch, b->cap_scratch, need);
+    if (rc != VAH_OK) return rc;
+    b->groups.clear();
+    for (const std::vector<int> &group : members) {
+        vah_batch::Group g;
+        for (int k = 0; k < vah::K_NUM; ++k) g.first[k] = (int)lists[k].size();
+        int seg[3] = {};  // march segments along y and eta, from the whole group's warps
+        for (int dir = 1; dir < 3; ++dir) {
+            auto along = [&](const vah_lattice &l) { return dir == 1 ? l.ny : l.nz; };
+            int longest = 1;
+            for (int s : group) longest = std::max(longest, along(b->slots[s].lat));
+            seg[dir] = vah::march_segment(longest, vah::kFluxMinb<S>, [&](int len) {
+                long long w = 0;
+                for (int s : group) {
+                    const vah_lattice &l = b->slots[s].lat;
+                    if (dir == 2 && l.nz == 1) continue;
+                    const long long strips = vah::march_strips<S>(dir == 1 ? l.nx * l.nz : l.nx * l.ny);
+                    w += (strips + 3) / 4 * 4 * ((along(l) + len - 1) / len);
+                }
+                return w;
+            });
         }
+        // the marches first (long), then the x strips, which fill the tail
+        for (int kind : {2, 1, 0})
+            for (int s : group) {
+                const vah_lattice &l = b->slots[s].lat;
+                if (kind == 2 && l.nz == 1) continue;
+                const int strips = kind == 0 ? vah::flux_x_strips<S>(l.nx, l.ny, l.nz)
+                                             : vah::march_strips<S>(kind == 1 ? l.nx * l.nz : l.nx * l.ny);
+                const int n = kind == 0 ? 1 : (kind == 1 ? l.ny : l.nz), len = kind == 0 ? 1 : seg[kind];
+                for (int r0 = 0; r0 < n; r0 += len)
+                    for (int i0 = 0; i0 < strips; i0 += 4)
+                        lists[vah::K_FLUX].push_back({s, kind, i0, r0, std::min(r0 + len, n)});
+            }
+        char *at = b->d_scratch;
+        for (int s : group) {
+            const vah_lattice &l = b->slots[s].lat;
+            for (int c0 = 0; c0 < cells(s); c0 += vah::kCellItem)
+                lists[l.nz > 1 ? vah::K_C3 : vah::K_C2].push_back({s, 0, c0, 0, 0});
+            SlotDesc<S> &d = *desc_host<S>(b, s);
+            for (int k = 0; k < (l.nz > 1 ? 3 : 2); ++k)
+                for (int n = 0; n < b->nq; ++n, at += per_field(s)) d.D[k][n] = (S *)at;
+        }
+        for (int k = 0; k < vah::K_NUM; ++k) g.count[k] = (int)lists[k].size() - g.first[k];
+        b->groups.push_back(g);
+    }
+    if (b->nslots)
+        VAH_TRY(cudaMemcpyAsync(b->d_desc, b->desc_host.data(), sizeof(SlotDesc<S>) * b->nslots, cudaMemcpyHostToDevice,
+                                b->stream));
+    auto *args = (vah::StageArgs<S> *)b->d_args;
+    rc = grow(b, args, b->cap_args, 2 * (size_t)b->nslots);
+    b->d_args = args;
+    if (rc != VAH_OK) return rc;
+    for (int k = 0; k < vah::K_NUM; ++k) {
+        const size_t n = lists[k].size();
+        if ((rc = grow(b, b->d_work[k], b->cap_work[k], n)) != VAH_OK) return rc;
         if (n) VAH_TRY(cudaMemcpyAsync(b->d_work[k], lists[k].data(), n * sizeof(WorkItem), cudaMemcpyHostToDevice,
                                        b->stream));
-        b->nwork[k] = n;
+        b->nwork[k] = (int)n;
     }
-    const int ncells = b->nwork[vah::K_C2] + b->nwork[vah::K_C3];
-    if (ncells > b->cap_partial) {
-        if (b->d_partial) VAH_TRY(cudaFreeAsync(b->d_partial, b->stream));
-        const int cap = std::max(ncells, 2 * b->cap_partial);
-        VAH_TRY(cudaMallocFromPoolAsync((void **)&b->d_partial, (size_t)cap * 5 * sizeof(double), b->pool, b->stream));
-        b->cap_partial = cap;
-    }
+    const size_t ncells = (size_t)b->nwork[vah::K_C2] + b->nwork[vah::K_C3];
+    if ((rc = grow(b, b->d_partial, b->cap_partial, 5 * ncells)) != VAH_OK) return rc;
     // the copies above read host vectors that die here
     VAH_TRY(cudaStreamSynchronize(b->stream));
     return VAH_OK;
 }
 
-// One launch of a kind known at run time.
-template <int PHYS, bool EXACT>
-cudaError_t launch_kind_rt(vah_batch *b, int kind, int stage, const vah::Eos &eos) {
+int rebuild(vah_batch *b) { return b->elem == sizeof(float) ? rebuild_work<float>(b) : rebuild_work<double>(b); }
+
+// A stage of one group: the flux launch (list K_FLUX) or a cell launch.
+template <typename S, int PHYS>
+cudaError_t launch_list(vah_batch *b, const vah_batch::Group &g, int list, int stage) {
     using namespace vah;
-    const SlotDesc<double> *descs = (const SlotDesc<double> *)b->d_desc;
-    const WorkItem *w = b->d_work[kind];
-    const int n = b->nwork[kind];
-    switch (kind) {
-    case K_FX: return launch_kind<PHYS, K_FX, EXACT>(descs, b->d_clk, w, n, stage, eos, b->sms, b->d_wcount + kind, b->stream);
-    case K_FY: return launch_kind<PHYS, K_FY, EXACT>(descs, b->d_clk, w, n, stage, eos, b->sms, b->d_wcount + kind, b->stream);
-    case K_FZ: return launch_kind<PHYS, K_FZ, EXACT>(descs, b->d_clk, w, n, stage, eos, b->sms, b->d_wcount + kind, b->stream);
-    // the cell kinds read the differences whichever way the faces were evaluated
-    case K_C2: return launch_kind<PHYS, K_C2, true>(descs, b->d_clk, w, n, stage, eos, b->sms, b->d_wcount + kind, b->stream);
-    case K_C3: return launch_kind<PHYS, K_C3, true>(descs, b->d_clk, w, n, stage, eos, b->sms, b->d_wcount + kind, b->stream);
-    default: return cudaErrorInvalidValue;
+    const StageArgs<S> *args = (const StageArgs<S> *)b->d_args;
+    const WorkItem *w = b->d_work[list] + g.first[list];
+    const int n = g.count[list], threads = kTX * kTY;
+    if (n == 0) return cudaSuccess;
+    if (list == K_FLUX) {
+        constexpr size_t smem = kTY * kMarchValues<S, PHYS> * sizeof(S);
+        auto kernel = batch_flux_kernel<S, PHYS, false>;
+        if constexpr (sizeof(S) == 8)
+            if (b->opt.flux == VAH_FLUX_PER_CELL) kernel = batch_flux_kernel<S, PHYS, true>;
+        static_assert(smem <= 44 * 1024, "with the arguments, within the default shared memory limit");
+        kernel<<<n, threads, smem, b->stream>>>(args, w, stage);
+    } else if (list == K_C2) {
+        batch_cell_kernel<S, PHYS, false><<<n, threads, 0, b->stream>>>(args, w, stage);
+    } else {
+        batch_cell_kernel<S, PHYS, true><<<n, threads, 0, b->stream>>>(args, w, stage);
+    }
+    return cudaGetLastError();
+}
+
+template <typename S>
+cudaError_t launch_list_s(vah_batch *b, const vah_batch::Group &g, int list, int stage) {
+    switch (b->opt.physics) {
+    case VAH_IDEAL: return launch_list<S, 0>(b, g, list, stage);
+    case VAH_PIMUNU: return launch_list<S, 1>(b, g, list, stage);
+    default: return launch_list<S, 2>(b, g, list, stage);
     }
 }
 
-cudaError_t launch_kind_any(vah_batch *b, int kind, int stage, const vah::Eos &eos) {
-    const bool exact = b->opt.flux == VAH_FLUX_PER_CELL;
-    switch (b->opt.physics) {
-    case VAH_IDEAL: return exact ? launch_kind_rt<0, true>(b, kind, stage, eos) : launch_kind_rt<0, false>(b, kind, stage, eos);
-    case VAH_PIMUNU: return exact ? launch_kind_rt<1, true>(b, kind, stage, eos) : launch_kind_rt<1, false>(b, kind, stage, eos);
-    default: return exact ? launch_kind_rt<2, true>(b, kind, stage, eos) : launch_kind_rt<2, false>(b, kind, stage, eos);
-    }
+cudaError_t launch_list_any(vah_batch *b, const vah_batch::Group &g, int list, int stage) {
+    return b->elem == sizeof(float) ? launch_list_s<float>(b, g, list, stage) : launch_list_s<double>(b, g, list, stage);
+}
+
+int launch_args(vah_batch *b) {
+    if (b->nslots == 0) return VAH_OK;
+    const dim3 block(96, 2);
+    const vah::Eos eos = batch_eos(b);
+    if (b->elem == sizeof(float))
+        vah::args_kernel<float><<<b->nslots, block, 0, b->stream>>>((const SlotDesc<float> *)b->d_desc, b->d_clk, eos,
+                                                                    (vah::StageArgs<float> *)b->d_args);
+    else
+        vah::args_kernel<double><<<b->nslots, block, 0, b->stream>>>((const SlotDesc<double> *)b->d_desc, b->d_clk, eos,
+                                                                     (vah::StageArgs<double> *)b->d_args);
+    VAH_TRY(cudaGetLastError());
+    return VAH_OK;
 }
 
 int enqueue_step(vah_batch *b) {
     using namespace vah;
-    const Eos eos = batch_eos(b);
+    const int rc = launch_args(b);
+    if (rc != VAH_OK) return rc;
     for (int stage = 1; stage <= 2; ++stage)
-        for (int kind = 0; kind < K_NUM; ++kind) VAH_TRY(launch_kind_any(b, kind, stage, eos));
+        for (const vah_batch::Group &g : b->groups)
+            for (int list = 0; list < K_NUM; ++list) VAH_TRY(launch_list_any(b, g, list, stage));
     advance_kernel<<<(kMaxSlots + 255) / 256, 256, 0, b->stream>>>(b->d_clk, b->d_dt, kMaxSlots, b->d_cross, b->d_vol,
                                                                  b->d_dv);
     VAH_TRY(cudaGetLastError());
     return VAH_OK;
-}
-
-// FP32 form: per stage one persistent tile launch per tile shape, then the clocks advance.
-int enqueue_tiles(vah_batch *b) {
-    using namespace vah;
-    const Eos eos = batch_eos(b);
-    const TileClock none{0.0, 0, 0, 0};
-    for (int stage = 1; stage <= 2; ++stage)
-        for (int k = 0; k < 2; ++k)
-            VAH_TRY(tile_launch(b->d_tdesc, (const TileClock *)b->d_clk, none, 0.0, b->d_titems[k], b->ntitems[k],
-                                k == 1, b->d_tcount, stage, b->opt.physics, eos, b->d_tcount + 1, b->stream));
-    advance_kernel<<<(kMaxSlots + 255) / 256, 256, 0, b->stream>>>(b->d_clk, b->d_dt, kMaxSlots, b->d_cross, b->d_vol,
-                                                                 b->d_dv);
-    VAH_TRY(cudaGetLastError());
-    return VAH_OK;
-}
-
-int enqueue(vah_batch *b) {
-    return b->tile ? enqueue_tiles(b) : enqueue_step(b);
 }
 
 int capture_graph(vah_batch *b) {
@@ -708,7 +637,7 @@ int capture_graph(vah_batch *b) {
     }
     cudaGraph_t g;
     VAH_TRY(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-    int rc = enqueue(b);
+    int rc = enqueue_step(b);
     cudaError_t e = cudaStreamEndCapture(b->stream, &g);
     if (rc != VAH_OK) return rc;
     VAH_TRY(e);
@@ -839,7 +768,6 @@ extern "C" int vah_batch_create(const vah_options *opt, const double *eos_table,
     b->opt = *opt;
     b->nq = nq_of(opt->physics);
     b->elem = opt->precision == VAH_FP32 ? sizeof(float) : sizeof(double);
-    b->tile = opt->precision == VAH_FP32;
     b->own_stream = opt->stream == nullptr;
     b->capacity = capacity_bytes;
     b->used = 0;
@@ -870,14 +798,8 @@ extern "C" int vah_batch_create(const vah_options *opt, const double *eos_table,
     chk(cudaMalloc((void **)&b->d_dv, sizeof(double) * vah::kMaxSlots));
     chk(cudaMalloc((void **)&b->d_counters, sizeof(unsigned long long) * 4 * vah::kMaxSlots));
     chk(cudaMalloc((void **)&b->d_maxbits, sizeof(unsigned long long) * vah::kMaxSlots));
-    chk(cudaMalloc((void **)&b->d_wcount, sizeof(unsigned) * vah::K_NUM));
     b->fstage = vah::kFieldStageValues;
     chk(cudaMalloc((void **)&b->d_fstage, sizeof(double) * b->fstage));
-    if (b->tile) {
-        chk(cudaMalloc((void **)&b->d_tdesc, sizeof(vah::TileSlot) * vah::kMaxSlots));
-        chk(cudaMalloc((void **)&b->d_tcount, 2 * sizeof(unsigned)));
-        if (rc == VAH_OK) chk(cudaMemset(b->d_tcount, 0, 2 * sizeof(unsigned)));
-    }
     if (rc == VAH_OK) {
         chk(cudaMemset(b->d_clk, 0, sizeof(SlotClock) * vah::kMaxSlots));
         chk(cudaMemset(b->d_dt, 0, sizeof(double) * vah::kMaxSlots));
@@ -920,9 +842,9 @@ extern "C" int vah_batch_destroy(vah_batch *b) {
         if (sl.mem) cudaFreeAsync(sl.mem, b->stream);
     for (int k = 0; k < vah::K_NUM; ++k)
         if (b->d_work[k]) cudaFreeAsync(b->d_work[k], b->stream);
-    for (int k = 0; k < 2; ++k)
-        if (b->d_titems[k]) cudaFreeAsync(b->d_titems[k], b->stream);
     if (b->d_partial) cudaFreeAsync(b->d_partial, b->stream);
+    if (b->d_args) cudaFreeAsync(b->d_args, b->stream);
+    if (b->d_scratch) cudaFreeAsync(b->d_scratch, b->stream);
     cudaStreamSynchronize(b->stream);
     cudaMemPoolDestroy(b->pool);
     cudaFree(b->d_desc);
@@ -933,10 +855,7 @@ extern "C" int vah_batch_destroy(vah_batch *b) {
     cudaFree(b->d_dv);
     cudaFree(b->d_counters);
     cudaFree(b->d_maxbits);
-    cudaFree(b->d_wcount);
     cudaFree(b->d_fstage);
-    cudaFree(b->d_tdesc);
-    cudaFree(b->d_tcount);
     cudaFree(b->d_tab);
     cudaFree(b->d_exc);
     cudaEventDestroy(b->t0);
@@ -1036,7 +955,7 @@ extern "C" int vah_batch_step(vah_batch *b, int nsteps) {
     VAH_TRY(cudaSetDevice(b->opt.device));
     int rc;
     if (b->dirty) {
-        if ((rc = rebuild_work(b)) != VAH_OK) return rc;
+        if ((rc = rebuild(b)) != VAH_OK) return rc;
         if ((rc = capture_graph(b)) != VAH_OK) return rc;
     }
     if (b->timing) VAH_TRY(cudaEventRecord(b->t0, b->stream));
@@ -1088,7 +1007,7 @@ extern "C" int vah_batch_get_field(vah_batch *b, int slot, int field, double *ho
     if (!b || !host || slot < 0 || slot >= vah::kMaxSlots || !b->slots[slot].used) return VAH_ERR_ARG;
     VAH_TRY(cudaSetDevice(b->opt.device));
     const vah_lattice &lat = b->slots[slot].lat;
-    const int ncx = slot_pitch(b, lat.nx), parity = (int)((b->steps - b->slots[slot].admitted) & 1);
+    const int ncx = lat.nx + 4, parity = (int)((b->steps - b->slots[slot].admitted) & 1);
     auto read = [&](auto *src) -> int {
         using S = std::remove_reference_t<decltype(*src)>;
         if (!src) return VAH_ERR_ARG;
@@ -1111,7 +1030,7 @@ extern "C" int vah_batch_fallback_mask(vah_batch *b, int slot, unsigned char *ho
     if (!b || !host || slot < 0 || slot >= vah::kMaxSlots || !b->slots[slot].used) return VAH_ERR_ARG;
     VAH_TRY(cudaSetDevice(b->opt.device));
     const vah_lattice &lat = b->slots[slot].lat;
-    const size_t ncx = slot_pitch(b, lat.nx), ncy = lat.ny + 4;
+    const size_t ncx = lat.nx + 4, ncy = lat.ny + 4;
     const unsigned char *src = b->elem == sizeof(float) ? slot_fallback<float>(b, slot) : slot_fallback<double>(b, slot);
     for (int k = 0; k < lat.nz; ++k)
         VAH_TRY(cudaMemcpy2DAsync(host + (size_t)lat.nx * lat.ny * k, lat.nx, src + 2 + ncx * (2 + ncy * (k + 2)), ncx,
@@ -1134,7 +1053,7 @@ extern "C" int vah_batch_max_energy_density(vah_batch *b, double *out, int nslot
     if (!b || !out || nslots < 1) return VAH_ERR_ARG;
     VAH_TRY(cudaSetDevice(b->opt.device));
     int rc;
-    if (b->dirty && (rc = rebuild_work(b)) != VAH_OK) return rc;
+    if (b->dirty && (rc = rebuild(b)) != VAH_OK) return rc;
     VAH_TRY(cudaMemsetAsync(b->d_maxbits, 0, sizeof(unsigned long long) * vah::kMaxSlots, b->stream));
     for (int kind : {vah::K_C2, vah::K_C3}) {
         if (!b->nwork[kind]) continue;
@@ -1163,7 +1082,7 @@ extern "C" int vah_batch_observables(vah_batch *b, double *out, int nslots) {
     if (!b || !out || nslots < 1) return VAH_ERR_ARG;
     VAH_TRY(cudaSetDevice(b->opt.device));
     int rc;
-    if (b->dirty && (rc = rebuild_work(b)) != VAH_OK) return rc;
+    if (b->dirty && (rc = rebuild(b)) != VAH_OK) return rc;
     const int n2 = b->nwork[vah::K_C2], n3 = b->nwork[vah::K_C3];
     auto launch = [&](int kind, double *part) -> cudaError_t {
         const int nw = b->nwork[kind];
@@ -1228,34 +1147,34 @@ extern "C" int vah_batch_kernel_time(vah_batch *b, double *ms, long long *steps)
 
 namespace {
 
-// The batch form of vah_event_autotune: each launch kind has one register cap
-// and a tile fixed by the work-list, so this times it: `reps` launches over the
-// whole work-list in stage-1 buffer roles (outputs are stage scratch); the
-// per-slot counters are restored.
+// The batch form of vah_event_autotune: times the flux launch (reported as the
+// first of the three flux kinds) and the cell launches of the first group,
+// `reps` times in stage-1 buffer roles (outputs are stage scratch); each has
+// one configuration. The per-slot counters are restored.
 int batch_autotune(vah_batch *b, int reps, vah_tune_report *out) {
     using namespace vah;
-    const Eos eos = batch_eos(b);
     std::vector<unsigned long long> saved((size_t)kMaxSlots * 4);
     VAH_TRY(cudaStreamSynchronize(b->stream));
     VAH_TRY(cudaMemcpy(saved.data(), b->d_counters, saved.size() * sizeof(unsigned long long),
                        cudaMemcpyDeviceToHost));
+    int rc = launch_args(b);
+    if (rc != VAH_OK) return rc;
     cudaEvent_t e0, e1;
     VAH_TRY(cudaEventCreate(&e0));
     VAH_TRY(cudaEventCreate(&e1));
-    int rc = VAH_OK;
-    out->nkinds = K_NUM;
-    for (int kind = 0; kind < K_NUM && rc == VAH_OK; ++kind) {
-        const int minb = kind == K_FX ? kFluxXMinb : (kind <= K_FZ ? kMarchMinb : kCellMinb);
-        out->kind[kind] = {kTX, kTY, minb, 0.0, 0.0};
-        if (b->nwork[kind] == 0) continue;
-        rc = VAH_ERR_CUDA;
-        bool ok = launch_kind_any(b, kind, 1, eos) == cudaSuccess && cudaEventRecord(e0, b->stream) == cudaSuccess;
-        for (int k = 0; k < reps && ok; ++k) ok = launch_kind_any(b, kind, 1, eos) == cudaSuccess;
+    out->nkinds = 5;
+    for (int kind = 0; kind < 5 && rc == VAH_OK; ++kind) {
+        const int list = kind < 3 ? K_FLUX : (kind == 3 ? K_C2 : K_C3);
+        out->kind[kind] = {kTX, kTY, kind < 3 ? 4 : 3, 0.0, 0.0};
+        if (kind == 1 || kind == 2 || b->groups.empty() || b->groups[0].count[list] == 0) continue;
+        auto launch = [&]() { return launch_list_any(b, b->groups[0], list, 1) == cudaSuccess; };
+        bool ok = launch() && cudaEventRecord(e0, b->stream) == cudaSuccess;
+        for (int k = 0; k < reps && ok; ++k) ok = launch();
         float f = 0;
-        if (ok && cudaEventRecord(e1, b->stream) == cudaSuccess && cudaEventSynchronize(e1) == cudaSuccess &&
-            cudaEventElapsedTime(&f, e0, e1) == cudaSuccess)
-            rc = VAH_OK;
-        out->kind[kind] = {kTX, kTY, minb, f / reps, f / reps};
+        if (!ok || cudaEventRecord(e1, b->stream) != cudaSuccess || cudaEventSynchronize(e1) != cudaSuccess ||
+            cudaEventElapsedTime(&f, e0, e1) != cudaSuccess)
+            rc = VAH_ERR_CUDA;
+        out->kind[kind].ms_default = out->kind[kind].ms_best = f / reps;
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
@@ -1271,10 +1190,10 @@ int batch_autotune(vah_batch *b, int reps, vah_tune_report *out) {
 extern "C" int vah_batch_autotune(vah_batch *b, int reps, vah_tune_report *out) {
     if (!b || !out || reps < 1) return VAH_ERR_ARG;
     memset(out, 0, sizeof(*out));
-    if (b->tile) return VAH_OK;  // one persistent tile launch per stage and shape: nothing to tune
+    if (b->elem == sizeof(float)) return VAH_OK;  // the FP32 form has nothing to tune
     VAH_TRY(cudaSetDevice(b->opt.device));
     if (b->dirty) {  // the work-list must describe the admitted events
-        const int rc = rebuild_work(b);
+        const int rc = rebuild(b);
         if (rc != VAH_OK) return rc;
     }
     return batch_autotune(b, reps, out);

@@ -12,61 +12,29 @@ namespace vah {
 template <typename S>
 cudaError_t launch_stage(const StageArgs<S> &a, int physics, cudaStream_t stream);
 
-// ---- flux/cell split: launch kinds and their tunable launch configuration --
-// Kinds of launch in one split stage: the flux launches per axis, then the
-// cell launch, all of 128-thread blocks. Each kind has one register cap: at
-// least minb resident blocks per SM, the fastest of its candidates on the
-// 121x121x81 event (x fluxes: 96 registers without spills, 105 us against 117
-// at 4 blocks; marches: 120 registers, 105 us against 152 at 5 blocks, which
-// spill; cell: 168 registers, 315 us). The cell launch's block shape bx x by
-// (x fastest) is the autotuner's choice; the flux launches' warps index
-// themselves.
+// ---- flux/cell split -------------------------------------------------------
+// A split stage is two launches: the flux differences along every axis (kinds
+// kFaceX, kFaceY, kFaceZ, which can also be launched one by one to time them),
+// then the cells (kCell). One register cap each, the fastest of its candidates
+// on the 121x121x81 event: FP64 fluxes 128 (5 blocks' 96 spill in the marches:
+// 152 us against 105 along y), FP64 cells 128 in blocks of 64 threads (0.610 ms
+// per stage against 0.620 at 168, although they spill), but 168 in 2+1D, where
+// the cell needs less (0.090 ms per stage of a 395x395 event against 0.095), FP32
+// cells 96 (0.392 against 0.401 at 80; in blocks of 128 threads 0.408).
 enum SplitKind { kFaceX = 0, kFaceY = 1, kFaceZ = 2, kCell = 3, kNumSplitKinds = 4 };
-constexpr int kSplitThreads = 128;
-constexpr int kFluxXMinb = 5, kMarchMinb = 4, kCellMinb = 3;
-
-struct KindConfig {
-    int bx, by, minb;
-};
-struct SplitConfig {
-    KindConfig k[kNumSplitKinds];
-};
-
-constexpr int kNumShapes = 2;
-constexpr int kShapes[kNumShapes][2] = {{32, 4}, {64, 2}};
-
-// Candidates of one kind, in a fixed order; returns their number.
-inline int split_candidates(int kind, KindConfig *out, int max) {
-    const int minb = kind == kCell ? kCellMinb : (kind == kFaceX ? kFluxXMinb : kMarchMinb);
-    int n = 0;
-    for (int s = 0; s < (kind == kCell ? kNumShapes : 1); ++s)
-        if (n < max) out[n++] = {kShapes[s][0], kShapes[s][1], minb};
-    return n;
-}
-
-inline bool valid_kind_config(int kind, const KindConfig &c) {
-    if (kind < 0 || kind >= kNumSplitKinds) return false;
-    KindConfig ok[kNumShapes];
-    const int n = split_candidates(kind, ok, kNumShapes);
-    for (int k = 0; k < n; ++k)
-        if (ok[k].bx == c.bx && ok[k].by == c.by && ok[k].minb == c.minb) return true;
-    return false;
-}
-
-// Untuned default.
-inline SplitConfig default_split_config() {
-    SplitConfig c;
-    for (int k = 0; k < kNumSplitKinds; ++k) split_candidates(k, &c.k[k], 1);
-    return c;
-}
+constexpr int kFluxThreads = 128, kCellThreads = 64;
+template <typename S>
+constexpr int kFluxMinb = sizeof(S) == 8 ? 4 : 5;
+template <typename S, bool IS3D>
+constexpr int kCellMinb = sizeof(S) == 4 ? 10 : (IS3D ? 8 : 6);
 
 // Cells per march segment along an axis of n cells, from the number of warps
-// a segment length makes: the fewest waves (148 SMs x 5 blocks x 4 warps)
+// a segment length makes: the fewest waves (148 SMs x minb blocks x 4 warps)
 // times the segment's length plus its start-up (one face and its first
 // loads, about 1.5 cells' work).
 template <typename Warps>
-inline int march_segment(int n, Warps warps) {
-    constexpr long long wave = 148 * kMarchMinb * 4;
+inline int march_segment(int n, int minb, Warps warps) {
+    const long long wave = 148 * 4 * minb;
     int best = 1;
     double cost = 1e300;
     for (int parts = 1; parts <= n; ++parts) {
@@ -80,17 +48,13 @@ inline int march_segment(int n, Warps warps) {
     return best;
 }
 
-// One launch of one split kind (a.D must point at the difference buffers).
-// exact = the reference's per-cell face evaluation.
+// One launch of one split kind over the planes from k0 that D holds (a.D must
+// point at the difference buffers). exact = the reference's per-cell face
+// evaluation (FP64).
 template <typename S>
-cudaError_t launch_split_kind(const StageArgs<S> &a, int physics, bool exact, int kind, const KindConfig &c,
-                              cudaStream_t stream);
+cudaError_t launch_split_kind(const StageArgs<S> &a, int physics, bool exact, int kind, cudaStream_t stream);
 
-// One RK stage on the flux/cell split: flux launches (x, y[, z]) then the
-// cell launch, with the given (or the default) launch configuration.
-template <typename S>
-cudaError_t launch_stage_split(const StageArgs<S> &a, int physics, bool exact, const SplitConfig &c,
-                               cudaStream_t stream);
+// One RK stage on the flux/cell split: the flux launch, then the cell launch.
 template <typename S>
 cudaError_t launch_stage_split(const StageArgs<S> &a, int physics, bool exact, cudaStream_t stream);
 

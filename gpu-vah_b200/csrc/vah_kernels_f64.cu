@@ -3,5 +3,6 @@
 
 namespace vah {
 VAH_INSTANTIATE_SETUP(double)
-VAH_INSTANTIATE_STAGE(double)
+VAH_INSTANTIATE_SPLIT(double)
+template cudaError_t launch_stage<double>(const StageArgs<double> &, int, cudaStream_t);
 }  // namespace vah

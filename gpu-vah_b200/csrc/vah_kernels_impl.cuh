@@ -3,15 +3,15 @@
 // and vah_kernels_f32.cu (separate translation units build in parallel).
 //
 // stage_kernel: one thread per interior cell runs the whole RK stage of that
-// cell (vah_stage.cuh). flux_x_kernel + flux_march_kernel + cell_kernel: the
-// same stage split into per-axis flux launches (vah_march.cuh) and one cell
-// launch (the default path). 128-thread blocks, x fastest so that every load
-// of a field is a coalesced row. The cell kernel takes its block shape at run
-// time; the autotuner picks it by timing on the event's own state.
+// cell (vah_stage.cuh; FP64). flux_kernel + cell_kernel: the same stage split
+// into one launch for the flux differences along every axis (vah_march.cuh)
+// and one for the cells (the default path, and the FP32 form). 128-
+// or 64-thread blocks, x fastest so that the loads of a field coalesce.
 #pragma once
 
 #include "vah_kernels.cuh"
 #include "vah_march.cuh"
+#include "vah_tile_cell.cuh"
 
 namespace vah {
 
@@ -39,25 +39,44 @@ __global__ void __launch_bounds__(kBX *kBY) stage_kernel(const StageArgs<S> a) {
     stage_cell<S, PHYS, IS3D>(a, i + 2, j + 2, k + 2);
 }
 
-// The x flux differences of the planes [k0, k1): a warp per strip.
-template <int PHYS, bool EXACT>
-__global__ void __launch_bounds__(kSplitThreads, kFluxXMinb) flux_x_kernel(const StageArgs<double> a, int strips) {
-    __shared__ HalfPointers hp;
-    set_half_pointers<PHYS>(hp, a, threadIdx.x);
-    __syncthreads();
-    const int strip = blockIdx.x * (kSplitThreads / 32) + threadIdx.x / 32;
-    if (strip < strips) flux_x<PHYS, EXACT>(a, hp, strip);
-}
+// What the blocks of one flux launch do: eta marches first, then y marches (the
+// long ones), then x strips, which fill the tail.
+struct FluxGrid {
+    int zblocks, yblocks, xblocks;
+    int zstrips, zseg, ystrips, yseg, xstrips;
+};
 
-// The y or eta flux differences: a warp per strip and segment of `seg` cells.
-template <int PHYS, int DIR, bool EXACT>
-__global__ void __launch_bounds__(kSplitThreads, kMarchMinb) flux_march_kernel(const StageArgs<double> a, int strips, int seg) {
-    extern __shared__ double march_sm[];
-    const int lo = DIR == 1 ? 0 : a.k0, hi = DIR == 1 ? a.ny : a.k1;
-    const int w = blockIdx.x * (kSplitThreads / 32) + threadIdx.x / 32;
-    const int part = w / strips, m0 = lo + part * seg;
-    if (m0 >= hi) return;
-    flux_march<PHYS, DIR, EXACT>(a, HalfSelect<PHYS>{a}, w - part * strips, m0, min(m0 + seg, hi), march_sm + (threadIdx.x / 32) * kMarchDoubles<PHYS>);
+// The flux differences of the planes [k0, k1): a warp per x strip, or per
+// strip and segment of a march.
+template <typename S, int PHYS, bool EXACT>
+__global__ void __launch_bounds__(kFluxThreads, kFluxMinb<S>) flux_kernel(const StageArgs<S> a, const FluxGrid g) {
+    extern __shared__ __align__(16) unsigned char flux_sm[];
+    const SelectPointers<S, PHYS> sel{a};
+    const int warp = threadIdx.x / 32;
+    int block = blockIdx.x;
+    S *sm = (S *)flux_sm + warp * kMarchValues<S, PHYS>;
+    if (block < g.zblocks) {
+        const int w = block * 4 + warp, part = w / g.zstrips, m0 = a.k0 + part * g.zseg;
+        if (m0 < a.k1)
+            flux_march<PHYS, 2, EXACT>(a, sel, w - part * g.zstrips, m0, min(m0 + g.zseg, a.k1), sm);
+        return;
+    }
+    block -= g.zblocks;
+    if (block < g.yblocks) {
+        const int w = block * 4 + warp, part = w / g.ystrips, m0 = part * g.yseg;
+        if (m0 < a.ny)
+            flux_march<PHYS, 1, EXACT>(a, sel, w - part * g.ystrips, m0, min(m0 + g.yseg, a.ny), sm);
+        return;
+    }
+    block -= g.yblocks;
+    if constexpr (Lanes<S, PHYS>::SPLIT) {
+        __shared__ TablePointers<S> tab;
+        set_table_pointers<PHYS>(tab, a, threadIdx.x);
+        __syncthreads();
+        if (block * 4 + warp < g.xstrips) flux_x<PHYS, EXACT>(a, tab, block * 4 + warp);
+    } else if (block * 4 + warp < g.xstrips) {
+        flux_x<PHYS, EXACT>(a, sel, block * 4 + warp);
+    }
 }
 
 // One warp per row at a time; PACK: device layout -> packed, else back.
@@ -76,13 +95,15 @@ __global__ void pack_kernel(S *__restrict__ field, double *__restrict__ packed, 
     }
 }
 
-template <int PHYS, bool IS3D>
-__global__ void __launch_bounds__(kSplitThreads, kCellMinb) cell_kernel(const StageArgs<double> a) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    const int r = row_block() * blockDim.y + threadIdx.y;
-    if (i >= a.nx || r >= a.ny * (a.k1 - a.k0)) return;
-    const int j = r % a.ny, k = r / a.ny + a.k0;
-    cell_compute<double, PHYS, IS3D, true>(a, i + 2, j + 2, k + 2);
+// Cells of the planes [k0, k1) in order, x fastest: a row's end does not idle
+// the lanes of a warp (rows of 81 left 15 of 96 idle as 32-wide tiles).
+template <typename S, int PHYS, bool IS3D>
+__global__ void __launch_bounds__(kCellThreads, kCellMinb<S, IS3D>) cell_kernel(const StageArgs<S> a) {
+    const int c = blockIdx.x * kCellThreads + threadIdx.x;
+    if (c >= a.nx * a.ny * (a.k1 - a.k0)) return;
+    const int r = c / a.nx, i = c - r * a.nx, k = r / a.ny, j = r - k * a.ny;
+    if constexpr (sizeof(S) == 4) cell_compute_f32<PHYS, IS3D>(a, i + 2, j + 2, k + a.k0 + 2);
+    else cell_compute<S, PHYS, IS3D, true>(a, i + 2, j + 2, k + a.k0 + 2);
 }
 
 template <typename S, int PHYS>
@@ -166,45 +187,77 @@ cudaError_t stage_dispatch(const StageArgs<S> &a, cudaStream_t stream) {
     return cudaGetLastError();
 }
 
-template <int PHYS, bool EXACT>
-cudaError_t flux_x_launch(const StageArgs<double> &a, cudaStream_t stream) {
-    const int strips = flux_x_strips(a.nx, a.ny, a.k1 - a.k0);
-    flux_x_kernel<PHYS, EXACT><<<(strips + 3) / 4, kSplitThreads, 0, stream>>>(a, strips);
-    return cudaGetLastError();
-}
-
-template <int PHYS, bool EXACT, int DIR>
-cudaError_t flux_march_launch(const StageArgs<double> &a, cudaStream_t stream) {
-    constexpr size_t smem = kSplitThreads / 32 * kMarchDoubles<PHYS> * sizeof(double);
-    auto kernel = flux_march_kernel<PHYS, DIR, EXACT>;
-    cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-    const int n = DIR == 1 ? a.ny : a.k1 - a.k0;
-    const int strips = march_strips(DIR == 1 ? a.nx * (a.k1 - a.k0) : a.nx * a.ny);
-    const int seg = march_segment(n, [&](int len) { return (long long)strips * ((n + len - 1) / len); });
-    const int warps = strips * ((n + seg - 1) / seg);
-    kernel<<<(warps + 3) / 4, kSplitThreads, smem, stream>>>(a, strips, seg);
-    return cudaGetLastError();
-}
-
-template <int PHYS, bool IS3D>
-cudaError_t cell_launch(const StageArgs<double> &a, const KindConfig &c, cudaStream_t stream) {
-    const dim3 block(c.bx, c.by), grid = row_grid(a.nx, (long long)a.ny * (a.k1 - a.k0), c.bx, c.by);
-    cell_kernel<PHYS, IS3D><<<grid, block, 0, stream>>>(a);
-    return cudaGetLastError();
-}
-
-template <int PHYS, bool EXACT>
-cudaError_t split_kind_dispatch(const StageArgs<double> &a, int kind, const KindConfig &c, cudaStream_t stream) {
-    if (a.k0 < 0 || a.k1 > a.nz || a.k0 > a.k1) return cudaErrorInvalidValue;
-    if (a.k0 == a.k1) return cudaSuccess;  // no planes
-    switch (kind) {
-    case kFaceX: return flux_x_launch<PHYS, EXACT>(a, stream);
-    case kFaceY: return flux_march_launch<PHYS, EXACT, 1>(a, stream);
-    case kFaceZ: return a.nz > 1 ? flux_march_launch<PHYS, EXACT, 2>(a, stream) : cudaSuccess;
-    case kCell: return a.nz > 1 ? cell_launch<PHYS, true>(a, c, stream) : cell_launch<PHYS, false>(a, c, stream);
-    default: return cudaErrorInvalidValue;
+// The flux launch; kind kFaceX, kFaceY or kFaceZ: that axis alone (for timing it), kCell: all.
+template <typename S, int PHYS, bool EXACT>
+cudaError_t flux_launch(const StageArgs<S> &a, int kind, cudaStream_t stream) {
+    constexpr size_t smem = kFluxThreads / 32 * kMarchValues<S, PHYS> * sizeof(S);
+    auto kernel = flux_kernel<S, PHYS, EXACT>;
+    static_assert(smem <= 48 * 1024, "within the default shared memory limit");
+    const int planes = a.k1 - a.k0;
+    FluxGrid g{};
+    if (kind == kFaceX || kind == kCell) {
+        g.xstrips = flux_x_strips<S>(a.nx, a.ny, planes);
+        g.xblocks = (g.xstrips + 3) / 4;
     }
+    auto march = [&](int columns, int n, int &strips, int &seg, int &blocks) {
+        strips = march_strips<S>(columns);
+        seg = march_segment(n, kFluxMinb<S>, [&](int len) { return (long long)strips * ((n + len - 1) / len); });
+        blocks = (strips * ((n + seg - 1) / seg) + 3) / 4;
+    };
+    if (kind == kFaceY || kind == kCell) march(a.nx * planes, a.ny, g.ystrips, g.yseg, g.yblocks);
+    if (a.nz > 1 && (kind == kFaceZ || kind == kCell)) march(a.nx * a.ny, planes, g.zstrips, g.zseg, g.zblocks);
+    const int grid = g.xblocks + g.yblocks + g.zblocks;
+    if (grid == 0) return cudaSuccess;
+    kernel<<<grid, kFluxThreads, smem, stream>>>(a, g);
+    return cudaGetLastError();
+}
+
+template <typename S, int PHYS, bool IS3D>
+cudaError_t cell_launch(const StageArgs<S> &a, cudaStream_t stream) {
+    const int cells = a.nx * a.ny * (a.k1 - a.k0);
+    cell_kernel<S, PHYS, IS3D><<<(cells + kCellThreads - 1) / kCellThreads, kCellThreads, 0, stream>>>(a);
+    return cudaGetLastError();
+}
+
+template <typename S, int PHYS>
+cudaError_t kind_dispatch(const StageArgs<S> &a, bool exact, int kind, cudaStream_t stream) {
+    if (kind == kCell) return a.nz > 1 ? cell_launch<S, PHYS, true>(a, stream) : cell_launch<S, PHYS, false>(a, stream);
+    if constexpr (sizeof(S) == 8)
+        if (exact) return flux_launch<S, PHYS, true>(a, kind, stream);
+    return flux_launch<S, PHYS, false>(a, kind, stream);
+}
+
+// The arguments of one slab [k0, k1) of planes that the difference buffers
+// hold: plane k0 is D's first.
+template <typename S>
+StageArgs<S> slab_args(const StageArgs<S> &a0, int k0, int k1) {
+    StageArgs<S> a = a0;
+    a.k0 = k0;
+    a.k1 = k1;
+    if (a0.d_planes > 0)
+        for (int d = 0; d < 3; ++d)
+            for (int n = 0; n < 16; ++n)
+                if (a.D[d][n]) a.D[d][n] -= a.plane * (k0 + 2);
+    return a;
+}
+
+// The stage of the planes [k0, k1), a slab at a time: each slab reads stage
+// inputs only and writes stage outputs, so their order is free.
+template <typename S, int PHYS>
+cudaError_t stage_split_dispatch(const StageArgs<S> &a0, bool exact, cudaStream_t stream) {
+    if (a0.k0 < 0 || a0.k1 > a0.nz || a0.k0 > a0.k1) return cudaErrorInvalidValue;
+    const int slab = a0.d_planes > 0 ? a0.d_planes : a0.nz;
+    for (int k0 = a0.k0; k0 < a0.k1; k0 += slab) {
+        const StageArgs<S> a = slab_args(a0, k0, k0 + slab < a0.k1 ? k0 + slab : a0.k1);
+        cudaError_t e;
+        if constexpr (sizeof(S) == 8)
+            e = exact ? flux_launch<S, PHYS, true>(a, kCell, stream) : flux_launch<S, PHYS, false>(a, kCell, stream);
+        else
+            e = flux_launch<S, PHYS, false>(a, kCell, stream);
+        if (e == cudaSuccess) e = kind_dispatch<S, PHYS>(a, exact, kCell, stream);
+        if (e != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 int grid_for(long long n, int block) {
@@ -227,36 +280,24 @@ cudaError_t launch_stage(const StageArgs<S> &a, int physics, cudaStream_t stream
 }
 
 template <typename S>
-cudaError_t launch_split_kind(const StageArgs<S> &a, int physics, bool exact, int kind, const KindConfig &c,
-                              cudaStream_t stream) {
-    if (!valid_kind_config(kind, c)) return cudaErrorInvalidValue;
+cudaError_t launch_split_kind(const StageArgs<S> &a0, int physics, bool exact, int kind, cudaStream_t stream) {
+    const StageArgs<S> a = slab_args(a0, a0.k0, a0.d_planes > 0 && a0.k0 + a0.d_planes < a0.k1 ? a0.k0 + a0.d_planes : a0.k1);
     switch (physics) {
-    case kIdeal:
-        return exact ? split_kind_dispatch<kIdeal, true>(a, kind, c, stream)
-                     : split_kind_dispatch<kIdeal, false>(a, kind, c, stream);
-    case kPimunu:
-        return exact ? split_kind_dispatch<kPimunu, true>(a, kind, c, stream)
-                     : split_kind_dispatch<kPimunu, false>(a, kind, c, stream);
-    case kPimunuPi:
-        return exact ? split_kind_dispatch<kPimunuPi, true>(a, kind, c, stream)
-                     : split_kind_dispatch<kPimunuPi, false>(a, kind, c, stream);
+    case kIdeal: return kind_dispatch<S, kIdeal>(a, exact, kind, stream);
+    case kPimunu: return kind_dispatch<S, kPimunu>(a, exact, kind, stream);
+    case kPimunuPi: return kind_dispatch<S, kPimunuPi>(a, exact, kind, stream);
     default: return cudaErrorInvalidValue;
     }
 }
 
 template <typename S>
-cudaError_t launch_stage_split(const StageArgs<S> &a, int physics, bool exact, const SplitConfig &c,
-                               cudaStream_t stream) {
-    for (int kind = 0; kind < kNumSplitKinds; ++kind) {
-        const cudaError_t e = launch_split_kind<S>(a, physics, exact, kind, c.k[kind], stream);
-        if (e != cudaSuccess) return e;
-    }
-    return cudaSuccess;
-}
-
-template <typename S>
 cudaError_t launch_stage_split(const StageArgs<S> &a, int physics, bool exact, cudaStream_t stream) {
-    return launch_stage_split<S>(a, physics, exact, default_split_config(), stream);
+    switch (physics) {
+    case kIdeal: return stage_split_dispatch<S, kIdeal>(a, exact, stream);
+    case kPimunu: return stage_split_dispatch<S, kPimunu>(a, exact, stream);
+    case kPimunuPi: return stage_split_dispatch<S, kPimunuPi>(a, exact, stream);
+    default: return cudaErrorInvalidValue;
+    }
 }
 
 template <typename S>
@@ -342,8 +383,6 @@ cudaError_t launch_ghost_pass(const FieldSet<S> &fields, int nx, int ny, int nz,
     return cudaGetLastError();
 }
 
-// The set-up launches and the validity diagnostics serve both storage types;
-// the stage launches are FP64 (the FP32 form has the tile kernel).
 #define VAH_INSTANTIATE_SETUP(S)                                                                                \
     template cudaError_t launch_validity<S>(const ValidityArgs<S> &, int, cudaStream_t);                        \
     template cudaError_t launch_set_conserved<S>(const FieldSet<S> &, const FieldSet<S> &, const FieldSet<S> &, \
@@ -356,12 +395,8 @@ cudaError_t launch_ghost_pass(const FieldSet<S> &fields, int nx, int ny, int nz,
                                           cudaStream_t);                                                        \
     template cudaError_t launch_ghosts<S>(const FieldSet<S> &, int, int, int, int, cudaStream_t);              \
     template cudaError_t launch_ghost_pass<S>(const FieldSet<S> &, int, int, int, int, int, cudaStream_t);
-#define VAH_INSTANTIATE_STAGE(S)                                                                                \
-    template cudaError_t launch_stage<S>(const StageArgs<S> &, int, cudaStream_t);                              \
-    template cudaError_t launch_split_kind<S>(const StageArgs<S> &, int, bool, int, const KindConfig &,         \
-                                              cudaStream_t);                                                    \
-    template cudaError_t launch_stage_split<S>(const StageArgs<S> &, int, bool, const SplitConfig &,            \
-                                               cudaStream_t);                                                   \
+#define VAH_INSTANTIATE_SPLIT(S)                                                                                \
+    template cudaError_t launch_split_kind<S>(const StageArgs<S> &, int, bool, int, cudaStream_t);              \
     template cudaError_t launch_stage_split<S>(const StageArgs<S> &, int, bool, cudaStream_t);
 
 }  // namespace vah

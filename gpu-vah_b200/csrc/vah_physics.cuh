@@ -748,10 +748,11 @@ VAH_HD int cell_sources(const Eos &eos, const R *Q, const CellGradT<R> &g, const
     const R inv_dt = k.inv_dt;
     const R dtut = (ut - g.utp) * inv_dt, dtux = (ux - g.uxp) * inv_dt;
     const R dtuy = (uy - g.uyp) * inv_dt, dtun = (un - g.unp) * inv_dt;
-    const R dux = ut * dtux + ux * dxux + uy * dyux + un * dnux;
-    const R duy = ut * dtuy + ux * dxuy + uy * dyuy + un * dnuy;
-    const R dun = ut * dtun + ux * dxun + uy * dyun + un * dnun;
-    const R dut = ut * dtut + ux * dxut + uy * dyut + un * dnut;  // = Dut - t un^2
+    // (fma: the compiler's choice of the fused product differs between kernels)
+    const R dux = fma(un, dnux, fma(uy, dyux, fma(ut, dtux, ux * dxux)));
+    const R duy = fma(un, dnuy, fma(uy, dyuy, fma(ut, dtuy, ux * dxuy)));
+    const R dun = fma(un, dnun, fma(uy, dyun, fma(ut, dtun, ux * dxun)));
+    const R dut = fma(un, dnut, fma(uy, dyut, fma(ut, dtut, ux * dxut)));  // = Dut - t un^2
     const R Dut = dut + t * un2;
     const R Dux = -dux, Duy = -duy;
     const R Dun = -t2 * (dun + 2 * ut * un * inv_t);

@@ -25,6 +25,7 @@ struct StageArgs {
     double t_src;     // time of the Euler step (stage 1: t, stage 2: t + dt)
     // derived per launch by finish_args: the sources' constants at t_src, dt / h and 1 / (2 h) per axis
     StepConsts ksrc;
+    StepConstsT<float> ksrc_f;  // the FP32 form's
     double c_h[3], inv2h[3];
     double t_inv;     // time of the inversion/regulator (t + dt)
     double dt, dx, dy, dz, etabar;
@@ -60,6 +61,7 @@ struct StageArgs {
     // cell evaluates both faces, written by the flux launches (vah_march.cuh)
     // and read by the cell launch; null: it differences H / HR itself
     S *D[3][16];
+    int d_planes;  // interior planes D holds; 0: all (launch_stage runs slabs of them)
 };
 
 VAH_HD void count_add(unsigned long long *c, unsigned long long v) {
@@ -75,6 +77,7 @@ VAH_HD void count_add(unsigned long long *c, unsigned long long v) {
 template <typename S>
 VAH_HD void finish_args(StageArgs<S> &a) {
     a.ksrc = step_consts(a.t_src, a.dt, a.etabar);
+    a.ksrc_f = step_consts((float)a.t_src, (float)a.dt, (float)a.etabar);
     const double h[3] = {a.dx, a.dy, a.dz};
     for (int d = 0; d < 3; ++d) {
         a.c_h[d] = a.dt / h[d];
@@ -176,9 +179,8 @@ VAH_HD unsigned axis_update(const StageArgs<S> &a, long long s, int dir, long lo
     return fails;
 }
 
-template <typename S, typename I>
-VAH_HD void store_cell(const StageArgs<S> &a, I s, int NQ, const double *val, const double *u, double e,
-                       double p) {
+template <typename S, typename I, typename V>
+VAH_HD void store_cell(const StageArgs<S> &a, I s, int NQ, const V *val, const V *u, V e, V p) {
     for (int n = 0; n < NQ; ++n) a.qout[n][s] = (S)val[n];
     for (int m = 0; m < 4; ++m) a.uout[m][s] = (S)u[m];
     a.eout[s] = (S)e;
@@ -303,6 +305,35 @@ VAH_HD unsigned face_compute(const StageArgs<S> &a, long long s, int dir, long l
     return fails;
 }
 
+// The end of a cell's stage: counters, flags, freeze-out crossings, the stores
+// of the cell and of the face ghost layers it is the boundary cell of
+// (setGhostCellsKernelI/J/K, DynamicalVariables.cpp:400-489). st: the
+// inversion's status.
+template <typename S, typename V>
+VAH_HD void cell_store(const StageArgs<S> &a, int s, int i, int j, int k, int NQ, int st, int bad, const V *val,
+                       const V *u, V e, V p) {
+    if (st != 0 && a.counters) count_add(a.counters + 1, 1ull);
+    if ((bad || st == 2) && a.counters) count_add(a.counters + 2, 1ull);
+    if (a.fallback) a.fallback[s] = st != 0;
+    if (a.hot && a.stage2 && st == 0) {  // the isotherm e = e_freeze passed this (converged) cell during the step
+        const unsigned char was = a.hot[s], now = (double)e > a.e_freeze;
+        if (was != now) {
+            a.hot[s] = now;
+            count_add(a.crossings + (was ? 0 : 1), 1ull);
+        }
+    }
+    store_cell(a, s, NQ, val, u, e, p);
+    const int sy = a.ncx, sz = (int)a.plane;
+    if (i == 2) { store_cell(a, s - 1, NQ, val, u, e, p); store_cell(a, s - 2, NQ, val, u, e, p); }
+    if (i == a.nx + 1) { store_cell(a, s + 1, NQ, val, u, e, p); store_cell(a, s + 2, NQ, val, u, e, p); }
+    if (j == 2) { store_cell(a, s - sy, NQ, val, u, e, p); store_cell(a, s - 2 * sy, NQ, val, u, e, p); }
+    if (j == a.ny + 1) { store_cell(a, s + sy, NQ, val, u, e, p); store_cell(a, s + 2 * sy, NQ, val, u, e, p); }
+    if (a.zghosts) {
+        if (k == 2) { store_cell(a, s - sz, NQ, val, u, e, p); store_cell(a, s - 2 * sz, NQ, val, u, e, p); }
+        if (k == a.nz + 1) { store_cell(a, s + sz, NQ, val, u, e, p); store_cell(a, s + 2 * sz, NQ, val, u, e, p); }
+    }
+}
+
 // One interior cell of the split path.
 template <typename S, int PHYS, bool IS3D, bool EXACT>
 VAH_HD void cell_compute(const StageArgs<S> &a, int i, int j, int k) {
@@ -358,26 +389,7 @@ VAH_HD void cell_compute(const StageArgs<S> &a, int i, int j, int k) {
     regulate<PHYS>(a.t_inv, e, p, val, u, a.regmap[0] ? rmap : nullptr);
     if (a.regmap[0] && Phys<PHYS>::PIMUNU)
         for (int m = 0; m < 11; ++m) a.regmap[m][s] = rmap[m];
-    if (st != 0 && a.counters) count_add(a.counters + 1, 1ull);
-    if ((bad || st == 2) && a.counters) count_add(a.counters + 2, 1ull);
-    if (a.fallback) a.fallback[s] = st != 0;
-    if (a.hot && a.stage2 && st == 0) {  // the isotherm e = e_freeze passed this (converged) cell during the step
-        const unsigned char was = a.hot[s], now = e > a.e_freeze;
-        if (was != now) {
-            a.hot[s] = now;
-            count_add(a.crossings + (was ? 0 : 1), 1ull);
-        }
-    }
-    store_cell(a, s, NQ, val, u, e, p);
-    const int sy = ncx, sz = plane;
-    if (i == 2) { store_cell(a, s - 1, NQ, val, u, e, p); store_cell(a, s - 2, NQ, val, u, e, p); }
-    if (i == a.nx + 1) { store_cell(a, s + 1, NQ, val, u, e, p); store_cell(a, s + 2, NQ, val, u, e, p); }
-    if (j == 2) { store_cell(a, s - sy, NQ, val, u, e, p); store_cell(a, s - 2 * sy, NQ, val, u, e, p); }
-    if (j == a.ny + 1) { store_cell(a, s + sy, NQ, val, u, e, p); store_cell(a, s + 2 * sy, NQ, val, u, e, p); }
-    if (a.zghosts) {
-        if (k == 2) { store_cell(a, s - sz, NQ, val, u, e, p); store_cell(a, s - 2 * sz, NQ, val, u, e, p); }
-        if (k == a.nz + 1) { store_cell(a, s + sz, NQ, val, u, e, p); store_cell(a, s + 2 * sz, NQ, val, u, e, p); }
-    }
+    cell_store<S>(a, s, i, j, k, NQ, st, bad, val, u, e, p);
 }
 
 // ------------------------------------------------------------ set-up ops --

@@ -1,19 +1,12 @@
-// vah_tile_cell.cuh -- the arithmetic of the FP32 form, shared by the
-// TMA-tiled stage kernel (vah_tile.cuh) and its host build (tests/hostcheck):
-// the face flux from an accessor of the conserved fields, and the cell update.
-// State and arithmetic in FP32; the Newton inversions in FP64.
+// vah_tile_cell.cuh -- the arithmetic of the FP32 form: the cell update, shared
+// by its cell launch and the host build (tests/hostcheck), and the face flux in
+// its plain form, one face at a time, which the host build runs (the device
+// evaluates the same expressions in vah_march.cuh). State and arithmetic in
+// FP32; the Newton inversions in FP64.
 #pragma once
 
 #include "vah_physics.cuh"
-
-// The face evaluation is inlined: the tile kernel calls it from one place (a
-// loop over the face jobs of a tile), so one copy of its code sits in the
-// kernel and no call saves registers around it.
-#if defined(__CUDACC__)
-#define VAH_TILE_FACE __host__ __device__ __forceinline__
-#else
-#define VAH_TILE_FACE inline
-#endif
+#include "vah_stage.cuh"
 
 namespace vah {
 
@@ -81,7 +74,7 @@ struct ArrQ {
 // destination, e.g. a shared face buffer). Returns the number of inversions
 // that fell back; bit 8 flags a NaN (ePrev: the left cell's e).
 template <int PHYS, typename QA>
-VAH_TILE_FACE unsigned tile_face(const QA q, long long L, long long st, int dir, double t, double ePrev, double uT,
+VAH_HD unsigned tile_face(const QA q, long long L, long long st, int dir, double t, double ePrev, double uT,
                                  float *H, int hs) {
     constexpr int NQ = Phys<PHYS>::NQ;
     float qR[NQ], qL[NQ];
@@ -140,15 +133,16 @@ struct TilePrims {
 // updated conserved values to val and the cell's e (the inversion's fallback
 // energy) to e_prev; sets bad when a source is NaN. The last part of the
 // stage that reads q and the primitives around the cell.
+// k, fh (1 / 2h per axis) and dtf: the launch's constants.
 template <int PHYS, bool IS3D, typename QA>
-VAH_HD void tile_cell_explicit(const QA &q, long long b, long long bsy, long long bsz, const TilePrims &pr,
-                               long long s, const float *flux, const Eos &eos, double t_src, double dt, double dx,
-                               double dy, double dz, double etabar, float *val, float &e_prev, int &bad) {
+VAH_HD void tile_cell_explicit_at(const QA &q, long long b, long long bsy, long long bsz, const TilePrims &pr,
+                                  long long s, const float *flux, const Eos &eos, const StepConstsT<float> &k,
+                                  const float *fh, float dtf, float *val, float &e_prev, int &bad) {
     constexpr int NQ = Phys<PHYS>::NQ;
     float qc[NQ];
 #pragma unroll
     for (int n = 0; n < NQ; ++n) qc[n] = q(n, b);
-    const float fx = (float)(0.5 / dx), fy = (float)(0.5 / dy), fz = (float)(0.5 / dz);
+    const float fx = fh[0], fy = fh[1], fz = fh[2];
     const float *E = pr.E, *PP = pr.P, *UT = pr.U[0], *UX = pr.U[1], *UY = pr.U[2], *UN = pr.U[3];
     const long long c = pr.pi, sy = pr.psy, sz = pr.psz;
     CellGradT<float> g;
@@ -178,15 +172,12 @@ VAH_HD void tile_cell_explicit(const QA &q, long long b, long long bsy, long lon
         g.dnp = g.dne = g.dnpl = 0.0f;
     }
 #undef VAH_TCD
-    const StepConstsT<float> k = step_consts((float)t_src, (float)dt, (float)etabar);
     float Sv[NQ];
     bad = cell_sources<PHYS>(eos, qc, g, k, Sv);
-    const float dtf = (float)dt;
 #pragma unroll
     for (int n = 0; n < NQ; ++n) val[n] = qc[n] + dtf * Sv[n] + flux[n];
     if (Phys<PHYS>::PIMUNU) {  // pi / Pi gradient sources along each axis (SourceTerms.cpp:46-176)
         const float ucomp[3] = {g.ux, g.uy, g.un};
-        const float fh[3] = {fx, fy, fz};
         const long long sts[3] = {1, bsy, bsz};
 #pragma unroll
         for (int dir = 0; dir < (IS3D ? 3 : 2); ++dir) {
@@ -200,6 +191,16 @@ VAH_HD void tile_cell_explicit(const QA &q, long long b, long long bsy, long lon
         }
     }
     e_prev = g.e;
+}
+
+template <int PHYS, bool IS3D, typename QA>
+VAH_HD void tile_cell_explicit(const QA &q, long long b, long long bsy, long long bsz, const TilePrims &pr,
+                               long long s, const float *flux, const Eos &eos, double t_src, double dt, double dx,
+                               double dy, double dz, double etabar, float *val, float &e_prev, int &bad) {
+    const float fh[3] = {(float)(0.5 / dx), (float)(0.5 / dy), (float)(0.5 / dz)};
+    tile_cell_explicit_at<PHYS, IS3D>(q, b, bsy, bsz, pr, s, flux, eos,
+                                      step_consts((float)t_src, (float)dt, (float)etabar), fh, (float)dt, val, e_prev,
+                                      bad);
 }
 
 // The rest of the cell's stage ([the convex combination],
@@ -242,5 +243,45 @@ VAH_HD int tile_cell(const QA &q, long long b, long long bsy, long long bsz, con
     return tile_cell_invert<PHYS>(pr, s, qavg, stage2, eos, t_inv, e_prev, val, e, p, u, rmap);
 }
 
+// One interior cell of the FP32 form's stage: the flux differences summed in
+// axis order, the update above, the stores and ghost layers of cell_compute.
+template <int PHYS, bool IS3D>
+VAH_HD void cell_compute_f32(const StageArgs<float> &a, int i, int j, int k) {
+    constexpr int NQ = Phys<PHYS>::NQ;
+    const int ncx = a.ncx, plane = (int)a.plane, s = i + ncx * j + plane * k;
+    float flux[NQ];
+    const float c[3] = {(float)a.c_h[0], (float)a.c_h[1], (float)a.c_h[2]};
+#pragma unroll
+    for (int n = 0; n < NQ; ++n) {
+        flux[n] = c[0] * ldg(a.D[0][n] + s);
+#pragma unroll
+        for (int d = 1; d < (IS3D ? 3 : 2); ++d) flux[n] = fmaf(c[d], ldg(a.D[d][n] + s), flux[n]);
+    }
+    struct Fields {
+        const float *const *f;
+        VAH_HD float operator()(int n, long long at) const { return ldg(f[n] + at); }
+    };
+    TilePrims pr;
+    pr.E = a.ein;
+    pr.P = a.pin;
+    for (int m = 0; m < 4; ++m) {
+        pr.U[m] = a.uin[m];
+        pr.UP[m] = a.upin[m];
+        pr.G[m] = a.guess[m];
+    }
+    pr.pi = s;
+    pr.psy = ncx;
+    pr.psz = plane;
+    const float fh[3] = {(float)a.inv2h[0], (float)a.inv2h[1], (float)a.inv2h[2]};
+    float val[NQ], e_prev, e, p, u[4], rmap[11];
+    int bad = 0;
+    tile_cell_explicit_at<PHYS, IS3D>(Fields{a.qin}, s, ncx, plane, pr, s, flux, a.eos, a.ksrc_f, fh, (float)a.dt, val,
+                                      e_prev, bad);
+    const int st = tile_cell_invert<PHYS>(pr, s, Fields{a.qavg}, a.stage2 != 0, a.eos, a.t_inv, e_prev, val, e, p, u,
+                                          a.regmap[0] ? rmap : nullptr);
+    if (a.regmap[0] && Phys<PHYS>::PIMUNU)
+        for (int m = 0; m < 11; ++m) a.regmap[m][s] = (double)rmap[m];
+    cell_store<float>(a, s, i, j, k, NQ, st, bad, val, u, e, p);
+}
 
 }  // namespace vah
