@@ -28,6 +28,43 @@ constexpr int kFluxMinb = sizeof(S) == 8 ? 4 : 5;
 template <typename S, bool IS3D>
 constexpr int kCellMinb = sizeof(S) == 4 ? 10 : (IS3D ? 8 : 6);
 
+// The stage launches of small FP64 2+1D events follow one another as
+// programmatic dependents: a launch's blocks may become resident while the last
+// blocks of the one before it still run, and wait there for its end before they
+// read anything it or an earlier launch wrote (after_previous_launch, which also
+// lets the next launch in). Every stage launch waits, so each one's end implies
+// those before it. That takes launch latency and a grid's ramp-up off the
+// chain: 45.5 -> 40.5 us per step at 61x61, 63.3 -> 62.1 at 200x200, 171.8 ->
+// 163.3 at 401x389. Elsewhere it gains nothing or loses, since cell blocks that
+// start beside flux blocks inherit their split of L1 and shared memory: 25x23x9
+// 50.4 -> 52.7, 121x121x81 616 -> 679 us per stage, FP32 200x200 55.6 -> 66.2.
+constexpr int kDependentCells = 189440;  // 2.5 waves of 16 warps per SM
+template <typename S>
+bool follows_closely(const StageArgs<S> &a) {
+    return sizeof(S) == 8 && a.nz == 1 && (long long)a.nx * a.ny <= kDependentCells;
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void after_previous_launch() {
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+template <typename... P, typename... A>
+cudaError_t launch_stage_kernel(void (*kernel)(P...), bool dependent, int grid, int block, size_t smem,
+                                cudaStream_t stream, A... args) {
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = dependent;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+#endif
+
 // Cells per march segment along an axis of n cells, from the number of warps
 // a segment length makes: the fewest waves (148 SMs x minb blocks x 4 warps)
 // times the segment's length plus its start-up (one face and its first

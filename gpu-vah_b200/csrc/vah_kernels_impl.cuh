@@ -51,6 +51,7 @@ struct FluxGrid {
 template <typename S, int PHYS, bool EXACT>
 __global__ void __launch_bounds__(kFluxThreads, kFluxMinb<S>) flux_kernel(const StageArgs<S> a, const FluxGrid g) {
     extern __shared__ __align__(16) unsigned char flux_sm[];
+    after_previous_launch();
     const SelectPointers<S, PHYS> sel{a};
     const int warp = threadIdx.x / 32;
     int block = blockIdx.x;
@@ -100,6 +101,7 @@ __global__ void pack_kernel(S *__restrict__ field, double *__restrict__ packed, 
 template <typename S, int PHYS, bool IS3D>
 __global__ void __launch_bounds__(kCellThreads, kCellMinb<S, IS3D>) cell_kernel(const StageArgs<S> a) {
     const int c = blockIdx.x * kCellThreads + threadIdx.x;
+    after_previous_launch();
     if (c >= a.nx * a.ny * (a.k1 - a.k0)) return;
     const int r = c / a.nx, i = c - r * a.nx, k = r / a.ny, j = r - k * a.ny;
     if constexpr (sizeof(S) == 4) cell_compute_f32<PHYS, IS3D>(a, i + 2, j + 2, k + a.k0 + 2);
@@ -208,15 +210,13 @@ cudaError_t flux_launch(const StageArgs<S> &a, int kind, cudaStream_t stream) {
     if (a.nz > 1 && (kind == kFaceZ || kind == kCell)) march(a.nx * a.ny, planes, g.zstrips, g.zseg, g.zblocks);
     const int grid = g.xblocks + g.yblocks + g.zblocks;
     if (grid == 0) return cudaSuccess;
-    kernel<<<grid, kFluxThreads, smem, stream>>>(a, g);
-    return cudaGetLastError();
+    return launch_stage_kernel(kernel, follows_closely(a), grid, kFluxThreads, smem, stream, a, g);
 }
 
 template <typename S, int PHYS, bool IS3D>
 cudaError_t cell_launch(const StageArgs<S> &a, cudaStream_t stream) {
     const int cells = a.nx * a.ny * (a.k1 - a.k0);
-    cell_kernel<S, PHYS, IS3D><<<(cells + kCellThreads - 1) / kCellThreads, kCellThreads, 0, stream>>>(a);
-    return cudaGetLastError();
+    return launch_stage_kernel(cell_kernel<S, PHYS, IS3D>, follows_closely(a), (cells + kCellThreads - 1) / kCellThreads, kCellThreads, 0, stream, a);
 }
 
 template <typename S, int PHYS>
