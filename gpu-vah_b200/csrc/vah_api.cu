@@ -345,11 +345,11 @@ extern "C" int vah_event_create(const vah_lattice *lat, const vah_hydro *hydro, 
         ev->stream = (cudaStream_t)opt->stream;
     }
     // one allocation: the state (2 N_q + 16 arrays), then the flux differences
-    // of as many planes as 1 GB holds (at least one; a stage runs slab by slab)
+    // of as many planes as 4 GB holds (at least one; a stage runs slab by slab)
     const bool split = opt->flux != VAH_FLUX_PER_CELL_FUSED || ev->elem == sizeof(float);
     const int ndir = lat->nz > 1 ? 3 : 2;
     const size_t plane = (size_t)ev->ncx * ev->ncy * ev->elem;
-    ev->d_planes = (int)std::min<size_t>(lat->nz, std::max<size_t>(1, ((size_t)1 << 30) / (plane * ndir * ev->nq)));
+    ev->d_planes = (int)std::min<size_t>(lat->nz, std::max<size_t>(1, ((size_t)4 << 30) / (plane * ndir * ev->nq)));
     auto padded = [](size_t n) { return (n + 255) / 256 * 256; };
     const size_t field = padded(ev->ncell * ev->elem), diff = padded(plane * ev->d_planes);
     const size_t state = field * (2 * ev->nq + 16);

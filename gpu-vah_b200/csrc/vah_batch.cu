@@ -368,8 +368,8 @@ int nq_of(int physics) { return physics == VAH_IDEAL ? 5 : (physics == VAH_PIMUN
 constexpr int kArraysPerEvent = 48;
 
 // The scratch that a group's flux differences share; an event that needs more
-// is a group of its own. With 1 GB the 256-event batch is one group.
-constexpr size_t kScratchBytes = (size_t)1 << 30;
+// is a group of its own. With 4 GB the 256-event batch is one group.
+constexpr size_t kScratchBytes = (size_t)4 << 30;
 
 size_t event_bytes(const vah_batch *b, const vah_lattice *lat) {
     const size_t ncell = (size_t)(lat->nx + 4) * (lat->ny + 4) * (lat->nz + 4);

@@ -455,10 +455,10 @@ VAH_HD void invert_root(double t, const InvIn &q, InvRoot &r) {
     r.s2 = 2 * bT2 * r.inv;
     r.bT = sqrt_estimate(bT2);
     r.G1 = 0.5 * b * r.bT;
-    // a root well below the parabola's top, u_T < 31, e > 0, and magnitudes
+    // a root well below the parabola's top, u_T and the longitudinal gamma < 31, e > 0, and magnitudes
     // at which the estimates above hold (b >= 1, so bT2 < G0^2 / 2)
-    const bool in = r.G0 > 1e-100 && r.G0 < 1e100 && disc > 1e-4 * G02 && r.s2 < (1 - 1e-5) * r.c0 &&
-                    2 * r.s2 * r.inv < 1 - 1e-3 && r.x2 > 1e-6;
+    const bool in = r.G0 > 1e-100 && r.G0 < 1e100 && disc > 1e-2 * G02 && r.s2 < (1 - 1e-5) * r.c0 &&
+                    2 * r.s2 * r.inv < 1 - 1e-3 && r.x2 > 1e-3;
     if (!in) r.G0 = NAN;
 }
 
