@@ -64,7 +64,7 @@ def parse():
     ap.add_argument("--extras-serve-seconds", type=float, default=2.0,
                     help="arrival window of the serving measurement in the extras (s)")
     ap.add_argument("--flux", default="per_cell", choices=["per_cell", "shared", "fused"],
-                    help="per_cell: reference face semantics, face+cell launches; fused: the same in one "
+                    help="per_cell: reference face semantics, flux+cell launches; fused: the same in one "
                          "launch per stage; shared: each face evaluated once")
     return ap.parse_args()
 
@@ -331,7 +331,7 @@ FP64_PEAK_TFLOPS = 64 * 2 * 148 * 1.965e9 / 1e12
 def fp64_roofline(cells, flux, precision, stage_s, peak=None):
     """FP64 FLOP/s of one RK stage against the FP64 peak (measured when given,
     else nominal), from the FLOP count per cell and stage in the committed ncu
-    summary (the FP32 form: the tile kernel's)."""
+    summary (the FP32 form: its own)."""
     tile = precision == "fp32"
     path = os.path.join(ROOT, "profiles", "tile_stage_dram.json" if tile else "split_stage_dram.json")
     if (flux != "per_cell" and not tile) or not os.path.exists(path) or not stage_s:
@@ -354,7 +354,7 @@ def fp64_roofline(cells, flux, precision, stage_s, peak=None):
 def traffic_per_launch(cells, flux, precision):
     """DRAM bytes of one RK stage (its launches) from the committed ncu
     summaries (bytes per interior cell, scaled to this event), or None. The
-    FP32 form runs the tile kernel whatever the face option."""
+    FP32 form evaluates faces once whatever the face option."""
     if precision == "fp32":
         path = os.path.join(ROOT, "profiles", "tile_stage_dram.json")
         if not os.path.exists(path):
@@ -439,7 +439,7 @@ def run_batch(args, rank, world, dist):
             "config": {"workload": f"vah batch: {args.events} 2+1D MC-Glauber events, sides {BATCH_SIDES}, dx=0.1, "
                                    f"b~U[0,12], table EoS, shear+bulk, dtau={BATCH_DT}",
                        "events": args.events, "cells_per_step": cells, "faces": args.flux,
-                       "l2": "inputs larger than L2", "launch": "persistent tile work-list, CUDA graph per step",
+                       "l2": "inputs larger than L2", "launch": "one work-list launch per flux and cell stage, CUDA graph per step",
                        "autotune": {k: c for k, c in zip(("face_x", "face_y", "face_z", "cell_2d", "cell_3d"), tune)}},
             "events_step_per_s": world * args.events * args.steps / elapsed,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
@@ -823,15 +823,15 @@ def run_vah(args, rank, world, dist):
                          "frac": achieved / peak, "traffic": traffic_per_launch(cells, args.flux, args.precision),
                          "peak_kind": f"{peak_kind} copy bandwidth",
                          "algorithmic_bytes_per_cell_update": bpc,
-                         "kernel": ("tile_kernel (one TMA-tiled launch per RK stage)" if prec == vah.VAH_FP32
+                         "kernel": ("one RK stage: flux_kernel + cell_kernel, FP32 form" if prec == vah.VAH_FP32
                                     else "stage_kernel (one fused RK stage)" if args.flux == "fused"
-                                    else "one RK stage: face_kernel x3 + cell_kernel") + ", average over the two stages",
+                                    else "one RK stage: flux_kernel + cell_kernel") + ", average over the two stages",
                          "avg_stage_ms": 1000 * avg_launch_s,
                          "fp64": fp64_roofline(cells, args.flux, args.precision, avg_launch_s, fp64_peak)},
             "e2e": {"value": e2e_value, "unit": "cell-updates/s", "h2d_bytes_per_step": state_bytes,
                     "d2h_bytes_per_step": state_bytes, "steps": args.e2e_steps,
                     "path": "vah_rk2_step_host (pinned host state in, one step, state out)"},
-            "gpu_launches": launches * (1 if args.flux == "fused" or prec == vah.VAH_FP32 else 4),
+            "gpu_launches": launches * (1 if args.flux == "fused" and prec != vah.VAH_FP32 else 2),
             "stats": {"face_fallbacks": stats.face_fallbacks, "cell_fallbacks": stats.cell_fallbacks,
                       "nan_cells": stats.nan_cells}}
     clk_summary = clk.summary()
@@ -851,8 +851,8 @@ def run_vah(args, rank, world, dist):
                                   "fp64": fp64_roofline(cells, args.flux,
                                                         "fp32" if other == vah.VAH_FP32 else "fp64",
                                                         form["avg_stage_ms"] / 1000.0, fp64_peak),
-                                  "kernel": "tile_kernel (one TMA-tiled launch per stage)" if other == vah.VAH_FP32
-                                  else "one RK stage: face_kernel x3 + cell_kernel"}})
+                                  "kernel": "one RK stage: flux_kernel + cell_kernel, FP32 form" if other == vah.VAH_FP32
+                                  else "one RK stage: flux_kernel + cell_kernel"}})
         line["fp32_form" if other == vah.VAH_FP32 else "fp64_form"] = form
         line["late"] = {name: late_regime_rates(vah, table, e0, p, local, stream)
                         for name, p in (("fp64", vah.VAH_FP64), ("fp32", vah.VAH_FP32))}

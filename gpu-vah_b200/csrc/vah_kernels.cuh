@@ -107,8 +107,7 @@ struct FieldSet {
 };
 
 // The set-up launches below index cell (i, j, k) of the ghosted grid at
-// i + pitch (j + (ny + 4) k): pitch = nx + 4 in the reference layout, or the
-// padded pitch of the tile layout.
+// i + pitch (j + (ny + 4) k): pitch = nx + 4 in the reference layout.
 // Primitive -> conserved over the interior (setConservedVariables):
 // q = 16 conserved slots, u/up = 4 velocity components each.
 template <typename S>

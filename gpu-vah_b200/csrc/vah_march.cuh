@@ -21,7 +21,7 @@
 // values per state), the lower lane finds the right state's root and the upper
 // lane the left one's, and they exchange the two velocities. FP32 faces fit one
 // lane (W = 32); split, their roots' overhead came twice as often (205 us
-// against SPLITUS for all axes).
+// against 178 for all axes).
 // Each writes H(-1/2) - H(+1/2) as the cell evaluates the two faces, which the
 // cell launch reads.
 // S: the storage and arithmetic type of states and fluxes (double, or float

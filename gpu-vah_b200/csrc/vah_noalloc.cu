@@ -5,10 +5,9 @@
 // queue work from a context where cudaMalloc is forbidden or would
 // synchronise the device, and processes that must keep their device
 // footprint fixed after start-up. vah_stage_noalloc serves them. It runs one
-// RK stage of the face/cell split (reference face semantics, FP64 storage)
-// on state buffers the caller owns, and keeps the stage's scratch -- the face
-// fluxes as each neighbour evaluates them, plus the fallback/NaN counters --
-// in the file-scope array below instead of allocating it.
+// RK stage of the flux/cell split (reference face semantics, FP64 storage)
+// on state buffers the caller owns, and keeps the stage's scratch -- the flux
+// differences along each axis, plus the fallback/NaN counters -- in the file-scope array below instead of allocating it.
 //
 // The array is a fixed part of the library's device image: every GPU that
 // loads libvah.so holds its VAH_NOALLOC_SCRATCH_BYTES until the process

@@ -283,7 +283,7 @@ class Event:
         return out
 
     def autotune(self, reps=3):
-        """Pick the fastest launch configuration per kernel kind (vah_event_autotune); returns the choices."""
+        """Time each launch kind on the event's state (vah_event_autotune)."""
         r = TuneReport()
         check(self.L.vah_event_autotune(self.ev, int(reps), C.byref(r)), "vah_event_autotune")
         return r.as_list()
@@ -446,7 +446,7 @@ class Batch:
         return ms.value, n.value
 
     def autotune(self, reps=3):
-        """Pick the fastest register-cap variant per launch kind (vah_batch_autotune); returns the choices."""
+        """Time the batch's launch kinds (vah_batch_autotune)."""
         r = TuneReport()
         check(self.L.vah_batch_autotune(self.b, int(reps), C.byref(r)), "vah_batch_autotune")
         return r.as_list()

@@ -50,13 +50,13 @@ extern "C" {
 /* ---- storage precision ---- */
 #define VAH_FP64 0 /* state stored and updated in FP64 */
 #define VAH_FP32 1 /* state, reconstruction, flux and sources in FP32; Newton inversions, closure fits and
-                     reductions in FP64; one TMA-tiled launch per RK stage */
+                     reductions in FP64; faces evaluated once (VAH_FLUX_SHARED's semantics) */
 
 /* ---- face-flux evaluation ---- */
 #define VAH_FLUX_PER_CELL 0       /* each face evaluated by both neighbouring cells with that cell's
                                      Newton guess and fallback energy, as the reference does
-                                     (FullyDiscreteKurganovTadmorScheme.cpp:179,183); face and cell
-                                     launches per stage, face fluxes in scratch buffers */
+                                     (FullyDiscreteKurganovTadmorScheme.cpp:179,183); a flux and a
+                                     cell launch per stage, flux differences in scratch buffers */
 #define VAH_FLUX_SHARED 1         /* each face evaluated once, with the left cell's guess and fallback
                                      energy: equal to the reference up to the Newton tolerance squared
                                      where inversions converge; it does not reproduce the reference's
@@ -243,19 +243,18 @@ int vah_event_set_validity(vah_event *ev, int on);
 int vah_event_get_validity(vah_event *ev, int id, double *host, int with_ghosts);
 
 /* ---- launch autotuning (no reference counterpart) ----
- * The face/cell kernels come in register-cap variants and take their block
- * shape at run time. vah_event_autotune times every candidate of each launch
- * kind (face x, face y, face z, cell; `reps` timed launches each, after one
- * warm-up) on the event's current state, keeps the fastest for the event's
- * later steps, and reports the choice and its time next to the default's.
- * It writes only stage scratch (the state is unchanged) and synchronises the
- * event's stream. Results do not depend on the choice. The fused flux mode has
- * nothing to tune (nkinds = 0). vah_batch_autotune does the same for a
- * batch's persistent launches (register cap only; tiles stay 32 x 4). */
+ * Each launch kind has one configuration, so there is nothing to choose:
+ * vah_event_autotune times the kinds (flux differences along x, y and eta, each
+ * launched by itself, and the cells; `reps` timed launches after one warm-up)
+ * on the event's current state and reports them (ms_best = ms_default; 0 for
+ * the eta kind in 2+1D). It writes only stage scratch (the state is unchanged)
+ * and synchronises the event's stream. The fused flux mode and the FP32 form
+ * report nothing (nkinds = 0). vah_batch_autotune reports a batch's flux launch
+ * (as the first of the flux kinds) and its 2+1D and 3+1D cell launches. */
 typedef struct vah_launch_choice {
-    int bx, by, minb;   /* block shape and minimum resident blocks per SM the compiler was held to */
-    double ms_default;  /* ms per launch of the configuration in use before the call */
-    double ms_best;     /* ms per launch of the chosen configuration */
+    int bx, by, minb;   /* 32 x 4 threads, and the resident blocks of that size per SM the compiler was held to */
+    double ms_default;  /* ms per launch */
+    double ms_best;     /* the same */
 } vah_launch_choice;
 typedef struct vah_tune_report {
     int nkinds;
@@ -273,15 +272,12 @@ int vah_event_autotune(vah_event *ev, int reps, vah_tune_report *out);
  * way back) by a kernel, through device staging in the host layout that the
  * first such call allocates (one field; every field where the copies
  * overlap).
- * FP64 storage, face/cell split, validity off and nz >= 6: the copies
+ * Flux/cell split or FP32 storage, validity off and nz >= 6: the copies
  * overlap the stages. The lattice is cut into slabs of planes along eta
  * (VAH_HOST_SLAB_PLANES planes each when that environment variable is set to
  * 2 or more, else nz / 6); copy-in of later slabs, the stages of earlier ones
  * and copy-out of finished ones run on three streams (the event's stream and
- * two the first such call creates), with the same results bit for bit.
- * FP32 storage, 3+1D, validity off: the same, in slabs of whole 4-plane tile
- * layers (the thickness above rounded to layers), where that gives at least
- * 3 slabs. The arrays should be pinned (cudaHostAlloc / cudaHostRegister)
+ * two the first such call creates), with the same results bit for bit. The arrays should be pinned (cudaHostAlloc / cudaHostRegister)
  * for the copies to overlap; pageable arrays give the same results, more
  * slowly. */
 int vah_rk2_step_host(vah_event *ev, double t, double dt, double *const *fields);
@@ -289,11 +285,13 @@ int vah_rk2_step_host(vah_event *ev, double t, double dt, double *const *fields)
 /* ---- batches: many events of uneven size in one launch per kernel kind ----
  * No single reference counterpart: the reference advances one event per
  * process (HydroPlugin.cpp:130-242). A batch keeps every admitted event's
- * state device-resident and advances all of them together: each launch walks
- * a work-list of 32x4-cell tiles over all events in a grid-stride loop, and
- * one RK2 step of the whole batch (face and cell launches of both stages and
- * the per-event clock advance) is replayed from a CUDA graph that is
- * re-captured only when events are added or removed. Every event keeps its
+ * state device-resident and advances all of them together: a launch's blocks
+ * take the items of a work-list over all events, and one RK2 step of the whole
+ * batch (flux and cell launches of both stages and the per-event clock
+ * advance) is replayed from a CUDA graph that is re-captured only when events
+ * are added or removed. The flux differences of a stage are scratch that the
+ * events share (up to 4 GB, or the largest event's; larger batches step in
+ * groups), allocated at the first step and not part of an event's footprint. Every event keeps its
  * own time and dt; all share the batch's physics options (VAH_FLUX_PER_CELL
  * or VAH_FLUX_SHARED). Admission is by device footprint: vah_batch_add
  * returns VAH_ERR_FULL when the event would exceed capacity_bytes. */
@@ -389,8 +387,7 @@ int vah_batch_freezeout_volume(vah_batch *b, double *out, int nslots);
 int vah_batch_fallback_mask(vah_batch *b, int slot, unsigned char *host);
 int vah_batch_set_timing(vah_batch *b, int on);
 int vah_batch_kernel_time(vah_batch *b, double *ms, long long *steps);
-/* Register-cap autotuning of the batch's launch kinds (face x, y, z, cell
- * 2+1D, cell 3+1D), as vah_event_autotune describes. */
+/* The batch form of vah_event_autotune: 5 kinds (flux; two unused; cell 2+1D, cell 3+1D). */
 int vah_batch_autotune(vah_batch *b, int reps, vah_tune_report *out);
 
 /* ---- serving: continuous batching of an open-loop request stream ----
@@ -456,9 +453,9 @@ int vah_ic_longitudinal(int nz, double dz, double eta_flat, double sigma_eta, do
  * allocate device memory (code inside a framework that owns all device memory
  * through its own pool, work queued where cudaMalloc is not allowed or would
  * synchronise the device, processes whose device footprint must stay fixed).
- * It runs one RK stage -- the face/cell launches with the reference's face
+ * It runs one RK stage -- the flux and cell launches with the reference's face
  * semantics, FP64 storage -- on state buffers the caller owns, and keeps the
- * stage's scratch (face fluxes, fallback counters) in a fixed array of
+ * stage's scratch (flux differences, fallback counters) in a fixed array of
  * VAH_NOALLOC_SCRATCH_BYTES inside the library, held by every GPU that loads
  * libvah.so until exit. It calls no allocator. Limit: 256 +
  * (2 or 3 axes) * N_q * 2 * 8 bytes per ghosted cell must fit, i.e. at most
