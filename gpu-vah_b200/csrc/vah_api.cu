@@ -760,8 +760,8 @@ int autotune_split(vah_event *ev, int reps, vah_tune_report *out) {
     int rc = VAH_OK;
     out->nkinds = vah::kNumSplitKinds;
     for (int kind = 0; kind < vah::kNumSplitKinds && rc == VAH_OK; ++kind) {
-        // as 128-thread blocks: 4 flux blocks, 7 cell blocks of 64 per SM
-        out->kind[kind] = {32, 4, kind == vah::kCell ? 3 : 4, 0.0, 0.0};
+        // as 128-thread blocks per SM: 4 flux blocks; 8 (2+1D: 6) cell blocks of 64
+        out->kind[kind] = {32, 4, kind == vah::kCell && ev->lat.nz == 1 ? 3 : 4, 0.0, 0.0};
         if (kind == vah::kFaceZ && ev->lat.nz == 1) continue;  // no eta faces in 2+1D
         bool ok = launch(kind) && cudaEventRecord(e0, ev->stream) == cudaSuccess;
         for (int r = 0; r < reps && ok; ++r) ok = launch(kind);

@@ -1,4 +1,4 @@
-// vah_batch.cu -- many events, one persistent launch per kernel kind.
+// vah_batch.cu -- many events, one launch per kernel kind.
 //
 // A batch holds up to kMaxSlots events of independent grid sizes. Every
 // launch of a step covers all events: a block takes an item of a work-list
@@ -7,7 +7,7 @@
 // The per-event state lives in one device allocation per event (stream-
 // ordered, from the batch's memory pool); per-event descriptors (buffer
 // pointers, geometry) and clocks (time, u/u_prev parity, step count) live in
-// device arrays, so a whole RK2 step -- face and cell launches of both stages
+// device arrays, so a whole RK2 step -- flux and cell launches of both stages
 // plus the clock advance -- is captured once as a CUDA graph and replayed.
 // The graph is re-captured only when events are added or removed.
 // The flux differences of a stage are scratch that events share: where one
@@ -1165,7 +1165,7 @@ int batch_autotune(vah_batch *b, int reps, vah_tune_report *out) {
     out->nkinds = 5;
     for (int kind = 0; kind < 5 && rc == VAH_OK; ++kind) {
         const int list = kind < 3 ? K_FLUX : (kind == 3 ? K_C2 : K_C3);
-        out->kind[kind] = {kTX, kTY, kind < 3 ? 4 : 3, 0.0, 0.0};
+        out->kind[kind] = {kTX, kTY, kind == 3 ? 3 : 4, 0.0, 0.0};
         if (kind == 1 || kind == 2 || b->groups.empty() || b->groups[0].count[list] == 0) continue;
         auto launch = [&]() { return launch_list_any(b, b->groups[0], list, 1) == cudaSuccess; };
         bool ok = launch() && cudaEventRecord(e0, b->stream) == cudaSuccess;
