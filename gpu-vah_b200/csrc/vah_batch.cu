@@ -368,7 +368,9 @@ int nq_of(int physics) { return physics == VAH_IDEAL ? 5 : (physics == VAH_PIMUN
 constexpr int kArraysPerEvent = 48;
 
 // The scratch that a group's flux differences share; an event that needs more
-// is a group of its own. With 4 GB the 256-event batch is one group.
+// is a group of its own. With 4 GB a batch of 256 2+1D events (sides 81 to
+// 201, 5.84 M cells) is one group: as two, its FP64 step had twice the launches
+// and their tails (6.10 against 5.98 ms).
 constexpr size_t kScratchBytes = (size_t)4 << 30;
 
 size_t event_bytes(const vah_batch *b, const vah_lattice *lat) {
@@ -482,9 +484,9 @@ int rebuild_work(vah_batch *b) {
     };
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cells(x) > cells(y); });
     // groups of events whose differences the scratch holds
-    auto per_field = [&](int s) {  // bytes of one field of differences
+    auto per_field = [&](int s) {  // bytes of one field of differences, which interior planes alone have
         const vah_lattice &l = b->slots[s].lat;
-        return ((size_t)(l.nx + 4) * (l.ny + 4) * (l.nz + 4) * sizeof(S) + 255) / 256 * 256;
+        return ((size_t)(l.nx + 4) * (l.ny + 4) * l.nz * sizeof(S) + 255) / 256 * 256;
     };
     auto scratch_of = [&](int s) { return per_field(s) * (b->slots[s].lat.nz > 1 ? 3 : 2) * b->nq; };
     std::vector<std::vector<int>> members;
@@ -539,7 +541,7 @@ int rebuild_work(vah_batch *b) {
                 lists[l.nz > 1 ? vah::K_C3 : vah::K_C2].push_back({s, 0, c0, 0, 0});
             SlotDesc<S> &d = *desc_host<S>(b, s);
             for (int k = 0; k < (l.nz > 1 ? 3 : 2); ++k)
-                for (int n = 0; n < b->nq; ++n, at += per_field(s)) d.D[k][n] = (S *)at;
+                for (int n = 0; n < b->nq; ++n, at += per_field(s)) d.D[k][n] = (S *)at - 2 * d.plane;
         }
         for (int k = 0; k < vah::K_NUM; ++k) g.count[k] = (int)lists[k].size() - g.first[k];
         b->groups.push_back(g);
