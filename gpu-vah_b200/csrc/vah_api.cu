@@ -969,14 +969,19 @@ int step_host_fp32(vah_event *ev, double t, double dt, double *const *fields) {
     return vah_event_sync(ev);
 }
 
-// Slab boundaries along eta for the overlapped host-buffer step: nz / thick
-// slabs (at least one) of as equal a thickness as nz allows, each of at least
-// `thick` >= 2 planes. (Thinner first and last slabs shorten the pipeline's
+// Slabs along eta for the overlapped host-buffer step, each of about `thick`
+// planes. FP64: nz / thick, of at least 2 planes. The FP32 form, whose slabs
+// also cost two conversions each, counts in layers of 4 planes, so that thin
+// lattices make fewer (33x41x12: 0.80 ms per step in 3 slabs, 1.19 in 6).
+int slab_count(int nz, int thick, bool fp32) {
+    if (!fp32) return std::max(1, nz / std::max(2, thick));
+    return std::max(1, (nz + 3) / 4 / std::max(1, (thick + 2) / 4));
+}
+
+// Their boundaries: of as equal a thickness as nz allows. (Thinner first and last slabs shorten the pipeline's
 // fill and drain but make more, smaller copies, which cost more than they
 // save on PCIe: measured on the 121x121x81 event.)
-std::vector<int> slab_bounds(int nz, int thick) {
-    thick = std::max(2, thick);
-    const int n = std::max(1, nz / thick);
+std::vector<int> slab_bounds(int nz, int n) {
     std::vector<int> b = {0};
     for (int m = 0; m < n; ++m) b.push_back(b.back() + nz / n + (m < nz % n ? 1 : 0));
     return b;
@@ -993,10 +998,9 @@ std::vector<int> slab_bounds(int nz, int thick) {
 // Host planes are read (copy-in) before they are written back (copy-out):
 // each copy-out covers planes that the copy-ins before the slab's stage 1
 // have read. One compute stream keeps the face buffers' reuse in order.
-int step_host_pipelined(vah_event *ev, double t, double dt, double *const *fields, int thick) {
+int step_host_pipelined(vah_event *ev, double t, double dt, double *const *fields, int nslab) {
     const int nz = ev->lat.nz;
-    const std::vector<int> bound = slab_bounds(nz, thick);
-    const int nslab = (int)bound.size() - 1;
+    const std::vector<int> bound = slab_bounds(nz, nslab);
     const size_t pbytes = (size_t)ev->ncx * ev->ncy * sizeof(double);
     if (!ev->s_in) VAH_TRY(cudaStreamCreateWithFlags(&ev->s_in, cudaStreamNonBlocking));
     if (!ev->s_out) VAH_TRY(cudaStreamCreateWithFlags(&ev->s_out, cudaStreamNonBlocking));
@@ -1102,10 +1106,9 @@ __global__ void widen_rows_kernel(FieldRows f, int hx, int pitch, size_t r0, siz
 // into a device copy of the host layout (d_stage_all) and are narrowed into
 // the FP32 fields on the event's stream before its stage 1; after its stage 2
 // they are widened there and copied back.
-int step_host_fp32_pipelined(vah_event *ev, double t, double dt, double *const *fields, int thick) {
+int step_host_fp32_pipelined(vah_event *ev, double t, double dt, double *const *fields, int nslab) {
     const int nz = ev->lat.nz, hx = ev->lat.nx + 4;
-    const std::vector<int> bound = slab_bounds(nz, thick);
-    const int nslab = (int)bound.size() - 1;
+    const std::vector<int> bound = slab_bounds(nz, nslab);
     const size_t hplane = (size_t)hx * ev->ncy, hn = hplane * ev->ncz;  // doubles per host plane, field
     if (!ev->d_stage_all) VAH_TRY(cudaMalloc((void **)&ev->d_stage_all, VAH_NUM_FIELDS * hn * sizeof(double)));
     if (!ev->s_in) VAH_TRY(cudaStreamCreateWithFlags(&ev->s_in, cudaStreamNonBlocking));
@@ -1222,16 +1225,17 @@ extern "C" int vah_rk2_step_host(vah_event *ev, double t, double dt, double *con
         return v ? atoi(v) : 0;
     }();
     const int slab = slab_env >= 2 ? slab_env : std::max(2, ev->lat.nz / 6);
+    const int nslab = slab_count(ev->lat.nz, slab, ev->elem != sizeof(double));
     if (ev->elem != sizeof(double)) {
-        if (!ev->validity && ev->lat.nz >= 3 * slab) {
+        if (!ev->validity && nslab >= 3) {
             if (!(dt > 0) || !(t > 0)) return VAH_ERR_ARG;
-            return step_host_fp32_pipelined(ev, t, dt, fields, slab);
+            return step_host_fp32_pipelined(ev, t, dt, fields, nslab);
         }
         return step_host_fp32(ev, t, dt, fields);
     }
-    if (ev->opt.flux != VAH_FLUX_PER_CELL_FUSED && !ev->validity && ev->lat.nz >= 3 * slab) {
+    if (ev->opt.flux != VAH_FLUX_PER_CELL_FUSED && !ev->validity && nslab >= 3) {
         if (!(dt > 0) || !(t > 0)) return VAH_ERR_ARG;
-        return step_host_pipelined(ev, t, dt, fields, slab);
+        return step_host_pipelined(ev, t, dt, fields, nslab);
     }
     const size_t bytes = ev->ncell * sizeof(double);
     // all copies are queued on the event's stream; one synchronisation at the end
