@@ -138,6 +138,26 @@ VAH_HD float quot(float f, float d) { return f / d; }
 VAH_HD double quot(double f, double, double inv_d) { return f * inv_d; }
 VAH_HD float quot(float f, float d, float) { return f / d; }
 
+// Sums of products. The compiler fuses one product of a b + c d, and whichever
+// it takes depends on the code around it. Dilute edge cells of 2+1D events amplify
+// a last bit of the FP32 form about 1e8 times within 50 steps (u off by 0.02
+// in such a cell), so the form's results are no more reproducible than its
+// bits: sums that came out differently in two of its kernels say here which
+// product is fused (fused) and which is rounded by itself (rounded,
+// add_rounded). The FP64 form leaves the first two to the compiler and fuses the last.
+VAH_HD double fused(double a, double b, double c) { return a * b + c; }
+VAH_HD float fused(float a, float b, float c) { return fmaf(a, b, c); }
+VAH_HD double rounded(double a, double b) { return a * b; }
+VAH_HD float rounded(float a, float b) {
+#ifdef __CUDA_ARCH__
+    return __fmul_rn(a, b);
+#else
+    return a * b;
+#endif
+}
+VAH_HD double add_rounded(double a, double b, double c) { return fma(a, b, c); }
+VAH_HD float add_rounded(float a, float b, float c) { return rounded(a, b) + c; }
+
 }  // namespace vah
 
 #include "vah_closure_polys.h"
@@ -750,7 +770,7 @@ VAH_HD int cell_sources(const Eos &eos, const R *Q, const CellGradT<R> &g, const
     const R dtuy = (uy - g.uyp) * inv_dt, dtun = (un - g.unp) * inv_dt;
     // (fma: the compiler's choice of the fused product differs between kernels)
     const R dux = fma(un, dnux, fma(uy, dyux, fma(ut, dtux, ux * dxux)));
-    const R duy = fma(un, dnuy, fma(uy, dyuy, fma(ut, dtuy, ux * dxuy)));
+    const R duy = fma(un, dnuy, add_rounded(uy, dyuy, fma(ut, dtuy, ux * dxuy)));
     const R dun = fma(un, dnun, fma(uy, dyun, fma(ut, dtun, ux * dxun)));
     const R dut = fma(un, dnut, fma(uy, dyut, fma(ut, dtut, ux * dxut)));  // = Dut - t un^2
     const R Dut = dut + t * un2;
@@ -773,20 +793,18 @@ VAH_HD int cell_sources(const Eos &eos, const R *Q, const CellGradT<R> &g, const
 
     // transverse / longitudinal split (SourceTerms.cpp:355-426)
     const R uT2 = ux * ux + uy * uy;
-    const R uTdxuT = ux * dxux + uy * dxuy;
+    const R uTdxuT = fused(ux, dxux, uy * dxuy);
     const R uTdyuT = ux * dyux + uy * dyuy;
     const R uTdnuT = ux * dnux + uy * dnuy;
-    const R uTduT = ut * (ux * dtux + uy * dtuy) + ux * uTdxuT + uy * uTdyuT + un * uTdnuT;
+    const R uTduT = fused(ut, ux * dtux + uy * dtuy, ux * uTdxuT) + uy * uTdyuT + un * uTdnuT;
     const R F = 1 + uT2;
     const R inv_F = quot(R(1.0), F);
     const R inv_sF = rsqrt_r(F);
     const R z0 = t * un * inv_sF;
     const R z3 = ut * inv_t * inv_sF;
     const R z02 = z0 * z0, z0z3 = z0 * z3, z32 = z3 * z3;
-    const R dz0 = (ut * un + t * dun - t * un * inv_F * uTduT) * inv_sF;
-    const R dz3 = (-ut2 * inv_t2 + dut * inv_t - ut * inv_t * inv_F * uTduT) * inv_sF;
-    const R Dz0 = dz0 + t * un * z3;
-    const R Dz3 = -t2 * (dz3 + (ut * z3 + un * z0) * inv_t);
+    const R Dz0 = fused(ut * un + t * dun - t * un * inv_F * uTduT, inv_sF, t * un * z3);
+    const R Dz3 = -t2 * fused(-ut2 * inv_t2 + dut * inv_t - ut * inv_t * inv_F * uTduT, inv_sF, (ut * z3 + un * z0) * inv_t);
     const R A = z02 * stt - 2 * t2 * z0z3 * stn + t2 * t2 * z32 * snn;
     const R B0 = z0 * stt - t2 * z3 * stn;
     const R B1 = z0 * stx - t2 * z3 * sxn;
@@ -847,7 +865,7 @@ VAH_HD int cell_sources(const Eos &eos, const R *Q, const CellGradT<R> &g, const
                          (2 * DP * uTdyuT * un * ut) * inv_F2;
     const R dnLtn = (DP * dnut * un) * inv_F + (DP * dnun * ut) * inv_F + (dnDP * un * ut) * inv_F -
                          (2 * DP * uTdnuT * un * ut) * inv_F2;
-    const R dnLnn = ((2 * DP * dnut * ut) * inv_F + (dnDP * ut2) * inv_F - (2 * DP * uTdnuT * ut2) * inv_F2) * inv_t2;
+    const R t2dnLnn = (2 * DP * dnut * ut) * inv_F + (dnDP * ut2) * inv_F - (2 * DP * uTdnuT * ut2) * inv_F2;
 
     const R zeta_zz = Rtilde * e - 3 * pl;
     const R zeta_zT = (Rtilde * e + pl) * R(0.5);
@@ -888,7 +906,8 @@ VAH_HD int cell_sources(const Eos &eos, const R *Q, const CellGradT<R> &g, const
     S[1] = -ttx * inv_t - dxptHat + dkvk * pitx;
     S[2] = -tty * inv_t - dyptHat + dkvk * pity;
     // SourceTerms.cpp:686: the reference adds dnLtn twice
-    S[3] = -3 * ttn * inv_t - dnptHat * inv_t2 + dkvk * (Ltn + pitn) + vx * dxLtn + vy * dyLtn + vn * (dnLtn + dnLtn) - dnLnn;
+    const R S3 = -3 * ttn * inv_t - dnptHat * inv_t2 + dkvk * (Ltn + pitn) + vx * dxLtn + vy * dyLtn + vn * (dnLtn + dnLtn);
+    S[3] = BULK ? fused(-t2dnLnn, inv_t2, S3) : S3 - rounded(t2dnLnn, inv_t2);
     int bad = isnan(S[4]) || isnan(S[0]);
 
     if (PIM) {
