@@ -163,7 +163,7 @@ __device__ __forceinline__ void copies_wait() { asm volatile("cp.async.wait_all;
 
 template <typename S>
 __device__ __forceinline__ Guess guess_at(const StageArgs<S> &a, int s) {
-    return newton_guess((double)ldg(a.uin[1] + s), (double)ldg(a.uin[2] + s));
+    return newton_guess((double)load(a.uin[1] + s), (double)load(a.uin[2] + s));
 }
 __device__ __forceinline__ double fma_(double x, double y, double z) { return fma(x, y, z); }
 __device__ __forceinline__ float fma_(float x, float y, float z) { return fmaf(x, y, z); }
@@ -200,8 +200,8 @@ __device__ __forceinline__ void set_weights(double vR, double vL, S &wR, S &wL) 
 // One state's velocity as the cell at s evaluates it, by the iteration.
 template <typename S>
 __device__ __forceinline__ int velocity_at(const StageArgs<S> &a, const InvIn &q, int dir, int s, double *v) {
-    const int st = face_velocity_iterated<sizeof(S) == 4>(a.t_src, q, dir, (double)ldg(a.ein + s),
-                                                          (double)ldg(a.uin[1] + s), (double)ldg(a.uin[2] + s), v);
+    const int st = face_velocity_iterated<sizeof(S) == 4>(a.t_src, q, dir, (double)load(a.ein + s),
+                                                          (double)load(a.uin[1] + s), (double)load(a.uin[2] + s), v);
     return (st != 0) + (st == 2 ? 256 : 0);
 }
 
@@ -286,7 +286,7 @@ __device__ __forceinline__ void flux_x(const StageArgs<S> &a, const Pointers &hp
 #pragma unroll
     for (int n = 0; n < N; ++n) {
         const S *q = hp.q(n, half) + s;
-        const S qm = ldg(q - 1), q0 = ldg(q), qp = ldg(q + 1);
+        const S qm = load(q - 1), q0 = load(q), qp = load(q + 1);
         const S m = limited4(q0 - qm, qp - q0, qp - qm);
         qL[n] = fma_(S(0.25), m, q0);
         qR[n] = __shfl_down_sync(kFullWarp, fma_(S(-0.25), m, q0), 1, W);
@@ -329,14 +329,14 @@ __device__ __forceinline__ void flux_march(const StageArgs<S> &a, const Pointers
 #pragma unroll
     for (int n = 0; n < N; ++n) {
         const S *q = hp.q(n, half) + s;
-        const S qm = ldg(q - st), q0 = ldg(q), qp = ldg(q + st);
+        const S qm = load(q - st), q0 = load(q), qp = load(q + st);
         copy_async(Q + (2 * N + n) * 32, q + 2 * st);
         QL[n * 32] = fma_(S(0.25), limited4(q0 - qm, qp - q0, qp - qm), q0);
         Q[n * 32] = q0;
         Q[(N + n) * 32] = qp;
     }
     Guess gl = guess_at(a, s);
-    S un1 = ldg(a.uin[1] + s + st), un2 = ldg(a.uin[2] + s + st);  // the right cell's velocity
+    S un1 = load(a.uin[1] + s + st), un2 = load(a.uin[2] + s + st);  // the right cell's velocity
     S *Q0 = Q, *Q1 = Q + N * 32, *Q2 = Q1 + N * 32;  // q of the left cell, the right one and the next
 #pragma unroll 1
     for (int m = m0 - 1; m < m1; ++m, s += st) {  // the face at +1/2 of cell m
@@ -358,8 +358,8 @@ __device__ __forceinline__ void flux_march(const StageArgs<S> &a, const Pointers
         if (m + 1 < m1) {
 #pragma unroll
             for (int n = 0; n < N; ++n) copy_async(Q2 + n * 32, hp.q(n, half) + s + 3 * st);
-            un1 = ldg(a.uin[1] + s + 2 * st);
-            un2 = ldg(a.uin[2] + s + 2 * st);
+            un1 = load(a.uin[1] + s + 2 * st);
+            un2 = load(a.uin[2] + s + 2 * st);
         }
         const bool mine = m >= m0;  // cell m belongs to this segment
         const bool need_l = EXACT ? mine : true, need_r = EXACT && m + 1 < m1;

@@ -174,6 +174,7 @@ VAH_HD uint32_t float_bits(float x) {
 #endif
 }
 
+// Read-only loads, of what no launch writes: the EoS table and the exception list.
 template <typename T>
 VAH_HD T ldg(const T *p) {
 #ifdef __CUDA_ARCH__
@@ -182,6 +183,13 @@ VAH_HD T ldg(const T *p) {
     return *p;
 #endif
 }
+
+// Loads of the state and of stage scratch: coherent. The blocks of a dependent
+// launch are resident while the launch before still writes what they read
+// after its end (after_previous_launch), and stage 2 reads q^n where it writes
+// q^{n+1}, so none of it is constant for a launch's lifetime, as __ldg asks.
+template <typename T>
+VAH_HD T load(const T *p) { return *p; }
 
 // ------------------------------------------------------------------- EoS --
 // Equation of state and zeta/s, passed by value into kernels.

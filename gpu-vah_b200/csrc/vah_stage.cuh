@@ -87,7 +87,7 @@ VAH_HD void finish_args(StageArgs<S> &a) {
 
 template <typename S, typename I>
 VAH_HD double ld(const S *p, I i) {
-    return (double)ldg(p + i);
+    return (double)load(p + i);
 }
 
 // Face values are read once, by the cell launch: loaded with the streaming

@@ -253,13 +253,13 @@ VAH_HD void cell_compute_f32(const StageArgs<float> &a, int i, int j, int k) {
     const float c[3] = {(float)a.c_h[0], (float)a.c_h[1], (float)a.c_h[2]};
 #pragma unroll
     for (int n = 0; n < NQ; ++n) {
-        flux[n] = c[0] * ldg(a.D[0][n] + s);
+        flux[n] = c[0] * load(a.D[0][n] + s);
 #pragma unroll
-        for (int d = 1; d < (IS3D ? 3 : 2); ++d) flux[n] = fmaf(c[d], ldg(a.D[d][n] + s), flux[n]);
+        for (int d = 1; d < (IS3D ? 3 : 2); ++d) flux[n] = fmaf(c[d], load(a.D[d][n] + s), flux[n]);
     }
     struct Fields {
         const float *const *f;
-        VAH_HD float operator()(int n, long long at) const { return ldg(f[n] + at); }
+        VAH_HD float operator()(int n, long long at) const { return load(f[n] + at); }
     };
     TilePrims pr;
     pr.E = a.ein;
