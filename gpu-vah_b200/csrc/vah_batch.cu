@@ -10,9 +10,12 @@
 // device arrays, so a whole RK2 step -- flux and cell launches of both stages
 // plus the clock advance -- is captured once as a CUDA graph and replayed.
 // The graph is re-captured only when events are added or removed.
-// The flux differences of a stage are scratch that events share: where one
-// scratch of kScratchBytes does not hold every event's, the events are stepped
-// in groups that it holds.
+// The flux differences of a stage are scratch that events share. Where it does
+// not hold every event's, the events are stepped in groups that it holds, and an
+// event that it does not hold in slabs of planes. It takes what the events leave
+// of the batch's capacity, up to kScratchBytes, and kScratchBeyond where they leave
+// less. One plane's share, without which an event cannot be stepped, is there from
+// admission on, so no step fails for want of it.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -40,7 +43,6 @@ struct SlotDesc {
     long long plane;
     double dx, dy, dz, dt, etabar;
     S *q[16], *qS[16], *ep[2][2], *uA[4], *uB[4], *uS[4];
-    S *D[3][16];  // flux differences per axis, in the shared scratch
     unsigned char *fallback;  // per ghosted cell: 1 where the latest cell inversion fell back
     unsigned char *hot;       // per ghosted cell: 1 while e > e_freeze (freeze-out crossings)
     double e_freeze;
@@ -55,28 +57,38 @@ struct SlotClock {
     long long steps;
 };
 
+// The planes [k0, k1) of an event that one group steps, and where the scratch
+// holds their differences: field n of axis d from D + (d N_q + n) stride.
+struct Slab {
+    int slot, k0, k1;
+    long long stride;
+    void *D;
+};
+
 // One block's piece of work: four strips (from strip i0) of flux_x (kind 0) or
 // of flux_march along y or eta (kind 1, 2) over the cells [r0, r1) along it; or
-// the 128 interior cells from i0 (cell lists).
+// the interior cells [i0, min(i0 + 128, r1)) of the event (cell lists).
 struct WorkItem {
-    int slot, kind, i0, r0, r1;
+    int slot, slab, kind, i0, r0, r1;
 };
 constexpr int kCellItem = kTX * kTY;
 
 // The work-lists: fluxes, 2+1D cells, 3+1D cells.
 enum { K_FLUX = 0, K_C2 = 1, K_C3 = 2, K_NUM = 3 };
 
-// StageArgs of one slot and stage (the buffer roles of vah_rk2_step), filled by
+// StageArgs of one slab and stage (the buffer roles of vah_rk2_step), filled by
 // 96 threads together (tid 0 to 95).
 template <typename S>
-__device__ void make_args(StageArgs<S> &a, const SlotDesc<S> &d, const SlotClock &c, int stage, const Eos &eos, int tid) {
+__device__ void make_args(StageArgs<S> &a, const SlotDesc<S> &d, const Slab &b, int nq, const SlotClock &c, int stage,
+                          const Eos &eos, int tid) {
     const int warp = tid >> 5, n = tid & 31;
     if (warp == 0) {
         if (n < 16) {
             a.qin[n] = stage == 1 ? d.q[n] : d.qS[n];
             a.qout[n] = stage == 1 ? d.qS[n] : d.q[n];
             a.qavg[n] = d.q[n];
-            for (int k = 0; k < 3; ++k) a.D[k][n] = d.D[k][n];
+            for (int k = 0; k < 3; ++k)  // indexed by ghosted cells: plane k0 is the scratch's first
+                a.D[k][n] = n < nq && (k < 2 || d.nz > 1) ? (S *)b.D + (k * nq + n) * b.stride - (b.k0 + 2) * d.plane : nullptr;
         } else if (n < 20) {
             const int m = n - 16;
             S *u = c.parity ? d.uB[m] : d.uA[m], *up = c.parity ? d.uA[m] : d.uB[m];
@@ -91,8 +103,8 @@ __device__ void make_args(StageArgs<S> &a, const SlotDesc<S> &d, const SlotClock
         a.nx = d.nx;
         a.ny = d.ny;
         a.nz = d.nz;
-        a.k0 = 0;
-        a.k1 = d.nz;
+        a.k0 = b.k0;
+        a.k1 = b.k1;
         a.ncx = d.ncx;
         a.ncy = d.ncy;
         a.plane = d.plane;
@@ -121,13 +133,14 @@ __device__ void make_args(StageArgs<S> &a, const SlotDesc<S> &d, const SlotClock
     }
 }
 
-// Both stages' arguments of every active slot, once per step (block: a slot,
+// Both stages' arguments of every slab, once per step (block: a slab,
 // threadIdx.y: the stage): the stage launches' blocks copy theirs from there.
 template <typename S>
-__global__ void args_kernel(const SlotDesc<S> *__restrict__ descs, const SlotClock *__restrict__ clk, const Eos eos,
-                            StageArgs<S> *args) {
-    const int slot = blockIdx.x;
-    if (clk[slot].active) make_args(args[2 * slot + threadIdx.y], descs[slot], clk[slot], threadIdx.y + 1, eos, threadIdx.x);
+__global__ void args_kernel(const SlotDesc<S> *__restrict__ descs, const Slab *__restrict__ slabs, int nq,
+                            const SlotClock *__restrict__ clk, const Eos eos, StageArgs<S> *args) {
+    const Slab b = slabs[blockIdx.x];
+    if (clk[b.slot].active)
+        make_args(args[2 * blockIdx.x + threadIdx.y], descs[b.slot], b, nq, clk[b.slot], threadIdx.y + 1, eos, threadIdx.x);
 }
 
 // A block's copy of its item's arguments into shared memory; a barrier before use.
@@ -145,16 +158,16 @@ __global__ void __launch_bounds__(kTX *kTY, kFluxMinb<S>)
     __shared__ StageArgs<S> sa;
     __shared__ TablePointers<S> tab;
     const WorkItem it = work[blockIdx.x];
-    const StageArgs<S> *from = args + 2 * it.slot + stage - 1;
+    const StageArgs<S> *from = args + 2 * it.slab + stage - 1;
     const int warp = threadIdx.x / 32, strip = it.i0 + warp;
     copy_args(sa, from, threadIdx.x);
     set_table_pointers<PHYS>(tab, *from, threadIdx.x);
     __syncthreads();
     S *sm = (S *)march_sm + warp * kMarchValues<S, PHYS>;
     if (it.kind == 0) {
-        if (strip < flux_x_strips<S>(sa.nx, sa.ny, sa.nz)) flux_x<PHYS, EXACT>(sa, tab, strip);
+        if (strip < flux_x_strips<S>(sa.nx, sa.ny, sa.k1 - sa.k0)) flux_x<PHYS, EXACT>(sa, tab, strip);
     } else if (it.kind == 1) {
-        if (strip < march_strips<S>(sa.nx * sa.nz)) flux_march<PHYS, 1, EXACT>(sa, tab, strip, it.r0, it.r1, sm);
+        if (strip < march_strips<S>(sa.nx * (sa.k1 - sa.k0))) flux_march<PHYS, 1, EXACT>(sa, tab, strip, it.r0, it.r1, sm);
     } else {
         if (strip < march_strips<S>(sa.nx * sa.ny)) flux_march<PHYS, 2, EXACT>(sa, tab, strip, it.r0, it.r1, sm);
     }
@@ -165,10 +178,10 @@ __global__ void __launch_bounds__(kTX *kTY, kCellMinb<S, IS3D> / 2)
     batch_cell_kernel(const StageArgs<S> *__restrict__ args, const WorkItem *__restrict__ work, int stage) {
     __shared__ StageArgs<S> sa;
     const WorkItem it = work[blockIdx.x];
-    copy_args(sa, args + 2 * it.slot + stage - 1, threadIdx.x);
+    copy_args(sa, args + 2 * it.slab + stage - 1, threadIdx.x);
     __syncthreads();
     const int c = it.i0 + threadIdx.x;
-    if (c >= sa.nx * sa.ny * sa.nz) return;
+    if (c >= it.r1) return;
     const int r = c / sa.nx, i = c - r * sa.nx, k = r / sa.ny, j = r - k * sa.ny;
     if constexpr (sizeof(S) == 4) cell_compute_f32<PHYS, IS3D>(sa, i + 2, j + 2, k + 2);
     else cell_compute<S, PHYS, IS3D, true>(sa, i + 2, j + 2, k + 2);
@@ -214,7 +227,7 @@ __global__ void max_e_kernel(const SlotDesc<S> *__restrict__ descs, const WorkIt
         const SlotDesc<S> &d = descs[it.slot];
         const int cell = it.i0 + threadIdx.y * kTX + threadIdx.x;
         double v = 0.0;
-        if (cell < d.nx * d.ny * d.nz) {
+        if (cell < it.r1) {
             const int r = cell / d.nx, i = cell - r * d.nx, j = r % d.ny, k = r / d.ny;
             const long long s = (i + 2) + (long long)d.ncx * (j + 2) + d.plane * (k + 2);
             v = (double)d.ep[cur_ep][0][s];
@@ -244,7 +257,7 @@ __global__ void observables_kernel(const SlotDesc<S> *__restrict__ descs, const 
         const SlotClock c = clk[it.slot];
         const int cell = it.i0 + tid;
         double acc[5] = {0, 0, 0, 0, 0};
-        const bool in = cell < d.nx * d.ny * d.nz;
+        const bool in = cell < it.r1;
         const int r = in ? cell / d.nx : 0, i = in ? cell - r * d.nx : 0, j = r % d.ny, k = r / d.ny;
         const long long s = (i + 2) + (long long)d.ncx * (j + 2) + d.plane * (k + 2);
         if (in && !d.fallback[s]) {  // converged cells only
@@ -324,11 +337,13 @@ struct vah_batch {
     double *d_fstage;  // staging of the field reads ...
     size_t fstage;     // ... of this many values
     WorkItem *d_work[vah::K_NUM];
-    void *d_args;        // StageArgs<S>[cap_args]: both stages' arguments by slot
+    void *d_args;        // StageArgs<S>[cap_args]: both stages' arguments by slab
     size_t cap_args;     // in StageArgs
-    int nslots;          // slots up to the last one in use
-    char *d_scratch;     // the flux differences of one group of events
+    char *d_scratch;     // the flux differences of one group of slabs
     size_t cap_scratch;
+    vah::Slab *d_slabs;
+    size_t cap_slabs;
+    int nslabs;
     struct Group {
         int first[vah::K_NUM], count[vah::K_NUM];  // its runs of the work-lists
     };
@@ -367,16 +382,27 @@ int nq_of(int physics) { return physics == VAH_IDEAL ? 5 : (physics == VAH_PIMUN
 // 4 uS; then one byte per cell of fallback flags and one of freeze-out state.
 constexpr int kArraysPerEvent = 48;
 
-// The scratch that a group's flux differences share; an event that needs more
-// is a group of its own. With 4 GB a batch of 256 2+1D events (sides 81 to
-// 201, 5.84 M cells) is one group: as two, its FP64 step had twice the launches
-// and their tails (6.10 against 5.98 ms).
+// The most that the scratch of a group's flux differences takes. With 4 GB a
+// batch of 256 2+1D events (sides 81 to 201, 5.84 M cells) is one group: as two,
+// its FP64 step had twice the launches and their tails (6.10 against 5.98 ms).
 constexpr size_t kScratchBytes = (size_t)4 << 30;
+// What it may take beyond the capacity where the events leave less: slabs of
+// this size (0.7 M FP64 cells) still fill the GPU, those of one plane do not.
+constexpr size_t kScratchBeyond = (size_t)256 << 20;
 
 size_t event_bytes(const vah_batch *b, const vah_lattice *lat) {
     const size_t ncell = (size_t)(lat->nx + 4) * (lat->ny + 4) * (lat->nz + 4);
     const size_t per = (ncell * b->elem + 255) / 256 * 256;
     return per * kArraysPerEvent + 2 * ((ncell + 255) / 256 * 256) + 256;
+}
+
+// The flux differences of `planes` planes of an event: bytes of one field (which
+// interior planes alone have), and of every field and axis.
+size_t diff_field_bytes(const vah_batch *b, const vah_lattice &l, int planes) {
+    return ((size_t)(l.nx + 4) * (l.ny + 4) * planes * b->elem + 255) / 256 * 256;
+}
+size_t diff_bytes(const vah_batch *b, const vah_lattice &l, int planes) {
+    return diff_field_bytes(b, l, planes) * (l.nz > 1 ? 3 : 2) * b->nq;
 }
 
 vah::Eos batch_eos(const vah_batch *b) {
@@ -467,90 +493,137 @@ int grow(vah_batch *b, T *&p, size_t &cap, size_t n) {  // device memory for n v
     return VAH_OK;
 }
 
+// Scratch of `want` bytes where the device has them, else of the half and so on
+// down to `least`; contents lost. What it frees stays in the batch's pool, so
+// that the old size can be had again.
+int set_scratch(vah_batch *b, size_t want, size_t least) {
+    if (b->d_scratch) VAH_TRY(cudaFreeAsync(b->d_scratch, b->stream));
+    b->d_scratch = nullptr;
+    b->cap_scratch = 0;
+    b->dirty = true;
+    for (;; want = std::max(least, want / 2)) {
+        const cudaError_t e = cudaMallocFromPoolAsync((void **)&b->d_scratch, want, b->pool, b->stream);
+        if (e == cudaSuccess) break;
+        cudaGetLastError();  // an allocation that fails leaves nothing else behind
+        b->d_scratch = nullptr;
+        if (want <= least) return cuda_status(e);
+    }
+    b->cap_scratch = want;
+    return VAH_OK;
+}
+
+// The scratch of the batch's events (and of one more, or null): all their
+// differences at once; the least that steps them, a plane of each by itself;
+// and the most it may take if they leave `free` bytes of the capacity.
+struct ScratchBounds {
+    size_t all, least, most;
+};
+ScratchBounds scratch_bounds(const vah_batch *b, const vah_lattice *more, size_t free) {
+    ScratchBounds r{0, 0, 0};
+    auto add = [&](const vah_lattice &l) {
+        r.all += diff_bytes(b, l, l.nz);
+        r.least = std::max(r.least, diff_bytes(b, l, 1));
+    };
+    for (const vah_batch::Slot &sl : b->slots)
+        if (sl.used) add(sl.lat);
+    if (more) add(*more);
+    r.most = std::max(std::max(r.least, kScratchBeyond), std::min(kScratchBytes, free));
+    return r;
+}
+
 // The work-lists, groups and scratch of the admitted events.
 template <typename S>
 int rebuild_work(vah_batch *b) {
     std::vector<WorkItem> lists[vah::K_NUM];
     std::vector<int> order;  // largest event first: its items start first, small ones fill the tail
-    b->nslots = 0;
     for (int s = 0; s < (int)b->slots.size(); ++s)
-        if (b->slots[s].used) {
-            order.push_back(s);
-            b->nslots = s + 1;
-        }
+        if (b->slots[s].used) order.push_back(s);
     auto cells = [&](int s) {
         const vah_lattice &l = b->slots[s].lat;
         return (long long)l.nx * l.ny * l.nz;
     };
     std::stable_sort(order.begin(), order.end(), [&](int x, int y) { return cells(x) > cells(y); });
-    // groups of events whose differences the scratch holds
-    auto per_field = [&](int s) {  // bytes of one field of differences, which interior planes alone have
-        const vah_lattice &l = b->slots[s].lat;
-        return ((size_t)(l.nx + 4) * (l.ny + 4) * l.nz * sizeof(S) + 255) / 256 * 256;
-    };
-    auto scratch_of = [&](int s) { return per_field(s) * (b->slots[s].lat.nz > 1 ? 3 : 2) * b->nq; };
-    std::vector<std::vector<int>> members;
-    size_t held = 0, need = 0;
-    for (int s : order) {
-        if (members.empty() || held + scratch_of(s) > kScratchBytes) {
-            members.emplace_back();
-            held = 0;
-        }
-        members.back().push_back(s);
-        held += scratch_of(s);
-        need = std::max(need, held);
-    }
-    int rc = grow(b, b->d_scratch, b->cap_scratch, need);
+    // the scratch grows to what the events can use of the room they leave (at
+    // least by half, so that a set that grows event by event seldom re-allocates)
+    const ScratchBounds sb = scratch_bounds(b, nullptr, b->capacity - b->used);
+    int rc = VAH_OK;
+    if (std::min(sb.all, sb.most) > b->cap_scratch)
+        rc = set_scratch(b, std::min(std::max(sb.all, b->cap_scratch + b->cap_scratch / 2), sb.most), sb.least);
     if (rc != VAH_OK) return rc;
+    // slabs that the scratch holds (an event, where it does), and groups of them
+    std::vector<vah::Slab> slabs;
+    std::vector<std::vector<int>> members;
+    size_t held = 0;
+    for (int s : order) {
+        const vah_lattice &l = b->slots[s].lat;
+        int planes = l.nz;
+        while (planes > 1 && diff_bytes(b, l, planes) > b->cap_scratch)
+            planes = std::max(1, std::min(planes - 1, (int)(b->cap_scratch / diff_bytes(b, l, 1))));
+        const int n = (l.nz + planes - 1) / planes;
+        for (int m = 0; m < n; ++m) {
+            const int k0 = (int)((long long)l.nz * m / n), k1 = (int)((long long)l.nz * (m + 1) / n);
+            const size_t field = diff_field_bytes(b, l, k1 - k0), bytes = diff_bytes(b, l, k1 - k0);
+            if (members.empty() || held + bytes > b->cap_scratch) {
+                members.emplace_back();
+                held = 0;
+            }
+            members.back().push_back((int)slabs.size());
+            slabs.push_back({s, k0, k1, (long long)(field / sizeof(S)), b->d_scratch + held});
+            held += bytes;
+        }
+    }
     b->groups.clear();
     for (const std::vector<int> &group : members) {
         vah_batch::Group g;
         for (int k = 0; k < vah::K_NUM; ++k) g.first[k] = (int)lists[k].size();
         int seg[3] = {};  // march segments along y and eta, from the whole group's warps
         for (int dir = 1; dir < 3; ++dir) {
-            auto along = [&](const vah_lattice &l) { return dir == 1 ? l.ny : l.nz; };
+            auto along = [&](const vah::Slab &p) { return dir == 1 ? b->slots[p.slot].lat.ny : p.k1 - p.k0; };
             int longest = 1;
-            for (int s : group) longest = std::max(longest, along(b->slots[s].lat));
+            for (int p : group) longest = std::max(longest, along(slabs[p]));
             seg[dir] = vah::march_segment(longest, vah::kFluxMinb<S>, [&](int len) {
                 long long w = 0;
-                for (int s : group) {
-                    const vah_lattice &l = b->slots[s].lat;
+                for (int p : group) {
+                    const vah_lattice &l = b->slots[slabs[p].slot].lat;
                     if (dir == 2 && l.nz == 1) continue;
-                    const long long strips = vah::march_strips<S>(dir == 1 ? l.nx * l.nz : l.nx * l.ny);
-                    w += (strips + 3) / 4 * 4 * ((along(l) + len - 1) / len);
+                    const long long strips = vah::march_strips<S>(l.nx * (dir == 1 ? slabs[p].k1 - slabs[p].k0 : l.ny));
+                    w += (strips + 3) / 4 * 4 * ((along(slabs[p]) + len - 1) / len);
                 }
                 return w;
             });
         }
         // the marches first (long), then the x strips, which fill the tail
         for (int kind : {2, 1, 0})
-            for (int s : group) {
-                const vah_lattice &l = b->slots[s].lat;
+            for (int p : group) {
+                const vah::Slab &sl = slabs[p];
+                const vah_lattice &l = b->slots[sl.slot].lat;
                 if (kind == 2 && l.nz == 1) continue;
-                const int strips = kind == 0 ? vah::flux_x_strips<S>(l.nx, l.ny, l.nz)
-                                             : vah::march_strips<S>(kind == 1 ? l.nx * l.nz : l.nx * l.ny);
-                const int n = kind == 0 ? 1 : (kind == 1 ? l.ny : l.nz), len = kind == 0 ? 1 : seg[kind];
-                for (int r0 = 0; r0 < n; r0 += len)
+                const int nk = sl.k1 - sl.k0;
+                const int strips = kind == 0 ? vah::flux_x_strips<S>(l.nx, l.ny, nk)
+                                             : vah::march_strips<S>(l.nx * (kind == 1 ? nk : l.ny));
+                const int at = kind == 2 ? sl.k0 : 0, n = kind == 0 ? 1 : (kind == 1 ? l.ny : sl.k1);
+                const int len = kind == 0 ? 1 : seg[kind];
+                for (int r0 = at; r0 < n; r0 += len)
                     for (int i0 = 0; i0 < strips; i0 += 4)
-                        lists[vah::K_FLUX].push_back({s, kind, i0, r0, std::min(r0 + len, n)});
+                        lists[vah::K_FLUX].push_back({sl.slot, p, kind, i0, r0, std::min(r0 + len, n)});
             }
-        char *at = b->d_scratch;
-        for (int s : group) {
-            const vah_lattice &l = b->slots[s].lat;
-            for (int c0 = 0; c0 < cells(s); c0 += vah::kCellItem)
-                lists[l.nz > 1 ? vah::K_C3 : vah::K_C2].push_back({s, 0, c0, 0, 0});
-            SlotDesc<S> &d = *desc_host<S>(b, s);
-            for (int k = 0; k < (l.nz > 1 ? 3 : 2); ++k)
-                for (int n = 0; n < b->nq; ++n, at += per_field(s)) d.D[k][n] = (S *)at - 2 * d.plane;
+        for (int p : group) {
+            const vah::Slab &sl = slabs[p];
+            const vah_lattice &l = b->slots[sl.slot].lat;
+            const int plane = l.nx * l.ny, end = plane * sl.k1;
+            for (int c0 = plane * sl.k0; c0 < end; c0 += vah::kCellItem)
+                lists[l.nz > 1 ? vah::K_C3 : vah::K_C2].push_back({sl.slot, p, 0, c0, 0, end});
         }
         for (int k = 0; k < vah::K_NUM; ++k) g.count[k] = (int)lists[k].size() - g.first[k];
         b->groups.push_back(g);
     }
-    if (b->nslots)
-        VAH_TRY(cudaMemcpyAsync(b->d_desc, b->desc_host.data(), sizeof(SlotDesc<S>) * b->nslots, cudaMemcpyHostToDevice,
+    b->nslabs = (int)slabs.size();
+    if ((rc = grow(b, b->d_slabs, b->cap_slabs, slabs.size())) != VAH_OK) return rc;
+    if (b->nslabs)
+        VAH_TRY(cudaMemcpyAsync(b->d_slabs, slabs.data(), sizeof(vah::Slab) * slabs.size(), cudaMemcpyHostToDevice,
                                 b->stream));
     auto *args = (vah::StageArgs<S> *)b->d_args;
-    rc = grow(b, args, b->cap_args, 2 * (size_t)b->nslots);
+    rc = grow(b, args, b->cap_args, 2 * slabs.size());
     b->d_args = args;
     if (rc != VAH_OK) return rc;
     for (int k = 0; k < vah::K_NUM; ++k) {
@@ -606,15 +679,15 @@ cudaError_t launch_list_any(vah_batch *b, const vah_batch::Group &g, int list, i
 }
 
 int launch_args(vah_batch *b) {
-    if (b->nslots == 0) return VAH_OK;
+    if (b->nslabs == 0) return VAH_OK;
     const dim3 block(96, 2);
     const vah::Eos eos = batch_eos(b);
     if (b->elem == sizeof(float))
-        vah::args_kernel<float><<<b->nslots, block, 0, b->stream>>>((const SlotDesc<float> *)b->d_desc, b->d_clk, eos,
-                                                                    (vah::StageArgs<float> *)b->d_args);
+        vah::args_kernel<float><<<b->nslabs, block, 0, b->stream>>>((const SlotDesc<float> *)b->d_desc, b->d_slabs, b->nq,
+                                                                    b->d_clk, eos, (vah::StageArgs<float> *)b->d_args);
     else
-        vah::args_kernel<double><<<b->nslots, block, 0, b->stream>>>((const SlotDesc<double> *)b->d_desc, b->d_clk, eos,
-                                                                     (vah::StageArgs<double> *)b->d_args);
+        vah::args_kernel<double><<<b->nslabs, block, 0, b->stream>>>((const SlotDesc<double> *)b->d_desc, b->d_slabs, b->nq,
+                                                                     b->d_clk, eos, (vah::StageArgs<double> *)b->d_args);
     VAH_TRY(cudaGetLastError());
     return VAH_OK;
 }
@@ -847,6 +920,7 @@ extern "C" int vah_batch_destroy(vah_batch *b) {
     if (b->d_partial) cudaFreeAsync(b->d_partial, b->stream);
     if (b->d_args) cudaFreeAsync(b->d_args, b->stream);
     if (b->d_scratch) cudaFreeAsync(b->d_scratch, b->stream);
+    if (b->d_slabs) cudaFreeAsync(b->d_slabs, b->stream);
     cudaStreamSynchronize(b->stream);
     cudaMemPoolDestroy(b->pool);
     cudaFree(b->d_desc);
@@ -900,8 +974,24 @@ int add_slot(vah_batch *b, const vah_lattice *lat, const vah_hydro *hydro, doubl
         b->d_fstage = wider;
         b->fstage = (size_t)lat->nx + 4;
     }
+    // the scratch: never less than the event needs, nor more than the room that it leaves
+    const ScratchBounds sb = scratch_bounds(b, lat, b->capacity - b->used - bytes);
+    int rc = VAH_OK;
+    if (b->cap_scratch < sb.least || b->cap_scratch > sb.most)
+        rc = set_scratch(b, std::min(std::max(sb.least, kScratchBeyond), sb.all), sb.least);
+    if (rc != VAH_OK) return rc;
     vah_batch::Slot &sl = b->slots[slot];
-    VAH_TRY(cudaMallocFromPoolAsync(&sl.mem, bytes, b->pool, b->stream));
+    cudaError_t e = cudaMallocFromPoolAsync(&sl.mem, bytes, b->pool, b->stream);
+    if (e == cudaErrorMemoryAllocation && b->cap_scratch > sb.least) {  // the scratch makes way
+        cudaGetLastError();
+        if ((rc = set_scratch(b, sb.least, sb.least)) != VAH_OK) return rc;
+        e = cudaMallocFromPoolAsync(&sl.mem, bytes, b->pool, b->stream);
+    }
+    if (e != cudaSuccess) {
+        cudaGetLastError();  // else the next launch's check would find it
+        sl.mem = nullptr;
+        return cuda_status(e);
+    }
     VAH_TRY(cudaMemsetAsync(sl.mem, 0, bytes, b->stream));
     sl.used = true;
     sl.lat = *lat;
@@ -910,7 +1000,7 @@ int add_slot(vah_batch *b, const vah_lattice *lat, const vah_hydro *hydro, doubl
     sl.bytes = bytes;
     sl.admitted = b->steps;
     b->used += bytes;
-    int rc = b->elem == sizeof(float) ? fill_slot<float>(b, slot) : fill_slot<double>(b, slot);
+    rc = b->elem == sizeof(float) ? fill_slot<float>(b, slot) : fill_slot<double>(b, slot);
     if (rc == VAH_OK)
         rc = b->elem == sizeof(float) ? init_slot<float>(b, slot, hydro->t0, e_interior, glauber, pl_mode)
                                       : init_slot<double>(b, slot, hydro->t0, e_interior, glauber, pl_mode);

@@ -164,7 +164,8 @@ extern "C" int vah_serve_run(const vah_serve_config *cfg, vah_serve_result *res,
             } else {
                 a = vah_batch_add(batch, &r.lat, &hy, cfg->dt, r.e.data(), VAH_PL_ISOTROPIC, &slot);
             }
-            if (a == VAH_ERR_FULL) {
+            // no room, or no device memory although the capacity has room: wait for a retirement
+            if (a == VAH_ERR_FULL || (a == VAH_ERR_NOMEM && !live.empty())) {
                 refused = live.empty() ? false : true;
                 if (live.empty()) {  // larger than the whole batch: reject the request
                     ++rejected;

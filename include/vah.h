@@ -289,12 +289,16 @@ int vah_rk2_step_host(vah_event *ev, double t, double dt, double *const *fields)
  * take the items of a work-list over all events, and one RK2 step of the whole
  * batch (flux and cell launches of both stages and the per-event clock
  * advance) is replayed from a CUDA graph that is re-captured only when events
- * are added or removed. The flux differences of a stage are scratch that the
- * events share (up to 4 GB, or the largest event's; larger batches step in
- * groups), allocated at the first step and not part of an event's footprint. Every event keeps its
- * own time and dt; all share the batch's physics options (VAH_FLUX_PER_CELL
- * or VAH_FLUX_SHARED). Admission is by device footprint: vah_batch_add
- * returns VAH_ERR_FULL when the event would exceed capacity_bytes. */
+ * are added or removed. Every event keeps its own time and dt; all share the
+ * batch's physics options (VAH_FLUX_PER_CELL or VAH_FLUX_SHARED). Admission is
+ * by device footprint: vah_batch_add returns VAH_ERR_FULL when the event would
+ * exceed capacity_bytes. The flux differences of a stage are scratch that the
+ * events share: it takes what the events leave of capacity_bytes, up to 4 GB,
+ * and may take 256 MB (or the differences of one plane of the largest event,
+ * if more) beyond it where they leave less. Events that it does not hold
+ * together are stepped in groups, one that it does not hold by itself in slabs
+ * of planes, with the same results; what a slab of one plane takes is there
+ * from admission on, so no step fails for want of scratch. */
 typedef struct vah_batch vah_batch;
 
 typedef struct vah_event_info {
