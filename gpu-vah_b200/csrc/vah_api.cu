@@ -237,6 +237,35 @@ extern "C" int vah_math_check(int device, double lo, double hi, int n, double *m
 
 namespace {
 
+__global__ void math_values_kernel(int op, const double *a, const double *b, double *out, int n) {
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const double x = a[i], y = b[i];
+        out[i] = op == VAH_MATH_QUOTIENT ? vah::quotient_d(x, y)
+                                         : (op == VAH_MATH_RECIPROCAL ? vah::recip_d(y) : vah::sqrt_estimate(x));
+    }
+}
+
+}  // namespace
+
+extern "C" int vah_math_values(int device, int op, const double *a, const double *b, int n, double *out) {
+    if (op < VAH_MATH_QUOTIENT || op > VAH_MATH_SQRT_ESTIMATE || !a || !b || !out || n < 1) return VAH_ERR_ARG;
+    VAH_TRY(cudaSetDevice(device));
+    double *d = nullptr;
+    const size_t bytes = (size_t)n * sizeof(double);
+    VAH_TRY(cudaMalloc((void **)&d, 3 * bytes));
+    cudaError_t e = cudaMemcpy(d, a, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) e = cudaMemcpy(d + n, b, bytes, cudaMemcpyHostToDevice);
+    if (e == cudaSuccess) {
+        math_values_kernel<<<148 * 4, 256>>>(op, d, d + n, d + 2 * (size_t)n, n);
+        e = cudaGetLastError();
+    }
+    if (e == cudaSuccess) e = cudaMemcpy(out, d + 2 * (size_t)n, bytes, cudaMemcpyDeviceToHost);
+    cudaFree(d);
+    return cuda_status(e);
+}
+
+namespace {
+
 // FP64 FMA throughput: every thread runs 8 independent chains of `iters`
 // dependent FMAs (enough independent work to hide the FMA latency at full
 // occupancy); the result is folded into one store so the chains stay live.

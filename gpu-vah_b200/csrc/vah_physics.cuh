@@ -92,11 +92,12 @@ VAH_HD float rsqrt_r(float x) {
 #endif
 }
 
-// 1/d and f/d to rounding level for d of ordinary magnitude. On the device: the
-// hardware reciprocal estimate (about 2^-20) refined by two Newton-Raphson
-// steps y += y (1 - d y), and for the quotient one residual correction
-// q += y (f - d q); outside |d| in [2^-1000, 2^1001), where the estimate
-// flushes or overflows, the IEEE quotient. On the host: IEEE.
+// 1/d and f/d to an ulp. On the device: the hardware reciprocal estimate (about
+// 2^-20) refined by two Newton-Raphson steps y += y (1 - d y), and for the
+// quotient one residual correction q += y (f - d q); outside |d| in [2^-1000,
+// 2^1001), where the estimate flushes or overflows, the IEEE quotient. The
+// reciprocal has no such test: its caller keeps the results of |d| in [1e-100,
+// 1e101] only. On the host: IEEE. (vah_math_values measures them.)
 VAH_HD double recip_d(double d) {
 #ifdef __CUDA_ARCH__
     double y;
@@ -108,12 +109,25 @@ VAH_HD double recip_d(double d) {
     return 1.0 / d;
 #endif
 }
-VAH_HD double quotient_d(double f, double d) {
+// f / d; a zero may come out as +0 for -0, and an infinity as a NaN (the residual
+// of one): for 1 / d, which is neither, and where neither shows.
+VAH_HD double quotient_normal(double f, double d) {
 #ifdef __CUDA_ARCH__
     const unsigned biased = ((unsigned)__double2hiint(d) >> 20) & 0x7ffu;
     if (biased - 23u > 2000u) return f / d;
     const double y = recip_d(d), q = f * y;
     return fma(y, fma(-d, q, f), q);
+#else
+    return f / d;
+#endif
+}
+// f / d with IEEE's zeros, infinities and NaNs: uncorrected where f y is not a normal number.
+VAH_HD double quotient_d(double f, double d) {
+#ifdef __CUDA_ARCH__
+    const unsigned biased = ((unsigned)__double2hiint(d) >> 20) & 0x7ffu;
+    if (biased - 23u > 2000u) return f / d;
+    const double y = recip_d(d), q = f * y, r = fma(y, fma(-d, q, f), q);
+    return (((unsigned)__double2hiint(q) >> 20) & 0x7ffu) - 1u < 0x7feu ? r : q;
 #else
     return f / d;
 #endif
@@ -137,6 +151,8 @@ VAH_HD double quot(double f, double d) { return quotient_d(f, d); }
 VAH_HD float quot(float f, float d) { return f / d; }
 VAH_HD double quot(double f, double, double inv_d) { return f * inv_d; }
 VAH_HD float quot(float f, float d, float) { return f / d; }
+VAH_HD double inverse(double d) { return quotient_normal(1.0, d); }
+VAH_HD float inverse(float d) { return 1.0f / d; }
 
 // Sums of products. The compiler fuses one product of a b + c d, and whichever
 // it takes depends on the code around it. Dilute edge cells of 2+1D events amplify
@@ -470,7 +486,7 @@ VAH_HD void invert_root(double t, const InvIn &q, InvRoot &r) {
     const double m0 = q.m0, m1 = q.m1, m2 = q.m2, m3 = q.m3, pl = q.pl, bulk = q.bulk;
     double m0pl = m0 + pl;
     if (m0pl == 0.0) m0pl = 1.e-16;
-    r.F = FAST ? quotient_fast(m3, m0pl) : quotient_d(m3, m0pl);
+    r.F = FAST ? quotient_fast(m3, m0pl) : quotient_normal(m3, m0pl);  // not admitted below if not finite
     const double Ft = t * r.F;
     const double Ft2 = Ft * Ft;
     r.x2 = fabs(fma(-Ft, Ft, 1.));
@@ -765,7 +781,7 @@ VAH_HD int cell_sources(const Eos &eos, const R *Q, const CellGradT<R> &g, const
     const R dyut = g.dyut, dyux = g.dyux, dyuy = g.dyuy, dyun = g.dyun;
     const R dnut = g.dnut, dnux = g.dnux, dnuy = g.dnuy, dnun = g.dnun;
 
-    const R inv_ut = quot(R(1.0), ut), inv_t = k.inv_t;
+    const R inv_ut = inverse(ut), inv_t = k.inv_t;
     const R vx = ux * inv_ut, vy = uy * inv_ut, vn = un * inv_ut;
     const R dkvk = (dxux - vx * dxut) * inv_ut + (dyuy - vy * dyut) * inv_ut + (dnun - vn * dnut) * inv_ut;
 
@@ -806,7 +822,7 @@ VAH_HD int cell_sources(const Eos &eos, const R *Q, const CellGradT<R> &g, const
     const R uTdnuT = ux * dnux + uy * dnuy;
     const R uTduT = fused(ut, ux * dtux + uy * dtuy, ux * uTdxuT) + uy * uTdyuT + un * uTdnuT;
     const R F = 1 + uT2;
-    const R inv_F = quot(R(1.0), F);
+    const R inv_F = inverse(F);
     const R inv_sF = rsqrt_r(F);
     const R z0 = t * un * inv_sF;
     const R z3 = ut * inv_t * inv_sF;
@@ -835,7 +851,7 @@ VAH_HD int cell_sources(const Eos &eos, const R *Q, const CellGradT<R> &g, const
     if (e == 0) e = R(1.e-7);
     R T, cs2;
     eos_T_cs2(eos, e, &T, &cs2);
-    const R inv_e = quot(R(1.0), e);
+    const R inv_e = inverse(e);
     // The closure fits are evaluated in FP64 whatever R is: their monomial
     // coefficients (up to ~1e7, alternating in sign) cancel to results of
     // O(1e-3), and in FP32 several lose every digit (Rbar0P turns infinite).

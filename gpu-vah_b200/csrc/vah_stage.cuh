@@ -350,7 +350,7 @@ VAH_HD void cell_compute(const StageArgs<S> &a, int i, int j, int k) {
     for (int n = 0; n < NQ; ++n) val[n] = qc[n] + a.dt * Sv[n];
     const int strides[3] = {1, ncx, plane};
     const double hs[3] = {a.dx, a.dy, a.dz};
-    const double ucomp[3] = {g.ux, g.uy, g.un}, inv_ut = quotient_d(1.0, g.ut);
+    const double ucomp[3] = {g.ux, g.uy, g.un}, inv_ut = inverse(g.ut);
 #pragma unroll
     for (int dir = 0; dir < (IS3D ? 3 : 2); ++dir) {
         const int st = strides[dir];
