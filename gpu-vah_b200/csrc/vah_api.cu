@@ -19,6 +19,7 @@
 #include "vah.h"
 #include "vah_ic_device.cuh"
 #include "vah_kernels.cuh"
+#include "vah_march.cuh"
 #include "vah_powf_exc.h"
 
 using vah::FieldSet;
@@ -240,15 +241,23 @@ namespace {
 __global__ void math_values_kernel(int op, const double *a, const double *b, double *out, int n) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const double x = a[i], y = b[i];
-        out[i] = op == VAH_MATH_QUOTIENT ? vah::quotient_d(x, y)
-                                         : (op == VAH_MATH_RECIPROCAL ? vah::recip_d(y) : vah::sqrt_estimate(x));
+        switch (op) {
+        case VAH_MATH_QUOTIENT: out[i] = vah::quotient_d(x, y); break;
+        case VAH_MATH_RECIPROCAL: out[i] = vah::recip_d(y); break;
+        case VAH_MATH_SQRT_ESTIMATE: out[i] = vah::sqrt_estimate(x); break;
+        case VAH_MATH_SLOPE: out[i] = 0.5 * vah::limited4(0.0 - x, y - 0.0, y - x); break;
+        default: {
+            const float xf = (float)x, yf = (float)y;
+            out[i] = (double)(0.5f * vah::limited4(0.0f - xf, yf - 0.0f, yf - xf));
+        }
+        }
     }
 }
 
 }  // namespace
 
 extern "C" int vah_math_values(int device, int op, const double *a, const double *b, int n, double *out) {
-    if (op < VAH_MATH_QUOTIENT || op > VAH_MATH_SQRT_ESTIMATE || !a || !b || !out || n < 1) return VAH_ERR_ARG;
+    if (op < VAH_MATH_QUOTIENT || op > VAH_MATH_SLOPE_FP32 || !a || !b || !out || n < 1) return VAH_ERR_ARG;
     VAH_TRY(cudaSetDevice(device));
     double *d = nullptr;
     const size_t bytes = (size_t)n * sizeof(double);

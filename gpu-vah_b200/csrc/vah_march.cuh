@@ -36,23 +36,31 @@ namespace vah {
 // cell are q -+ limited4 / 4, bit for bit q -+ 0.5 approx_derivative. dl, dr:
 // the differences to either neighbour, cc = the neighbours' difference. With
 // m = min(|dl|, |dr|), slope = min(1.1 m, |cc| / 2) = min(2.2 m, |cc|) / 2.
-// The minima compare bit patterns (non-negative doubles order like integers,
-// NaNs above all, so a NaN is passed over as fmin does) and the signs are bit
-// tests: integer work beside a busy FP64 pipe.
+// The minima compare bit patterns (non-negative numbers order like integers,
+// NaNs above all, so a NaN is passed over as fmin does) and the signs are tests of
+// the upper bits, a NaN not being below zero whatever its sign bit (the device's
+// own FP64 NaN has it set): integer work beside a busy FP64 pipe.
+VAH_HD bool below_zero(uint64_t bits) { return (uint32_t)(bits >> 32) - 0x80000000u <= 0x7ff00000u; }
+VAH_HD bool below_zero(uint32_t bits) { return bits - 0x80000000u <= 0x7f800000u; }
+template <typename U>
+VAH_HD U smaller(U a, U b) { return b < a ? b : a; }
+
 VAH_HD double limited4(double dl, double dr, double cc) {
-#ifdef __CUDA_ARCH__
-    constexpr unsigned long long kAbs = 0x7fffffffffffffffull;
-    const unsigned long long bl = (unsigned long long)__double_as_longlong(dl), br = (unsigned long long)__double_as_longlong(dr);
-    const unsigned long long m = min(bl & kAbs, br & kAbs);
-    const double m22 = 2.2 * __longlong_as_double((long long)m);
-    unsigned long long r = min((unsigned long long)__double_as_longlong(m22), (unsigned long long)__double_as_longlong(cc) & kAbs);
-    r |= bl & ~kAbs;
-    return (long long)(bl ^ br) < 0 ? 0.0 : __longlong_as_double((long long)r);
-#else
-    const double m = fmin(2.2 * fmin(fabs(dl), fabs(dr)), fabs(cc));
-    const bool neg = dl < 0.0;
-    return neg == (dr < 0.0) ? (neg ? -m : m) : 0.0;
-#endif
+    constexpr uint64_t kSign = 1ull << 63;
+    const uint64_t bl = double_bits(dl), br = double_bits(dr);
+    const double m22 = 2.2 * bits_double(smaller(bl & ~kSign, br & ~kSign));
+    const uint64_t r = smaller(double_bits(m22), double_bits(cc) & ~kSign);
+    const bool neg = below_zero(bl);
+    return neg != below_zero(br) ? 0.0 : bits_double(r | (neg ? kSign : 0));
+}
+// The same in FP32.
+VAH_HD float limited4(float dl, float dr, float cc) {
+    constexpr uint32_t kSign = 1u << 31;
+    const uint32_t bl = float_bits(dl), br = float_bits(dr);
+    const float m22 = 2.2f * bits_float(smaller(bl & ~kSign, br & ~kSign));
+    const uint32_t r = smaller(float_bits(m22), float_bits(cc) & ~kSign);
+    const bool neg = below_zero(bl);
+    return neg != below_zero(br) ? 0.0f : bits_float(r | (neg ? kSign : 0));
 }
 
 // The lanes' shares of a face: whether two lanes split its fields, the columns
@@ -93,21 +101,6 @@ VAH_HD int march_strips(int columns) {
 // state and the lower face's flux per field and column.
 template <typename S, int PHYS>
 constexpr int kMarchValues = 5 * Lanes<S, PHYS>::N * 32;
-
-// The same in FP32.
-VAH_HD float limited4(float dl, float dr, float cc) {
-#ifdef __CUDA_ARCH__
-    constexpr unsigned kAbs = 0x7fffffffu;
-    const unsigned bl = __float_as_uint(dl), br = __float_as_uint(dr);
-    const float m22 = 2.2f * __uint_as_float(min(bl & kAbs, br & kAbs));
-    const unsigned r = min(__float_as_uint(m22), __float_as_uint(cc) & kAbs) | (bl & ~kAbs);
-    return (int)(bl ^ br) < 0 ? 0.0f : __uint_as_float(r);
-#else
-    const float m = fminf(2.2f * fminf(fabsf(dl), fabsf(dr)), fabsf(cc));
-    const bool neg = dl < 0.0f;
-    return neg == (dr < 0.0f) ? (neg ? -m : m) : 0.0f;
-#endif
-}
 
 #ifdef __CUDACC__
 

@@ -180,6 +180,7 @@ VAH_HD float add_rounded(float a, float b, float c) { return rounded(a, b) + c; 
 
 namespace vah {
 
+// Numbers as bit patterns and back.
 VAH_HD uint32_t float_bits(float x) {
 #ifdef __CUDA_ARCH__
     return __float_as_uint(x);
@@ -187,6 +188,33 @@ VAH_HD uint32_t float_bits(float x) {
     uint32_t u;
     memcpy(&u, &x, 4);
     return u;
+#endif
+}
+VAH_HD float bits_float(uint32_t u) {
+#ifdef __CUDA_ARCH__
+    return __uint_as_float(u);
+#else
+    float x;
+    memcpy(&x, &u, 4);
+    return x;
+#endif
+}
+VAH_HD uint64_t double_bits(double x) {
+#ifdef __CUDA_ARCH__
+    return (uint64_t)__double_as_longlong(x);
+#else
+    uint64_t u;
+    memcpy(&u, &x, 8);
+    return u;
+#endif
+}
+VAH_HD double bits_double(uint64_t u) {
+#ifdef __CUDA_ARCH__
+    return __longlong_as_double((long long)u);
+#else
+    double x;
+    memcpy(&x, &u, 8);
+    return x;
 #endif
 }
 

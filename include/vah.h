@@ -506,11 +506,14 @@ int vah_stage_noalloc(const vah_lattice *lat, double eta_over_s, int physics, in
  * IEEE arithmetic on the CPU. */
 int vah_math_check(int device, double lo, double hi, int n, double *max_rel_rcp, double *max_rel_rsqrt);
 /* Values of the step's other hand-written device arithmetic, for the same
- * purpose: out[i] = a[i] / b[i], 1 / b[i] (for |b| in [1e-100, 1e101]), or an
- * estimate of sqrt(a[i]) (host arrays of n values). */
+ * purpose: out[i] = a[i] / b[i], 1 / b[i] (for |b| in [1e-100, 1e101]), an
+ * estimate of sqrt(a[i]), or the flux launches' limited slope through the
+ * values a[i], 0, b[i], in FP64 or FP32 (host arrays of n values). */
 #define VAH_MATH_QUOTIENT 0
 #define VAH_MATH_RECIPROCAL 1
 #define VAH_MATH_SQRT_ESTIMATE 2
+#define VAH_MATH_SLOPE 3
+#define VAH_MATH_SLOPE_FP32 4
 int vah_math_values(int device, int op, const double *a, const double *b, int n, double *out);
 
 /* FP64 FMA throughput of the device, measured: a persistent grid

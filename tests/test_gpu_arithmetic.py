@@ -1,5 +1,5 @@
-"""The step's quotient, reciprocal and square root estimate on the device
-(vah_math_values) against IEEE arithmetic.
+"""The step's quotient, reciprocal, square root estimate and limited slope on
+the device (vah_math_values) against IEEE arithmetic.
 
 Bounds: the reciprocal's last Newton-Raphson step leaves e^2 (2^-80) and two
 roundings, 2^-52 relative; the quotient's residual correction leaves its
@@ -13,7 +13,7 @@ import pytest
 import vahlib as V
 
 D = C.POINTER(C.c_double)
-QUOTIENT, RECIPROCAL, SQRT_ESTIMATE = 0, 1, 2
+QUOTIENT, RECIPROCAL, SQRT_ESTIMATE, SLOPE, SLOPE_FP32 = range(5)
 
 
 def values(op, a, b):
@@ -33,7 +33,7 @@ def test_math_values_argument_errors():
     L = V.library()
     L.vah_math_values.argtypes = [C.c_int, C.c_int, D, D, C.c_int, D]
     x = (C.c_double * 1)(1.0)
-    for op, n, a in ((-1, 1, x), (3, 1, x), (0, 0, x), (0, 1, None)):
+    for op, n, a in ((-1, 1, x), (5, 1, x), (0, 0, x), (0, 1, None)):
         assert L.vah_math_values(0, op, a, x, n, x) == -1
 
 
@@ -78,3 +78,29 @@ def test_reciprocal_and_square_root_estimate():
     x = np.abs(x)
     assert np.max(np.abs(values(SQRT_ESTIMATE, x, x) / np.sqrt(x) - 1)) <= 2e-6
     assert np.array_equal(values(SQRT_ESTIMATE, [0.0], [1.0]), [0.0])
+
+
+def slope(dl, dr, cc):
+    """The limiter by its formula: theta = 1.1, a NaN passed over by the minima
+    (fmin) and not below zero."""
+    t = dl.dtype.type
+    with np.errstate(all="ignore"):
+        m = np.fmin(t(1.1) * np.fmin(abs(dl), abs(dr)), abs(cc * t(0.5)))
+        neg = dl < 0
+        return np.where(neg == (dr < 0), np.where(neg, -m, m), t(0))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("op,t", [(SLOPE, np.float64), (SLOPE_FP32, np.float32)])
+def test_limited_slope_equals_the_limiter(op, t):
+    """Value for value, beside NaNs and infinities too: the device's own NaN of
+    an FP64 difference has its sign bit set, which is not a negative slope."""
+    rng = np.random.default_rng(3)
+    x = np.array([0.0, -0.0, 1e-30, -1e-30, 1.0, -1.0, 1.1, 3.0, -2.5, 1e30, np.inf, -np.inf, np.nan, -np.nan])
+    a, b = (v.ravel() for v in np.meshgrid(x, x))
+    a = np.concatenate([a, rng.normal(size=300_000), rng.normal(size=300_000)]).astype(t)
+    b = np.concatenate([b, rng.normal(size=300_000), a[-300_000:] * t(-1) + t(1e-3) * rng.normal(size=300_000).astype(t)]).astype(t)
+    with np.errstate(all="ignore"):
+        want = slope(t(0) - a, b - t(0), b - a)
+    got = values(op, a.astype(np.float64), b.astype(np.float64)).astype(t)
+    assert np.array_equal(got, want, equal_nan=True)
