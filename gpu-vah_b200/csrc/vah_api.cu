@@ -382,18 +382,26 @@ extern "C" int vah_event_create(const vah_lattice *lat, const vah_hydro *hydro, 
     } else {
         ev->stream = (cudaStream_t)opt->stream;
     }
+    if (rc == VAH_OK && cudaMalloc((void **)&ev->d_fstage, ev->fstage * sizeof(double)) != cudaSuccess) rc = VAH_ERR_NOMEM;
     // one allocation: the state (2 N_q + 16 arrays), then the flux differences
-    // of as many planes as 4 GB holds (at least one; a stage runs slab by slab)
+    // of as many planes as 4 GB holds, or of fewer where the device has less (at
+    // least one; a stage runs slab by slab)
     const bool split = opt->flux != VAH_FLUX_PER_CELL_FUSED || ev->elem == sizeof(float);
     const int ndir = lat->nz > 1 ? 3 : 2;
     const size_t plane = (size_t)ev->ncx * ev->ncy * ev->elem;
     ev->d_planes = (int)std::min<size_t>(lat->nz, std::max<size_t>(1, ((size_t)4 << 30) / (plane * ndir * ev->nq)));
     auto padded = [](size_t n) { return (n + 255) / 256 * 256; };
-    const size_t field = padded(ev->ncell * ev->elem), diff = padded(plane * ev->d_planes);
-    const size_t state = field * (2 * ev->nq + 16);
+    const size_t field = padded(ev->ncell * ev->elem), state = field * (2 * ev->nq + 16);
+    size_t diff = padded(plane * ev->d_planes);
     char *at = nullptr;
     if (rc == VAH_OK) {
         cudaError_t e = cudaMalloc(&ev->block, state + (split ? diff * ndir * ev->nq : 0));
+        while (e == cudaErrorMemoryAllocation && split && ev->d_planes > 1) {  // half as many planes, down to one
+            cudaGetLastError();  // else the next launch's check would find it
+            ev->d_planes = (ev->d_planes + 1) / 2;
+            diff = padded(plane * ev->d_planes);
+            e = cudaMalloc(&ev->block, state + diff * ndir * ev->nq);
+        }
         if (e == cudaSuccess) e = cudaMemset(ev->block, 0, state);
         if (e != cudaSuccess) rc = cuda_status(e);
         at = (char *)ev->block;
@@ -419,7 +427,6 @@ extern "C" int vah_event_create(const vah_lattice *lat, const vah_hydro *hydro, 
             for (int d = 0; d < ndir; ++d)
                 for (int n = 0; n < ev->nq; ++n) ev->D[d][n] = next(diff);
     }
-    if (rc == VAH_OK && cudaMalloc((void **)&ev->d_fstage, ev->fstage * sizeof(double)) != cudaSuccess) rc = VAH_ERR_NOMEM;
     if (rc == VAH_OK && cudaMalloc((void **)&ev->d_counters, 4 * sizeof(unsigned long long)) != cudaSuccess)
         rc = VAH_ERR_NOMEM;
     if (rc == VAH_OK) cudaMemset(ev->d_counters, 0, 4 * sizeof(unsigned long long));
