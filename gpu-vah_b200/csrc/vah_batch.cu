@@ -336,6 +336,7 @@ struct vah_batch {
     std::vector<unsigned char> desc_host;  // host mirror of the descriptor array
     double *d_fstage;  // staging of the field reads ...
     size_t fstage;     // ... of this many values
+    std::vector<WorkItem> lists[vah::K_NUM];  // the work-lists, kept for their memory
     WorkItem *d_work[vah::K_NUM];
     void *d_args;        // StageArgs<S>[cap_args]: both stages' arguments by slab
     size_t cap_args;     // in StageArgs
@@ -531,10 +532,18 @@ ScratchBounds scratch_bounds(const vah_batch *b, const vah_lattice *more, size_t
     return r;
 }
 
+template <typename Item>
+void append(std::vector<WorkItem> &list, int n, Item item) {
+    const size_t at = list.size();
+    list.resize(at + n);
+    for (int m = 0; m < n; ++m) list[at + m] = item(m);
+}
+
 // The work-lists, groups and scratch of the admitted events.
 template <typename S>
 int rebuild_work(vah_batch *b) {
-    std::vector<WorkItem> lists[vah::K_NUM];
+    std::vector<WorkItem>(&lists)[vah::K_NUM] = b->lists;
+    for (auto &l : lists) l.clear();
     std::vector<int> order;  // largest event first: its items start first, small ones fill the tail
     for (int s = 0; s < (int)b->slots.size(); ++s)
         if (b->slots[s].used) order.push_back(s);
@@ -602,17 +611,18 @@ int rebuild_work(vah_batch *b) {
                 const int strips = kind == 0 ? vah::flux_x_strips<S>(l.nx, l.ny, nk)
                                              : vah::march_strips<S>(l.nx * (kind == 1 ? nk : l.ny));
                 const int at = kind == 2 ? sl.k0 : 0, n = kind == 0 ? 1 : (kind == 1 ? l.ny : sl.k1);
-                const int len = kind == 0 ? 1 : seg[kind];
+                const int len = kind == 0 ? 1 : seg[kind], quads = (strips + 3) / 4;
                 for (int r0 = at; r0 < n; r0 += len)
-                    for (int i0 = 0; i0 < strips; i0 += 4)
-                        lists[vah::K_FLUX].push_back({sl.slot, p, kind, i0, r0, std::min(r0 + len, n)});
+                    append(lists[vah::K_FLUX], quads, [&](int m) -> WorkItem {
+                        return {sl.slot, p, kind, 4 * m, r0, std::min(r0 + len, n)};
+                    });
             }
         for (int p : group) {
             const vah::Slab &sl = slabs[p];
             const vah_lattice &l = b->slots[sl.slot].lat;
-            const int plane = l.nx * l.ny, end = plane * sl.k1;
-            for (int c0 = plane * sl.k0; c0 < end; c0 += vah::kCellItem)
-                lists[l.nz > 1 ? vah::K_C3 : vah::K_C2].push_back({sl.slot, p, 0, c0, 0, end});
+            const int first = l.nx * l.ny * sl.k0, end = l.nx * l.ny * sl.k1;
+            append(lists[l.nz > 1 ? vah::K_C3 : vah::K_C2], (end - first + vah::kCellItem - 1) / vah::kCellItem,
+                   [&](int m) -> WorkItem { return {sl.slot, p, 0, first + vah::kCellItem * m, 0, end}; });
         }
         for (int k = 0; k < vah::K_NUM; ++k) g.count[k] = (int)lists[k].size() - g.first[k];
         b->groups.push_back(g);

@@ -68,19 +68,22 @@ cudaError_t launch_stage_kernel(void (*kernel)(P...), bool dependent, int grid, 
 // Cells per march segment along an axis of n cells, from the number of warps
 // a segment length makes: the fewest waves (148 SMs x minb blocks x 4 warps)
 // times the segment's length plus its start-up (one face and its first
-// loads, about 1.5 cells' work).
+// loads, about 1.5 cells' work). The lengths tried are those of n cells in 1, 2,
+// ... parts, each once (fewer than 2 sqrt(n): a batch sums over its events for each).
 template <typename Warps>
 inline int march_segment(int n, int minb, Warps warps) {
     const long long wave = 148 * 4 * minb;
     int best = 1;
     double cost = 1e300;
-    for (int parts = 1; parts <= n; ++parts) {
-        const int len = (n + parts - 1) / parts;
+    for (int len = n; len >= 1;) {
         const double c = (double)((warps(len) + wave - 1) / wave) * (len + 1.5);
         if (c < cost) {
             cost = c;
             best = len;
         }
+        if (len == 1) break;
+        const int parts = (n + len - 2) / (len - 1);  // the fewest whose cells are shorter
+        len = (n + parts - 1) / parts;
     }
     return best;
 }
