@@ -14,10 +14,8 @@
 
 #ifdef __CUDACC__
 #define VAH_HD __host__ __device__ __forceinline__
-#define VAH_COLD __host__ __device__ __forceinline__
 #else
 #define VAH_HD inline
-#define VAH_COLD inline
 #endif
 
 namespace vah {
@@ -565,9 +563,8 @@ VAH_HD double root_velocity(const InvRoot &r, double m_dir, int dir) {
 // reached e or u). out = {e, p, ut, ux, uy, un}. PF32 (the FP32 form): the
 // pressure from the EoS in FP32 arithmetic (the form stores p in FP32).
 // Its iterated form: (e, u^mu) by Newton's iteration or the fallback; the
-// status without the NaN test. Out of line on the device: seldom run, and its
-// registers stay out of the callers.
-VAH_COLD int invert_iterated(double t, InvIn q, double ePrev, double uT0, double *out) {
+// status without the NaN test. Seldom run.
+VAH_HD int invert_iterated(double t, InvIn q, double ePrev, double uT0, double *out) {
     InvSetup s;
     invert_setup(t, q, s);
     double uT;
@@ -635,7 +632,7 @@ VAH_HD int invert(const Eos &eos, double t, const double *q, double ePrev, doubl
 // The velocity of one face state by the iteration (u^dir / u^tau of its root,
 // 0 after a fallback): 0 converged, 1 fallback, 2 NaN. Seldom run.
 template <bool FAST>
-VAH_COLD int face_velocity_iterated(double t, InvIn q, int dir, double ePrev, double ux0, double uy0, double *v) {
+VAH_HD int face_velocity_iterated(double t, InvIn q, int dir, double ePrev, double ux0, double uy0, double *v) {
     InvSetup s;
     invert_setup<FAST>(t, q, s);
     double uT;
@@ -959,6 +956,7 @@ VAH_HD int cell_sources(const Eos &eos, const R *Q, const CellGradT<R> &g, const
     S[2] = -tty * inv_t - dyptHat + dkvk * pity;
     // SourceTerms.cpp:686: the reference adds dnLtn twice
     const R S3 = -3 * ttn * inv_t - dnptHat * inv_t2 + dkvk * (Ltn + pitn) + vx * dxLtn + vy * dyLtn + vn * (dnLtn + dnLtn);
+    // (with and without bulk the kernels of the FP32 form rounded this product differently)
     S[3] = BULK ? fused(-t2dnLnn, inv_t2, S3) : S3 - rounded(t2dnLnn, inv_t2);
     int bad = isnan(S[4]) || isnan(S[0]);
 

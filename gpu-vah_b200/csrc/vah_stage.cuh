@@ -90,10 +90,10 @@ VAH_HD double ld(const S *p, I i) {
     return (double)load(p + i);
 }
 
-// Face values are read once, by the cell launch: loaded with the streaming
+// Flux differences are read once, by the cell launch: loaded with the streaming
 // (evict-first) cache policy, so that they do not push the state's neighbour
-// reuse out of L1 and L2 (cell launch 3% faster; streaming stores in the face
-// launches cost those 2%, so they store normally).
+// reuse out of L1 and L2 (cell launch 3% faster; streaming stores in the flux
+// launch cost it 2%, so it stores normally). A coherent load, as load().
 template <typename S, typename I>
 VAH_HD double ld_stream(const S *p, I i) {
 #ifdef __CUDA_ARCH__

@@ -49,16 +49,7 @@ VAH_HD Pair approx_derivative2(Pair x, Pair y, Pair z) {
 }
 
 // --------------------------------------------- the FP32 form's cell algebra --
-// Host-and-device code: the kernel runs it on the shared-memory box, and the
-// host build (tests/hostcheck) on plain arrays, through accessors
-// q(n, index) of the conserved fields.
-
-// The shared-memory box: field n at n * BOXN.
-template <int BOXN>
-struct BoxQ {
-    const float *s;
-    VAH_HD float operator()(int n, long long i) const { return s[n * BOXN + i]; }
-};
+// Host-and-device code, through accessors q(n, index) of the conserved fields.
 
 // One array per field.
 struct ArrQ {
@@ -71,7 +62,7 @@ struct ArrQ {
 // states reconstructed in FP32, inverted in FP64 from the guess uT (the left
 // cell's |u_T|; the setup's and the velocities' divisions through
 // quotient_fast), H[n hs] = wR qR + wL qL in FP32 (hs: the stride of the
-// destination, e.g. a shared face buffer). Returns the number of inversions
+// destination). Returns the number of inversions
 // that fell back; bit 8 flags a NaN (ePrev: the left cell's e).
 template <int PHYS, typename QA>
 VAH_HD unsigned tile_face(const QA q, long long L, long long st, int dir, double t, double ePrev, double uT,
@@ -117,9 +108,8 @@ VAH_HD unsigned tile_face(const QA q, long long L, long long st, int dir, double
 }
 
 // Stage-input primitives: e, p, u read at the cell and its +-1 neighbours
-// (index pi, strides psy, psz: the shared-memory box on the device, the
-// field arrays on the host), and at the cell only (global index s) the
-// previous stage's u and the inversion's guess u.
+// (index pi, strides psy, psz), and at the cell only (index s) the previous
+// stage's u and the inversion's guess u.
 struct TilePrims {
     const float *E, *P, *U[4];
     long long pi, psy, psz;
@@ -127,7 +117,7 @@ struct TilePrims {
 };
 
 // The explicit part of a cell's stage (eulerStepKernelSource and the axis
-// sources): q: the stage-input conserved fields at box index b (strides bsy,
+// sources): q: the stage-input conserved fields at index b (strides bsy,
 // bsz); pr: the primitives; s: the cell's global index; flux[n]: the flux
 // differences dt/h (H(-1/2) - H(+1/2)) summed over the axes. Writes the
 // updated conserved values to val and the cell's e (the inversion's fallback
